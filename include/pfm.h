@@ -149,6 +149,11 @@ int pfm_measure_fp32_peak(float* sink, int blocks_per_sm, int iters, int reps, i
 #define PFM_TUNE_MIDPOINT_CENTRE 5 /* 1: the 3D midpoint's first RK stage, which samples the face centre,
                                      uses its constant weights and leaves out the zero-weight taps
                                      (interior faces, power-of-two dx); 0: the generic taps (1) */
+#define PFM_TUNE_MG_CLUSTER 6     /* 1: an MGPCG solve whose levels fit the shared memory of one thread-block
+                                     cluster is one launch, and so are the coarse levels of a larger
+                                     one's V-cycle; 0: grid-wide kernels (1).  The other MGPCG keys act
+                                     on what runs grid-wide; sums are grouped differently, so the two
+                                     settings agree to rounding. */
 int pfm_set_tuning(pfm_handle* h, int key, int value);
 int pfm_get_tuning(const pfm_handle* h, int key, int* value);
 

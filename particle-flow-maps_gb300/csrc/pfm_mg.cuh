@@ -1,0 +1,121 @@
+// Definitions shared by the MGPCG translation units: levels, boundary flags, level storage, the
+// 7- (5-) point stencil, compensated sums and the stopping rule.
+#pragma once
+
+#include <cuda_bf16.h>
+#include <cuda_fp16.h>
+
+#include "pfm_internal.cuh"
+
+namespace pfm {
+
+struct Lvl {
+  int n0, n1, n2;
+  int64_t count;
+  Div32 d1, d2;  // divisors n1, n2
+  Div32 dh;      // divisor (last extent + 1) / 2: the cell pairs of a smoothing sweep
+};
+
+static inline Lvl make_lvl(int n0, int n1, int n2, int D) {
+  const int last = (D == 3) ? n2 : n1;
+  return Lvl{n0, n1, n2, (int64_t)n0 * n1 * n2, make_div32((unsigned)n1), make_div32((unsigned)n2),
+             make_div32((unsigned)((last + 1) >> 1))};
+}
+
+struct BC {
+  int lo[3], hi[3];  // 2 = Neumann
+};
+
+static inline Lvl lvl_of(const pfm_handle* h, int l) {
+  return make_lvl(h->lv[l].n[0], h->lv[l].n[1], h->lv[l].n[2], h->cfg.dim);
+}
+
+// Multigrid level storage: FP32 (the reference), or FP16 / BF16 in the mixed-precision solve;
+// values are widened to FP32 on load and rounded to nearest on store.
+__device__ __forceinline__ float ldv(const float* p) { return *p; }
+__device__ __forceinline__ float ldv(const __half* p) { return __half2float(*p); }
+__device__ __forceinline__ float ldv(const __nv_bfloat16* p) { return __bfloat162float(*p); }
+__device__ __forceinline__ void stv(float* p, float v) { *p = v; }
+__device__ __forceinline__ void stv(__half* p, float v) { *p = __float2half_rn(v); }
+__device__ __forceinline__ void stv(__nv_bfloat16* p, float v) { *p = __float2bfloat16_rn(v); }
+
+// neighbor_sum / num_fluid_neighbors (3D/mgpcg.py:92-115)
+template <int D, typename S>
+__device__ __forceinline__ void stencil(const S* __restrict__ f, const Lvl& L, const BC& bc, int i, int j,
+                                        int k, int64_t e, float& nb, float& mult) {
+  float ret = 0.f;
+  float num = 2.f * D;
+  const int64_t sx = (int64_t)L.n1 * L.n2, sy = L.n2;
+  if (i < L.n0 - 1) ret += ldv(f + e + sx);
+  if (i > 0) ret += ldv(f + e - sx);
+  if (D == 3) {
+    if (j < L.n1 - 1) ret += ldv(f + e + sy);
+    if (j > 0) ret += ldv(f + e - sy);
+    if (k < L.n2 - 1) ret += ldv(f + e + 1);
+    if (k > 0) ret += ldv(f + e - 1);
+  } else {
+    if (j < L.n1 - 1) ret += ldv(f + e + sy);
+    if (j > 0) ret += ldv(f + e - sy);
+  }
+  if (i <= 0 && bc.lo[0] == 2) num -= 1.f;
+  if (i >= L.n0 - 1 && bc.hi[0] == 2) num -= 1.f;
+  if (j <= 0 && bc.lo[1] == 2) num -= 1.f;
+  if (j >= L.n1 - 1 && bc.hi[1] == 2) num -= 1.f;
+  if (D == 3) {
+    if (k <= 0 && bc.lo[2] == 2) num -= 1.f;
+    if (k >= L.n2 - 1 && bc.hi[2] == 2) num -= 1.f;
+  }
+  nb = ret;
+  mult = num;
+}
+
+// num_fluid_neighbors alone (the mult of stencil<D>, no loads)
+template <int D>
+__device__ __forceinline__ float stencil_mult(const Lvl& L, const BC& bc, int i, int j, int k) {
+  float num = 2.f * D;
+  if (i <= 0 && bc.lo[0] == 2) num -= 1.f;
+  if (i >= L.n0 - 1 && bc.hi[0] == 2) num -= 1.f;
+  if (j <= 0 && bc.lo[1] == 2) num -= 1.f;
+  if (j >= L.n1 - 1 && bc.hi[1] == 2) num -= 1.f;
+  if (D == 3) {
+    if (k <= 0 && bc.lo[2] == 2) num -= 1.f;
+    if (k >= L.n2 - 1 && bc.hi[2] == 2) num -= 1.f;
+  }
+  return num;
+}
+
+__device__ __forceinline__ void decode(const Lvl& L, int64_t e, int& i, int& j, int& k) {
+  split3((unsigned)e, L.d1, L.d2, i, j, k);
+}
+
+// Per-thread partial sums of the mixed solve: Neumaier-compensated f32 (each thread adds at most a
+// few hundred terms; the block and grid sums are f64).  Per-element f64 arithmetic would run on
+// GB300's narrow FP64 pipe and cost about 0.1 ms per PCG iteration at 256^3.
+struct CompSum {
+  float s = 0.f, c = 0.f;
+  __device__ __forceinline__ void add(float x) {
+    const float t = s + x;
+    c += (fabsf(s) >= fabsf(x)) ? ((s - t) + x) : ((x - t) + s);
+    s = t;
+  }
+  __device__ __forceinline__ double value() const { return (double)s + (double)c; }
+};
+
+// the stopping rule of k_update_xr / k_true_residual; the relative rules accept an exactly zero
+// residual, so a zero right-hand side (a fluid at rest) ends at the first check
+__device__ __forceinline__ bool converged(double rTr, const SolveState* st, double tol, int tol_mode) {
+  if (tol_mode == 0) return rTr < tol;
+  const double ref = (tol_mode == 1) ? st->rTr0 : st->bTb;
+  return rTr == 0.0 || sqrt(rTr) < tol * sqrt(ref);
+}
+
+static inline BC bc_of(const pfm_handle* h) {
+  BC b;
+  for (int d = 0; d < 3; ++d) {
+    b.lo[d] = (d < h->cfg.dim) ? h->cfg.boundary[d][0] : 2;
+    b.hi[d] = (d < h->cfg.dim) ? h->cfg.boundary[d][1] : 2;
+  }
+  return b;
+}
+
+}  // namespace pfm

@@ -1,0 +1,53 @@
+// The cluster-resident MGPCG (pfm_mgcluster.cu): plan types and host entry points.
+#pragma once
+
+#include "pfm_mg.cuh"
+
+namespace pfm {
+
+constexpr int kClusterThreads = 512;
+// A cluster grows until its CTAs hold at most this many cells of the finest level (a vector of
+// four cells of a colour for every fourth thread).
+constexpr int kCellsPerCta = 1024;
+// Levels of at most this many cells run on one CTA of a whole solve.
+constexpr int kSoloCells = 4096;
+
+struct CLev {
+  int n0, n1, nk;    // rows, middle extent (1 in 2D), last extent
+  int half, hs;      // (nk + 1) / 2, and rounded up to a multiple of four: the stride of a row's colour
+  int plane;         // n1 * hs: one colour of a row
+  int rmax, shift;   // rows of the largest share; share boundaries are (c nbase / nc) << shift
+  int cz, cr;        // elements per colour of z (a ghost row on either side, a zero pad) and of r
+  Div32 dh, dhv, dh2, d1;  // divisors half, hs / 4, half / 2, n1
+  unsigned z, r;     // byte offsets in shared memory
+};
+
+struct CPlan {
+  int nc, L, l0, lg;  // CTAs; levels l0 .. lg-1 distributed, lg .. L-1 solo
+  int ld, nbase;      // the level whose rows define the shares (the first solo level, else the last), its rows
+  int pre_post, bottom;
+  BC bc;
+  CLev lv[kMaxLevels];
+};
+
+struct CSolve {
+  const float* rhs;
+  float *x, *p, *Ap, *b;
+  SolveState* st;
+  double tol;
+  float eps_s, eps_c, tol_s, tol_c, inv_n_s, inv_n_c;  // eps, tol and 1 / cells as sums of two floats
+  int tol_mode, max_iters, warm, true_every, keep_b, neu;
+  unsigned rf;  // byte offset of the FP32 residual
+};
+
+// Whether a solve of this handle and these options runs as one cluster launch, and that launch: from
+// the right-hand side in r_0 (and x, warm-started) of the workspace to x and the solve state.
+bool cluster_solve_fits(const pfm_handle* h, const pfm_solve_opts& o);
+int cluster_solve_launch(pfm_handle* h, const pfm_solve_opts& o, cudaStream_t s);
+
+// The first level (at least 1) from which a V-cycle runs as one cluster launch, or h->L; the launch.
+int cluster_tail_level(const pfm_handle* h, int precision);
+int cluster_tail_launch(pfm_handle* h, int precision, int l0, void* z, const void* r, const SolveState* st,
+                        cudaStream_t s);
+
+}  // namespace pfm

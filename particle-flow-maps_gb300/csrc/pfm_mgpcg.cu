@@ -9,98 +9,17 @@
 //    f64 block and grid combination in block order (no float atomics);
 //  * the restriction scatter (r_{l+1}[I//2] += res/(dim-1), 3D/mgpcg.py:152-158) is a gather
 //    over the 8 (4 in 2D) children, so it needs no atomics either.
-#include <cuda_bf16.h>
-#include <cuda_fp16.h>
-
 #include <cmath>
 #include <algorithm>
 #include <atomic>
 #include <type_traits>
 #include <vector>
 
-#include "pfm_internal.cuh"
+#include "pfm_mg.cuh"
+#include "pfm_mgcluster.cuh"
 #include "pfm_tma.cuh"
 
 namespace pfm {
-
-struct Lvl {
-  int n0, n1, n2;
-  int64_t count;
-  Div32 d1, d2;  // divisors n1, n2
-  Div32 dh;      // divisor (last extent + 1) / 2: the cell pairs of a smoothing sweep
-};
-
-static inline Lvl make_lvl(int n0, int n1, int n2, int D) {
-  const int last = (D == 3) ? n2 : n1;
-  return Lvl{n0, n1, n2, (int64_t)n0 * n1 * n2, make_div32((unsigned)n1), make_div32((unsigned)n2),
-             make_div32((unsigned)((last + 1) >> 1))};
-}
-
-struct BC {
-  int lo[3], hi[3];  // 2 = Neumann
-};
-
-static inline Lvl lvl_of(const pfm_handle* h, int l) {
-  return make_lvl(h->lv[l].n[0], h->lv[l].n[1], h->lv[l].n[2], h->cfg.dim);
-}
-
-// Multigrid level storage: FP32 (the reference), or FP16 / BF16 in the mixed-precision solve;
-// values are widened to FP32 on load and rounded to nearest on store.
-__device__ __forceinline__ float ldv(const float* p) { return *p; }
-__device__ __forceinline__ float ldv(const __half* p) { return __half2float(*p); }
-__device__ __forceinline__ float ldv(const __nv_bfloat16* p) { return __bfloat162float(*p); }
-__device__ __forceinline__ void stv(float* p, float v) { *p = v; }
-__device__ __forceinline__ void stv(__half* p, float v) { *p = __float2half_rn(v); }
-__device__ __forceinline__ void stv(__nv_bfloat16* p, float v) { *p = __float2bfloat16_rn(v); }
-
-// neighbor_sum / num_fluid_neighbors (3D/mgpcg.py:92-115)
-template <int D, typename S>
-__device__ __forceinline__ void stencil(const S* __restrict__ f, const Lvl& L, const BC& bc, int i, int j,
-                                        int k, int64_t e, float& nb, float& mult) {
-  float ret = 0.f;
-  float num = 2.f * D;
-  const int64_t sx = (int64_t)L.n1 * L.n2, sy = L.n2;
-  if (i < L.n0 - 1) ret += ldv(f + e + sx);
-  if (i > 0) ret += ldv(f + e - sx);
-  if (D == 3) {
-    if (j < L.n1 - 1) ret += ldv(f + e + sy);
-    if (j > 0) ret += ldv(f + e - sy);
-    if (k < L.n2 - 1) ret += ldv(f + e + 1);
-    if (k > 0) ret += ldv(f + e - 1);
-  } else {
-    if (j < L.n1 - 1) ret += ldv(f + e + sy);
-    if (j > 0) ret += ldv(f + e - sy);
-  }
-  if (i <= 0 && bc.lo[0] == 2) num -= 1.f;
-  if (i >= L.n0 - 1 && bc.hi[0] == 2) num -= 1.f;
-  if (j <= 0 && bc.lo[1] == 2) num -= 1.f;
-  if (j >= L.n1 - 1 && bc.hi[1] == 2) num -= 1.f;
-  if (D == 3) {
-    if (k <= 0 && bc.lo[2] == 2) num -= 1.f;
-    if (k >= L.n2 - 1 && bc.hi[2] == 2) num -= 1.f;
-  }
-  nb = ret;
-  mult = num;
-}
-
-// num_fluid_neighbors alone (the mult of stencil<D>, no loads)
-template <int D>
-__device__ __forceinline__ float stencil_mult(const Lvl& L, const BC& bc, int i, int j, int k) {
-  float num = 2.f * D;
-  if (i <= 0 && bc.lo[0] == 2) num -= 1.f;
-  if (i >= L.n0 - 1 && bc.hi[0] == 2) num -= 1.f;
-  if (j <= 0 && bc.lo[1] == 2) num -= 1.f;
-  if (j >= L.n1 - 1 && bc.hi[1] == 2) num -= 1.f;
-  if (D == 3) {
-    if (k <= 0 && bc.lo[2] == 2) num -= 1.f;
-    if (k >= L.n2 - 1 && bc.hi[2] == 2) num -= 1.f;
-  }
-  return num;
-}
-
-__device__ __forceinline__ void decode(const Lvl& L, int64_t e, int& i, int& j, int& k) {
-  split3((unsigned)e, L.d1, L.d2, i, j, k);
-}
 
 // ---------------------------------------------------------------------------------------------
 // deterministic block/grid reduction
@@ -960,27 +879,6 @@ __global__ void __launch_bounds__(256) k_zero(S* __restrict__ a, int64_t n, cons
 // ---------------------------------------------------------------------------------------------
 enum RedKind { RED_ZTR_INIT = 0, RED_ZTR = 1, RED_RTR0 = 2, RED_MEAN = 3, RED_BTB = 4 };
 
-// Per-thread partial sums of the mixed solve: Neumaier-compensated f32 (each thread adds at most a
-// few hundred terms; the block and grid sums are f64).  Per-element f64 arithmetic would run on
-// GB300's narrow FP64 pipe and cost about 0.1 ms per PCG iteration at 256^3.
-struct CompSum {
-  float s = 0.f, c = 0.f;
-  __device__ __forceinline__ void add(float x) {
-    const float t = s + x;
-    c += (fabsf(s) >= fabsf(x)) ? ((s - t) + x) : ((x - t) + s);
-    s = t;
-  }
-  __device__ __forceinline__ double value() const { return (double)s + (double)c; }
-};
-
-// the stopping rule of k_update_xr / k_true_residual; the relative rules accept an exactly zero
-// residual, so a zero right-hand side (a fluid at rest) ends at the first check
-__device__ __forceinline__ bool converged(double rTr, const SolveState* st, double tol, int tol_mode) {
-  if (tol_mode == 0) return rTr < tol;
-  const double ref = (tol_mode == 1) ? st->rTr0 : st->bTb;
-  return rTr == 0.0 || sqrt(rTr) < tol * sqrt(ref);
-}
-
 // sum(a*b) (or sum(a) for RED_MEAN) with a finalizer that updates the solve state.  Per-thread
 // partials accumulate in f32 (the reference solve) or f64 (f64 != 0, the mixed solve).
 template <typename SA>
@@ -1598,15 +1496,6 @@ struct OpTail {
 // ---------------------------------------------------------------------------------------------
 // host orchestration
 // ---------------------------------------------------------------------------------------------
-static BC bc_of(const pfm_handle* h) {
-  BC b;
-  for (int d = 0; d < 3; ++d) {
-    b.lo[d] = (d < h->cfg.dim) ? h->cfg.boundary[d][0] : 2;
-    b.hi[d] = (d < h->cfg.dim) ? h->cfg.boundary[d][1] : 2;
-  }
-  return b;
-}
-
 static unsigned red_blocks(int64_t n) {
   unsigned b = grid_for(n, kReduceThreads);
   return b > (unsigned)kReduceBlocks ? (unsigned)kReduceBlocks : b;
@@ -1722,7 +1611,9 @@ template <int D, typename S>
 static void vcycle(pfm_handle* h, const SolveState* st, cudaStream_t s) {
   const int L = h->L;
   const BC bc = bc_of(h);
-  const int l0 = tail_level(h);
+  const int precision = sizeof(S) == 4 ? 0 : (std::is_same<S, __half>::value ? 1 : 2);
+  const int lc = cluster_tail_level(h, precision);  // from here on one cluster launch, where the level fits
+  const int l0 = std::min(lc, tail_level(h));
   bool zero_first[kMaxLevels] = {};
   auto flush = [&](int l) {  // a use of z_l other than a half-sweep: zero it now if still due
     if (zero_first[l]) {
@@ -1747,7 +1638,10 @@ static void vcycle(pfm_handle* h, const SolveState* st, cudaStream_t s) {
       launch(h, k_restrict<D, S>, grid_for(Lc.count, 256), 256, 0, s, (const S*)level_z<S>(h, l),
              (const S*)level_r<S>(h, l), Lf, level_r<S>(h, l + 1), Lc, bc, st);
   }
-  if (l0 < L) {
+  if (lc < L) {
+    zero_first[lc] = false;  // the cluster writes all of z_lc
+    cluster_tail_launch(h, precision, lc, level_z<S>(h, lc), level_r<S>(h, lc), st, s);
+  } else if (l0 < L) {
     TailPlan T{};
     T.l0 = l0;
     T.L = L;
@@ -1961,6 +1855,22 @@ struct SolveKernels {
   }
 };
 
+// The statistics and the status of a finished solve from its state.
+static int solve_result(pfm_handle* h, const SolveState& hs, bool true_res, pfm_solve_stats* stats) {
+  if (stats) {
+    stats->converged = hs.done == 1;
+    stats->iterations = hs.done ? hs.conv_it : hs.it;
+    stats->rTr = hs.rTr;
+    stats->rTr0 = hs.rTr0;
+    stats->bTb = hs.bTb;
+    stats->rTr_true = true_res ? hs.rTr_true : -1.0;
+  }
+  if (hs.done == 3) return set_error(h, PFM_ERR_NONFINITE, "MGPCG: non-finite residual");
+  if (hs.done == 4) return set_error(h, PFM_ERR_CUDA, "MGPCG: a smoother's tile copy did not arrive");
+  if (hs.done != 1) return set_error(h, PFM_ERR_NOT_CONVERGED, "MGPCG: iteration limit reached");
+  return PFM_OK;
+}
+
 // MGPCG.solve (3D/mgpcg.py:202-280) on r_0 (already k r); the solution is left in the workspace
 // vector x.  Two graphs per handle, captured once per option set: the setup graph and the loop
 // graph (k_loop_begin -> WHILE(not done and it < it_stop) { body } -> finish -> the device state
@@ -1973,6 +1883,13 @@ static int solve_impl(pfm_handle* h, const pfm_solve_opts& o, pfm_solve_stats* s
   const int mi = K.mi;
   const int chunk = K.chunk;
   SolveState* hs = h->h_state;
+  if (cluster_solve_fits(h, o)) {  // a small grid: the whole solve is one cluster launch
+    int rc = cluster_solve_launch(h, o, s);
+    if (!rc)
+      rc = check_cuda(h, cudaMemcpyAsync(hs, K.st, sizeof(SolveState), cudaMemcpyDeviceToHost, s), "solve state read");
+    if (!rc) rc = check_cuda(h, cudaStreamSynchronize(s), "mgpcg sync");
+    return rc ? rc : solve_result(h, *hs, K.true_res, stats);
+  }
   const int key_mode = (o.precision & 3) | (K.warm ? 4 : 0) | (K.replace ? 8 : 0);
   if (!h->g_valid || h->g_eps != o.eps || h->g_tol != o.tol || h->g_mode != o.tol_mode || h->g_max_iters != mi ||
       h->g_chunk != chunk || h->g_variant != key_mode || h->g_true_every != o.true_residual_every) {
@@ -2018,18 +1935,7 @@ static int solve_impl(pfm_handle* h, const pfm_solve_opts& o, pfm_solve_stats* s
     it_before = hs->it;
     if (hs->done || mi >= 0) break;
   }
-  if (stats) {
-    stats->converged = hs->done == 1;
-    stats->iterations = hs->done ? hs->conv_it : hs->it;
-    stats->rTr = hs->rTr;
-    stats->rTr0 = hs->rTr0;
-    stats->bTb = hs->bTb;
-    stats->rTr_true = K.true_res ? hs->rTr_true : -1.0;
-  }
-  if (hs->done == 3) return set_error(h, PFM_ERR_NONFINITE, "MGPCG: non-finite residual");
-  if (hs->done == 4) return set_error(h, PFM_ERR_CUDA, "MGPCG: a smoother's tile copy did not arrive");
-  if (hs->done != 1) return set_error(h, PFM_ERR_NOT_CONVERGED, "MGPCG: iteration limit reached");
-  return PFM_OK;
+  return solve_result(h, *hs, K.true_res, stats);
 }
 
 template <int D>
@@ -2206,6 +2112,7 @@ int append_poisson_pre(GraphCursor& gc, float* const* u, float* p_io, const pfm_
   else
     launch_divergence<2>(h, u[0], u[1], nullptr, r0, -1.f, q);
   if (o.warm_start && !gc.rc) gc.rc = warm_start_init(h, x, p_io, o.warm_start, q);
+  if (cluster_solve_fits(h, o)) return gc.rc;  // the setup is part of the cluster's launch
   dispatch_solve(D, o.precision, [&](auto dd, auto ss) {
     SolveKernels<decltype(dd)::value, decltype(ss)> K(h, o);
     K.setup(gc.seg());
@@ -2216,6 +2123,15 @@ int append_poisson_pre(GraphCursor& gc, float* const* u, float* p_io, const pfm_
 int append_poisson_loop(GraphCursor& gc, const pfm_solve_opts& opts, float* p_io, StepCtl* ctl, int which) {
   pfm_solve_opts o = opts;
   if (!p_io) o.warm_start = 0;
+  if (cluster_solve_fits(gc.h, o)) {
+    if (!gc.rc) {
+      const int rc = cluster_solve_launch(gc.h, o, gc.seg());
+      if (rc) gc.rc = rc;
+    }
+    launch(gc.h, k_record_solve, 1, 1, 0, gc.seg(), ctl, (const SolveState*)ws_ptr<SolveState>(gc.h, gc.h->o_state),
+           which, 0);
+    return gc.rc;
+  }
   dispatch_solve(gc.h->cfg.dim, o.precision,
                  [&](auto dd, auto ss) { append_solve<decltype(dd)::value, decltype(ss)>(gc, o, ctl, which); });
   return gc.rc;

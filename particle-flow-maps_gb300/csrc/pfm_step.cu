@@ -15,7 +15,7 @@
 #include <string>
 #include <vector>
 
-#include "pfm_internal.cuh"
+#include "pfm_mgcluster.cuh"
 
 namespace pfm {
 
@@ -474,11 +474,39 @@ static int build_batch_worklist(pfm_batch* b, cudaGraph_t G) {
     }
     return PFM_OK;
   };
+  // small scenes solve as one cluster launch in their own branch; the others join in the batched loop
+  std::vector<size_t> joint;
+  for (size_t s = 0; s < n; ++s)
+    if (!cluster_solve_fits(hs[s], b->scenes[s].p.poisson)) joint.push_back(s);
+  std::vector<pfm_handle*> jhs;
+  std::vector<StepCtl*> jctls;
+  for (size_t s : joint) {
+    jhs.push_back(hs[s]);
+    jctls.push_back(ctls[s]);
+  }
   uint64_t joint_body = 0;  // batched body kernels: counted on the device, not as fixed kernels
+  auto p_of = [&](size_t s, int which) {
+    const auto& sc = b->scenes[s];
+    return which == 0 ? (sc.dim == 3 ? sc.f3.p_mid : sc.f2.p_mid) : (sc.dim == 3 ? sc.f3.p : sc.f2.p);
+  };
   auto batched = [&](int which) -> int {
-    GraphCursor J(hs[0], G, b->cap);
+    for (size_t s = 0, j = 0; s < n; ++s) {
+      if (j < joint.size() && joint[j] == s) {
+        ++j;
+        continue;
+      }
+      GraphCursor& gc = *cur[s];
+      append_poisson_loop(gc, b->scenes[s].p.poisson, p_of(s, which), ctls[s], which);
+      gc.close();
+      if (gc.rc) {
+        b->err = b->scenes[s].h->err;
+        return gc.rc;
+      }
+    }
+    if (joint.empty()) return PFM_OK;
+    GraphCursor J(jhs[0], G, b->cap);
     J.ndeps = 0;
-    for (size_t s = 0; s < n; ++s)
+    for (size_t s : joint)
       for (size_t d = 0; d < cur[s]->ndeps; ++d) {
         if (J.ndeps == sizeof(J.deps) / sizeof(J.deps[0])) {
           b->err = "work-list batch: too many branch ends to join";
@@ -486,21 +514,20 @@ static int build_batch_worklist(pfm_batch* b, cudaGraph_t G) {
         }
         J.deps[J.ndeps++] = cur[s]->deps[d];
       }
-    int rc = append_batched_loop(J, hs.data(), (int)n, s0.p.poisson, ctls.data(), which);
+    int rc = append_batched_loop(J, jhs.data(), (int)jhs.size(), s0.p.poisson, jctls.data(), which);
     J.close();
     if (!rc) rc = J.rc;
     if (rc) {
-      b->err = hs[0]->err;
+      b->err = jhs[0]->err;
       return rc;
     }
     joint_body += J.body_launches;
-    for (size_t s = 0; s < n; ++s) {  // fork: each scene's finish and statistics, then its next part
+    for (size_t s : joint) {  // fork: each scene's finish and statistics, then its next part
       const auto& sc = b->scenes[s];
       GraphCursor& gc = *cur[s];
       gc.ndeps = J.ndeps;
       for (size_t d = 0; d < J.ndeps; ++d) gc.deps[d] = J.deps[d];
-      float* p_io = which == 0 ? (sc.dim == 3 ? sc.f3.p_mid : sc.f2.p_mid) : (sc.dim == 3 ? sc.f3.p : sc.f2.p);
-      append_poisson_finish(gc, sc.p.poisson, p_io, ctls[s], which);
+      append_poisson_finish(gc, sc.p.poisson, p_of(s, which), ctls[s], which);
       gc.close();  // the branches share one capture stream: one open segment at a time
       if (gc.rc) {
         b->err = sc.h->err;
@@ -519,7 +546,7 @@ static int build_batch_worklist(pfm_batch* b, cudaGraph_t G) {
     const auto& sc = b->scenes[s];
     GraphCursor& gc = *cur[s];
     gc.close();
-    se[s].fixed = (sc.h->launches - before[s]) - gc.body_launches - (s == 0 ? joint_body : 0);
+    se[s].fixed = (sc.h->launches - before[s]) - gc.body_launches - (!joint.empty() && s == joint[0] ? joint_body : 0);
     sc.h->launches = before[s];
     rc = patch_control(sc.h, se[s]);
     if (rc) {
