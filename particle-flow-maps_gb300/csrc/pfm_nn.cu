@@ -6,18 +6,15 @@
 // operand an MMA needs a canonical no-swizzle K-major tile in shared memory without any copy:
 //
 //  * Forward / data-gradient convolution (k_conv3_fwd): implicit GEMM D[voxel][cout] =
-//    sum over 27 taps and cin of X[voxel + tap][ci] W[tap][co][ci].  A CTA owns 128 output voxels
-//    (one d0 plane, 16 rows of 8 along d2).  One TMA tiled load brings the 3 x 18 x 10 input brick
-//    with its halo (zero fill outside the grid is the convolution's padding) as
-//    [cin/8][3][18][10][8]: for a fixed 8-channel block, 8 consecutive voxels along d2 are 8
-//    consecutive 16-byte rows, i.e. an 8x16B "core matrix"; the 16 rows of the tile are 160 bytes
-//    apart and the channel blocks 8640 bytes apart.  Each tap is then just another start address of
-//    the same shared-memory descriptor (LBO 8640, SBO 160): no im2col in memory or in shared
-//    memory.  The weights of one tap, [cin/8][npad][8], are a plain bulk copy (cp.async.bulk) into a
-//    four-stage ring.  One thread issues tcgen05.mma (M 128, N npad, K 16, kind::f16 BF16 x BF16 ->
-//    F32) into a TMEM accumulator; four warps read it back with tcgen05.ld for the epilogue (bias,
-//    ReLU, BF16 or F32 store).  The data gradient is the same kernel on the output gradient with the
-//    weights flipped and transposed (k_nn_pack_w).
+//    sum over 27 taps and cin of X[voxel + tap][ci] W[tap][co][ci].  A CTA sweeps tiles of 128 voxels
+//    (16 rows of 8 along d2) along d0.  TMA tiled loads bring each input plane with its halo (zero fill
+//    outside the grid is the convolution's padding) as [cin/8][18][10][8]: for a fixed 8-channel block,
+//    8 consecutive voxels along d2 are 8 consecutive 16-byte rows, i.e. an 8x16B "core matrix"; the rows
+//    of the tile are 160 bytes apart.  Each (b, c) tap is then just another start address of the same
+//    shared-memory descriptor: no im2col in memory or in shared memory.  tcgen05.mma (M 128, K 16,
+//    kind::f16 BF16 x BF16 -> F32) accumulates in TMEM; four warps read it back with tcgen05.ld for the
+//    epilogue (bias, ReLU, BF16 or F32 store).  The data gradient is the same kernel on the output
+//    gradient with the weights flipped and transposed (k_pack_w).
 //  * Weight gradient (k_conv3_wgrad): D[(tap, ci)][co] = sum over voxels X[v + tap][ci] dY[v][co],
 //    K = voxels.  The operands need voxels along the 16-byte rows, so the CTA transposes 8x8 blocks
 //    of the TMA-loaded brick and output-gradient tile into K-major core matrices in shared memory
@@ -41,13 +38,12 @@
 namespace pfm {
 namespace nn {
 
-constexpr int kThreads = 128;
 constexpr int kTileD1 = 16, kTileD2 = 8;  // 128 output voxels per CTA
 constexpr int kBoxD0 = 3, kBoxD1 = kTileD1 + 2, kBoxD2 = kTileD2 + 2;
 constexpr int kBoxVox = kBoxD0 * kBoxD1 * kBoxD2;  // 540
 constexpr int kChunkBytes = kBoxVox * 16;          // one 8-channel block of the brick: 8640 B
 constexpr int kRowBytes = kBoxD2 * 16;             // one brick row along d2: 160 B
-constexpr int kStages = 4;                         // weight ring depth
+constexpr int kSms = 152;
 constexpr int kMaxCin = 128, kMaxNpad = 128;
 constexpr int kSmPerGpuSmem = 233472;                  // shared memory per SM (228 KB)
 constexpr int kMaxDynSmem = 232448 - 64;               // per-CTA limit (227 KB) less the static flag
@@ -76,6 +72,17 @@ __device__ __forceinline__ void mma_bf16(uint32_t d_tmem, uint64_t adesc, uint64
       : "memory");
 }
 
+// true in one lane of a converged warp
+__device__ __forceinline__ bool elect_one() {
+  uint32_t p;
+  asm volatile(
+      "{\n\t.reg .pred e;\n\t"
+      "elect.sync _|e, 0xffffffff;\n\t"
+      "selp.u32 %0, 1, 0, e;\n\t}\n"
+      : "=r"(p));
+  return p != 0;
+}
+
 // arrives on `bar` once every tcgen05.mma this thread issued before has completed
 __device__ __forceinline__ void mma_commit(uint64_t* bar) {
   asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(su32(bar))
@@ -97,6 +104,16 @@ __device__ __forceinline__ void tmem_ld16(uint32_t taddr, float (&v)[16]) {
   for (int i = 0; i < 16; ++i) v[i] = __uint_as_float(r[i]);
 }
 
+// zeros into 16 consecutive 32-bit TMEM columns of this warp's 32 lanes
+__device__ __forceinline__ void tmem_zero16(uint32_t taddr) {
+  asm volatile(
+      "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1, %1, %1, %1, %1, %1, %1, %1, %1, %1, %1, %1, %1, %1, %1, %1};"
+      ::"r"(taddr), "r"(0)
+      : "memory");
+}
+
+__device__ __forceinline__ void tmem_st_wait() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
+
 // Shared-memory matrix descriptor, no swizzle: start address, leading-dimension byte offset (the
 // stride between core matrices along K) and stride-dimension byte offset (between 8-row groups
 // along M or N), all in 16-byte units; bit 46 is the descriptor version of this architecture.
@@ -111,16 +128,22 @@ __host__ __device__ constexpr uint32_t idesc_bf16(int M, int N) {
   return (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(N >> 3) << 17) | ((uint32_t)(M >> 4) << 24);
 }
 
+constexpr int kFwdThreads = 192;  // warp 0: TMA, warp 1: MMA, warps 2-5: epilogue
+constexpr int kMaxRing = 16;      // output planes a CTA keeps in TMEM
+constexpr int kPlaneStages = 4, kTapStages = 9;
+
 struct ConvFwdParams {
   int n0, n1, n2;
   int tiles2;          // tiles along d2 (8 voxels each); blockIdx.x = t1 * tiles2 + t2
+  int mt;              // 128-voxel tiles per CTA, side by side along d1
+  int seg;             // output planes per CTA (blockIdx.y)
+  int ring;            // output planes with an accumulator at a time (per tile)
   int cin, c1;         // input channels (x1 holds the first c1)
-  int npad, cout;      // MMA N (multiple of 16) and real output channels
+  int npad, cout;      // columns of one output plane (multiple of 16) and real output channels
   int ncols;           // TMEM columns allocated
-  int nstage;          // weight ring depth in taps (27: every tap's weights loaded up front)
-  uint32_t idesc;
-  const __nv_bfloat16* w;  // [27][cin/8][npad][8]
-  const float* bias;       // [cout] or null
+  int nstage;          // ring of input planes
+  int wstage;          // 9: every tap's weights stay in shared memory; else a ring of (b, c) taps
+  const float* bias;   // [cout] or null
   int relu;
   __nv_bfloat16* y1;  // channel-blocked output, channels [0, cy1)
   int cy1;
@@ -130,131 +153,297 @@ struct ConvFwdParams {
   int* err;
 };
 
-__global__ void __launch_bounds__(kThreads) k_conv3_fwd(const __grid_constant__ CUtensorMap tm1,
-                                                        const __grid_constant__ CUtensorMap tm2,
-                                                        const ConvFwdParams p) {
+// A CTA owns mt x 128 voxels of the (d1, d2) plane and sweeps `seg` output planes along d0.  Every input
+// plane is loaded once and multiplied by the taps of all three d0 offsets at once: the N columns of one MMA
+// are the three output planes the input plane reaches, side by side in TMEM (column groups of npad, newest
+// plane first), so a plane takes 9 (b, c) taps x cin/16 MMAs of N = 3 npad instead of 27 x cin/16 of
+// N = npad.  An MMA here takes some 34 + N/2 cycles (reading A, 128 x 16 values, is not hidden: 57 at N 48,
+// 80 at 96, 125 at 192), so that halves the tensor core's time, and the input is read 1.4 (seg + 2) / seg
+// times instead of 4.2 times.  The column groups form a ring that the epilogue frees, zeroed, plane by plane,
+// so `seg` is not bound by TMEM; where three planes straddle the ring's end their MMAs come in two.  An output
+// plane's terms arrive in the order of its 27 taps: the planes below, beside and above it in turn, each by
+// (b, c) and channel block.  Three roles overlap: TMA (a ring of planes, the weights once or as a ring of
+// taps), MMA (one lane), epilogue of finished planes.  Bound by the tensor core for 48 channels and more
+// (MMAs at 58 of 57 cycles), by the issuing warp (some 1000 cycles per plane beside its MMAs) for 16.
+// 16 -> 16 at 192^3 684 -> 169 us, 48 -> 16 at 192^3 2359 -> 374 us, 96 -> 32 at 96^3 1094 -> 162 us
+// (one tile per CTA, all 27 taps in turn, before).
+__global__ void __launch_bounds__(kFwdThreads) k_conv3_fwd(const __grid_constant__ CUtensorMap tm1,
+                                                           const __grid_constant__ CUtensorMap tm2,
+                                                           const __grid_constant__ CUtensorMap tmw,
+                                                           const ConvFwdParams p) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   unsigned char* smem = (unsigned char*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  __shared__ int s_skip;
-  if (tid == 0) s_skip = *(volatile int*)p.err;
-  __syncthreads();
-  if (s_skip) return;  // an earlier CTA gave up: do nothing (uniform over the CTA)
-
-  const int nchunk = p.cin >> 3;
-  const uint32_t box_bytes = (uint32_t)nchunk * kChunkBytes;
-  const uint32_t stage_bytes = (uint32_t)p.npad * p.cin * 2;
-  unsigned char* box = smem;
-  unsigned char* wring = smem + ((box_bytes + 127) & ~127u);
-  const int ns = p.nstage;
-  uint64_t* bars = (uint64_t*)(wring + ns * stage_bytes);
-  uint64_t* box_bar = bars;
-  uint64_t* full = bars + 1;
-  uint64_t* done = bars + 1 + ns;
-  uint64_t* final_bar = bars + 1 + 2 * ns;
-  uint32_t* slot = (uint32_t*)(bars + 2 + 2 * ns);
+  const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;
+  const int kc = p.cin >> 3;
+  const uint32_t chunk = (uint32_t)(p.mt * kTileD1 + 2) * kRowBytes;  // one 8-channel block of a plane
+  const uint32_t plane_bytes = (uint32_t)kc * chunk;
+  const uint32_t plane_pitch = (plane_bytes + 127) & ~127u;
+  const uint32_t wtap_bytes = (uint32_t)kc * 3u * (uint32_t)p.npad * 16u;  // one (b, c): [cin/8][3][npad][8]
+  unsigned char* wbuf = smem + (size_t)p.nstage * plane_pitch;
+  uint64_t* full = (uint64_t*)(wbuf + (size_t)p.wstage * wtap_bytes);
+  uint64_t *empty = full + kPlaneStages, *wfull = empty + kPlaneStages, *wempty = wfull + kTapStages,
+           *pdone = wempty + kTapStages, *pfree = pdone + kMaxRing, *fin = pfree + kMaxRing;
+  uint32_t* slot = (uint32_t*)(fin + 1);
+  int* skip = (int*)(slot + 1);
+  float* s_bias = (float*)(slot + 2);
 
   const int t1 = blockIdx.x / p.tiles2, t2 = blockIdx.x - t1 * p.tiles2;
-  const int z = blockIdx.y, y0 = t1 * kTileD1, x0 = t2 * kTileD2;
+  const int y0 = t1 * p.mt * kTileD1, x0 = t2 * kTileD2;
+  const int zs = (int)blockIdx.y * p.seg, ze = min(zs + p.seg, p.n0);
+  const int in0 = max(zs - 1, 0), in1 = min(ze, p.n0 - 1);  // input planes inside the grid
+  const bool resident = p.wstage == 9;
 
-  if (tid == 0) {
-    mbar_init(box_bar, 1);
-    for (int s = 0; s < ns; ++s) {
-      mbar_init(full + s, 1);
-      mbar_init(done + s, 1);
+  if (warp == 0) {  // each lane its barriers
+    if (lane < kPlaneStages) {
+      mbar_init(full + lane, 1);
+      mbar_init(empty + lane, 1);
+    } else if (lane < kPlaneStages + kTapStages) {
+      mbar_init(wfull + (lane - kPlaneStages), 1);
+      mbar_init(wempty + (lane - kPlaneStages), 1);
+    } else if (lane == 31) {
+      mbar_init(fin, 1);
+      *skip = *(volatile int*)p.err;
     }
-    mbar_init(final_bar, 1);
+    if (lane < kMaxRing) {
+      mbar_init(pdone + lane, 1);
+      mbar_init(pfree + lane, 128);
+    }
     fence_mbar_init();
+  } else if (warp == 1) {
+    tmem_alloc(slot, (uint32_t)p.ncols);
+  } else {
+    if (warp == 2 && lane == 0) {
+      prefetch_map(&tm1);
+      prefetch_map(&tmw);
+      if (p.cin > p.c1) prefetch_map(&tm2);
+    }
+    for (int i = tid - 64; i < p.npad; i += 128) s_bias[i] = p.bias && i < p.cout ? p.bias[i] : 0.f;
   }
-  if (warp == 0) tmem_alloc(slot, (uint32_t)p.ncols);
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem = *slot;
+  if (*skip) {  // an earlier CTA gave up: do nothing (uniform over the CTA)
+    if (warp == 1) tmem_dealloc(tmem, (uint32_t)p.ncols);
+    return;
+  }
 
-  if (tid == 0) {
-    bool ok = true;
-    mbar_expect_tx(box_bar, box_bytes);
-    tma_load_5d(box, &tm1, 0, x0 - 1, y0 - 1, z - 1, 0, box_bar);
-    if (p.cin > p.c1) tma_load_5d(box + (size_t)(p.c1 >> 3) * kChunkBytes, &tm2, 0, x0 - 1, y0 - 1, z - 1, 0, box_bar);
-    for (int t = 0; t < ns; ++t) {
-      mbar_expect_tx(full + t, stage_bytes);
-      bulk_load(wring + t * stage_bytes, (const unsigned char*)p.w + (size_t)t * stage_bytes, stage_bytes, full + t);
+  if (warp == 0) {
+    if (lane == 0) {
+      bool ok = true;
+      // the weights of tap pair (b, c): rows [a = 0][a = 1][a = 2] of each channel block, so that the columns
+      // of an MMA are the output planes z + 1, z, z - 1 of input plane z
+      auto load_tap = [&](int bc, int s) {
+        mbar_expect_tx(wfull + s, wtap_bytes);
+        tma_load_4d(wbuf + (size_t)s * wtap_bytes, &tmw, 0, 0, 0, bc, wfull + s);
+      };
+      int wi = 0, i = 0;  // taps and planes asked for
+      for (; i <= in1 - in0; ++i) {
+        const int s = i % p.nstage;
+        if (i >= p.nstage) ok = mbar_wait(empty + s, (unsigned)(i / p.nstage - 1) & 1u, p.err, 1);
+        if (!ok) break;
+        unsigned char* dst = smem + (size_t)s * plane_pitch;
+        mbar_expect_tx(full + s, plane_bytes);
+        tma_load_4d(dst, &tm1, 8 * (x0 - 1), y0 - 1, in0 + i, 0, full + s);
+        if (p.cin > p.c1)
+          tma_load_4d(dst + (size_t)(p.c1 >> 3) * chunk, &tm2, 8 * (x0 - 1), y0 - 1, in0 + i, 0, full + s);
+        if (!resident || i == 0)
+          for (int bc = 0; bc < 9; ++bc, ++wi) {
+            const int ws = wi % p.wstage;
+            if (wi >= p.wstage) ok = mbar_wait(wempty + ws, (unsigned)(wi / p.wstage - 1) & 1u, p.err, 2);
+            if (!ok) break;
+            load_tap(bc, ws);
+          }
+        if (!ok) {
+          ++i;
+          break;
+        }
+      }
+      if (*(volatile int*)p.err != 0) {  // giving up: the copies in flight land before this memory is given back
+        for (int q = max(0, i - p.nstage); q < i; ++q) mbar_drain(full + q % p.nstage, (unsigned)(q / p.nstage) & 1u);
+        for (int q = max(0, wi - p.wstage); q < wi; ++q) mbar_drain(wfull + q % p.wstage, (unsigned)(q / p.wstage) & 1u);
+      }
     }
-    ok = mbar_wait(box_bar, 0, p.err, 1);
-    const uint32_t box_addr = su32(box), ring_addr = su32(wring);
-    const uint32_t blbo = (uint32_t)p.npad * 16;
-    for (int t = 0; t < 27 && ok; ++t) {
-      const int s = t % ns;
-      ok = mbar_wait(full + s, (t / ns) & 1, p.err, 2);
+  } else if (warp == 1) {
+    // The whole warp runs the loop, so that descriptors stay in uniform registers, and one lane issues: with
+    // the loop inside a one-lane branch each MMA took 500 to 700 cycles to issue, more than it takes to run.
+    const bool lead = elect_one();
+    bool ok = true;
+    int s = 0, ws = 0;               // plane and tap stage
+    unsigned phase = 0, wphase = 0;
+    int at = zs == 0 && ze > 1 ? 1 : 0, done = 0;  // ring slots of the newest plane and of the next one to finish
+    unsigned lap = 0;
+    const int gmax = 256 / p.npad;  // output planes one MMA can hold (N <= 256)
+    const int nj = p.cin >> 4;
+    const uint32_t lbo_b = 3u * (uint32_t)p.npad * 16u;
+    // descriptors advance by their address field (16-byte units): no carry leaves it
+    const uint32_t a_step = 2 * chunk / 16, b_step = 2 * lbo_b / 16, w_step = wtap_bytes / 16;
+    const uint32_t a_tile = kTileD1 * kBoxD2, d_tile = (uint32_t)(p.ring * p.npad);
+    const uint64_t bd0 = smem_desc(su32(wbuf), lbo_b, 128);
+    const uint64_t a_first = smem_desc(su32(smem), chunk, kRowBytes);
+    if (resident)
+      for (int bc = 0; bc < 9; ++bc) ok = ok && mbar_wait(wfull + bc, 0, p.err, 4);
+    if (at == 1) ok = ok && mbar_wait(pfree, 0, p.err, 6);
+    // a plane's input and its new accumulator are looked for while the plane before is issued
+    bool has_in = false, has_acc = false;
+    for (int z = in0; z <= in1; ++z) {
+      const int lo = max(z - 1, zs), hi = min(z + 1, ze - 1);
+      if (!has_acc) ok = ok && mbar_wait(pfree + at, lap & 1u, p.err, 6);
+      if (!has_in) ok = ok && mbar_wait(full + s, phase, p.err, 3);
+      ok = __all_sync(0xffffffffu, ok);
       if (!ok) break;
       tc_fence_after();
-      const int a = t / 9, b = (t / 3) % 3, c = t % 3;
-      const uint32_t a0 = box_addr + (uint32_t)(((a * kBoxD1 + b) * kBoxD2 + c) * 16);
-      const uint32_t b0 = ring_addr + (uint32_t)s * stage_bytes;
-      for (int j = 0; j < (p.cin >> 4); ++j) {
-        const uint64_t ad = smem_desc(a0 + (uint32_t)(2 * j) * kChunkBytes, kChunkBytes, kRowBytes);
-        const uint64_t bd = smem_desc(b0 + (uint32_t)(2 * j) * blbo, blbo, 128);
-        mma_bf16(tmem, ad, bd, p.idesc, (t | j) != 0);
-      }
-      mma_commit(done + s);
-      // refill the stage the previous tap used once its MMAs have completed
-      if (t >= 1 && t - 1 + ns < 27) {
-        const int sp = (t - 1) % ns;
-        ok = mbar_wait(done + sp, ((t - 1) / ns) & 1, p.err, 3);
-        if (!ok) break;
-        mbar_expect_tx(full + sp, stage_bytes);
-        bulk_load(wring + sp * stage_bytes, (const unsigned char*)p.w + (size_t)(t - 1 + ns) * stage_bytes,
-                  stage_bytes, full + sp);
-      }
-    }
-    mma_commit(final_bar);
-  }
-  const bool fin = mbar_wait(final_bar, 0, p.err, 4);
-  tc_fence_after();
-
-  // epilogue: warp w holds TMEM lanes 32w..32w+31 = output voxels m = 32w + lane
-  const int m = warp * 32 + lane;
-  const int yy = y0 + (m >> 3), xx = x0 + (m & 7);
-  const bool valid = fin && yy < p.n1 && xx < p.n2;
-  const size_t V = (size_t)p.n0 * p.n1 * p.n2;
-  const size_t vox = ((size_t)z * p.n1 + yy) * p.n2 + xx;
-  const float scale = (p.yf && p.yf_scale) ? *p.yf_scale : 1.f;
-  for (int c0 = 0; c0 < p.npad; c0 += 16) {
-    float v[16];
-    tmem_ld16(tmem + ((uint32_t)(warp * 32) << 16) + (uint32_t)c0, v);
-    if (!valid) continue;
+      const int s1 = s + 1 == p.nstage ? 0 : s + 1, at1 = z + 2 > ze - 1 ? at : at + 1 == p.ring ? 0 : at + 1;
+      const unsigned phase1 = phase ^ (s1 == 0), lap1 = lap + (at1 < at);
+      has_in = mbar_test(full + s1, phase1);
+      has_acc = at1 == at || mbar_test(pfree + at1, lap1 & 1u);
+      const uint64_t ad0 = a_first + (uint32_t)s * (plane_pitch / 16);
+      const uint64_t bdz = bd0 + (uint32_t)((z + 1 - hi) * p.npad);  // rows of the planes that are not there left out
+      // the planes' columns in runs: cut at the ring's end and at N = 256
+      const int n = hi - lo + 1, r1 = min(min(n, at + 1), gmax);
+      const int at2 = r1 > at ? p.ring - 1 : at - r1, r2 = min(min(n - r1, at2 + 1), gmax);
+      const int at3 = r2 > at2 ? p.ring - 1 : at2 - r2, r3 = n - r1 - r2;
+      const uint32_t d1 = tmem + (uint32_t)((p.ring - 1 - at) * p.npad), id1 = idesc_bf16(128, r1 * p.npad);
+      const uint32_t d2 = tmem + (uint32_t)((p.ring - 1 - at2) * p.npad), id2 = idesc_bf16(128, r2 * p.npad);
+      const uint32_t d3 = tmem + (uint32_t)((p.ring - 1 - at3) * p.npad), id3 = idesc_bf16(128, r3 * p.npad);
+      const uint32_t b2 = (uint32_t)(r1 * p.npad), b3 = (uint32_t)((r1 + r2) * p.npad);
+      auto step = [&](uint64_t ad, uint64_t bd) {
+        mma_bf16(d1, ad, bd, id1, 1u);
+        if (r2) mma_bf16(d2, ad, bd + b2, id2, 1u);
+        if (r3) mma_bf16(d3, ad, bd + b3, id3, 1u);
+        if (p.mt == 2) {
+          mma_bf16(d1 + d_tile, ad + a_tile, bd, id1, 1u);
+          if (r2) mma_bf16(d2 + d_tile, ad + a_tile, bd + b2, id2, 1u);
+          if (r3) mma_bf16(d3 + d_tile, ad + a_tile, bd + b3, id3, 1u);
+        }
+      };
+      if (resident && r2 == 0) {
+        if (lead) {
 #pragma unroll
-    for (int q = 0; q < 2; ++q) {
-      const int nb = c0 + 8 * q;
-      if (nb >= p.cout) break;
-      float o[8];
-#pragma unroll
-      for (int e = 0; e < 8; ++e) {
-        float r = v[8 * q + e];
-        if (p.bias && nb + e < p.cout) r += p.bias[nb + e];
-        if (p.relu) r = fmaxf(r, 0.f);
-        o[e] = r;
-      }
-      if (p.yf) {
-        for (int e = 0; e < 8 && nb + e < p.cout; ++e) p.yf[(size_t)(nb + e) * V + vox] = o[e] * scale;
+          for (int bc = 0; bc < 9; ++bc) {
+            const uint64_t ad = ad0 + (uint32_t)((bc / 3) * kBoxD2 + bc % 3);
+            const uint64_t bd = bdz + (uint32_t)bc * w_step;
+            mma_bf16(d1, ad, bd, id1, 1u);
+            for (int j = 1; j < nj; ++j) mma_bf16(d1, ad + (uint32_t)j * a_step, bd + (uint32_t)j * b_step, id1, 1u);
+          }
+        }
       } else {
-        uint4 pk;
-        __nv_bfloat162 h0 = __floats2bfloat162_rn(o[0], o[1]), h1 = __floats2bfloat162_rn(o[2], o[3]);
-        __nv_bfloat162 h2 = __floats2bfloat162_rn(o[4], o[5]), h3 = __floats2bfloat162_rn(o[6], o[7]);
-        pk.x = *(uint32_t*)&h0;
-        pk.y = *(uint32_t*)&h1;
-        pk.z = *(uint32_t*)&h2;
-        pk.w = *(uint32_t*)&h3;
-        __nv_bfloat16* dst = nb < p.cy1 ? p.y1 + ((size_t)(nb >> 3) * V + vox) * 8
-                                        : p.y2 + ((size_t)((nb - p.cy1) >> 3) * V + vox) * 8;
-        *(uint4*)dst = pk;
+        uint64_t adr = ad0;
+        bool has_tap = false;
+        for (int b = 0; b < 3 && ok; ++b, adr += kBoxD2) {
+#pragma unroll
+          for (int c = 0; c < 3; ++c) {
+            const int ws1 = ws + 1 == p.wstage ? 0 : ws + 1;
+            const unsigned wphase1 = wphase ^ (ws1 == 0);
+            if (!resident) {
+              if (!has_tap) ok = ok && mbar_wait(wfull + ws, wphase, p.err, 4);
+              ok = __all_sync(0xffffffffu, ok);
+              has_tap = mbar_test(wfull + ws1, wphase1);
+            }
+            if (ok && lead) {
+              uint64_t ad = adr + c, bd = bdz + (uint32_t)ws * w_step;
+              if (r2) {
+                for (int j = 0; j < nj; ++j, ad += a_step, bd += b_step) step(ad, bd);
+              } else if (p.mt == 2) {
+                for (int j = 0; j < nj; ++j, ad += a_step, bd += b_step) {
+                  mma_bf16(d1, ad, bd, id1, 1u);
+                  mma_bf16(d1 + d_tile, ad + a_tile, bd, id1, 1u);
+                }
+              } else {
+                for (int j = 0; j < nj; ++j, ad += a_step, bd += b_step) mma_bf16(d1, ad, bd, id1, 1u);
+              }
+              if (!resident) mma_commit(wempty + ws);
+            }
+            ws = ws1;
+            wphase = wphase1;
+          }
+        }
+        if (!ok) break;
+      }
+      if (lead) {
+        mma_commit(empty + s);
+        if (z > zs) mma_commit(pdone + done);
+      }
+      if (z > zs && ++done == p.ring) done = 0;
+      s = s1;
+      phase = phase1;
+      at = at1;
+      lap = lap1;
+    }
+    if (ok && lead && in1 == ze - 1) mma_commit(pdone + done);  // the grid ends with the segment
+    if (*(volatile int*)p.err != 0) {  // giving up: what was issued ends before its operands and TMEM go
+      if (lead) mma_commit(fin);
+      mbar_drain(fin, 0);
+    }
+    __syncwarp();
+  } else {
+    // epilogue: warp w reads TMEM lanes 32 (w % 4) .. + 31 = output voxels m = 32 (w % 4) + lane
+    const int m = (warp & 3) * 32 + lane;
+    const int xx = x0 + (m & 7);
+    const size_t V = (size_t)p.n0 * p.n1 * p.n2;
+    const float scale = (p.yf && p.yf_scale) ? *p.yf_scale : 1.f;
+    const uint32_t lanes = tmem + ((uint32_t)((warp & 3) * 32) << 16);
+    // accumulators start from zero: here, and again as each plane is read
+    for (int c0 = 0; c0 < p.mt * p.ring * p.npad; c0 += 16) tmem_zero16(lanes + (uint32_t)c0);
+    tmem_st_wait();
+    tc_fence_before();
+    for (int s = 0; s < p.ring; ++s) mbar_arrive(pfree + s);
+    int r = 0;
+    unsigned phase = 0;
+    for (int z = zs; z < ze; ++z) {
+      if (!mbar_wait(pdone + r, phase, p.err, 5)) break;
+      tc_fence_after();
+      for (int tile = 0; tile < p.mt; ++tile) {
+        const int yy = y0 + tile * kTileD1 + (m >> 3);
+        const bool inside = yy < p.n1 && xx < p.n2;
+        const size_t vox = ((size_t)z * p.n1 + yy) * p.n2 + xx;
+        const uint32_t col = (uint32_t)((tile * p.ring + p.ring - 1 - r) * p.npad);
+        for (int c0 = 0; c0 < p.npad; c0 += 16) {
+          float v[16];
+          tmem_ld16(lanes + col + (uint32_t)c0, v);
+          tmem_zero16(lanes + col + (uint32_t)c0);
+          if (!inside) continue;
+#pragma unroll
+          for (int q = 0; q < 2; ++q) {
+            const int nb = c0 + 8 * q;
+            if (nb >= p.cout) break;
+            float o[8];
+#pragma unroll
+            for (int e = 0; e < 8; ++e) {
+              float u = v[8 * q + e];
+              if (p.bias) u += s_bias[nb + e];
+              if (p.relu) u = fmaxf(u, 0.f);
+              o[e] = u;
+            }
+            if (p.yf) {
+              for (int e = 0; e < 8 && nb + e < p.cout; ++e) p.yf[(size_t)(nb + e) * V + vox] = o[e] * scale;
+            } else {
+              uint4 pk;
+              __nv_bfloat162 h0 = __floats2bfloat162_rn(o[0], o[1]), h1 = __floats2bfloat162_rn(o[2], o[3]);
+              __nv_bfloat162 h2 = __floats2bfloat162_rn(o[4], o[5]), h3 = __floats2bfloat162_rn(o[6], o[7]);
+              pk.x = *(uint32_t*)&h0;
+              pk.y = *(uint32_t*)&h1;
+              pk.z = *(uint32_t*)&h2;
+              pk.w = *(uint32_t*)&h3;
+              __nv_bfloat16* dst = nb < p.cy1 ? p.y1 + ((size_t)(nb >> 3) * V + vox) * 8
+                                              : p.y2 + ((size_t)((nb - p.cy1) >> 3) * V + vox) * 8;
+              *(uint4*)dst = pk;
+            }
+          }
+        }
+      }
+      tmem_st_wait();
+      tc_fence_before();
+      mbar_arrive(pfree + r);
+      if (++r == p.ring) {
+        r = 0;
+        phase ^= 1u;
       }
     }
   }
   tc_fence_before();
-  __syncthreads();
-  if (warp == 0) tmem_dealloc(tmem, (uint32_t)p.ncols);
+  __syncthreads();  // every role is done: the epilogue has waited for the last MMAs
+  if (warp == 1) tmem_dealloc(tmem, (uint32_t)p.ncols);
 }
 
 // ---------------------------------------------------------------------------------------------
@@ -357,9 +546,9 @@ __global__ void __launch_bounds__(kWgThreads) k_conv3_wgrad(const __grid_constan
     if (tid == 0) {
       fence_proxy_async();
       mbar_expect_tx(box_bar, box_bytes + dy_bytes);
-      tma_load_5d(box, &tm1, 0, x0 - 1, y0 - 1, z - 1, 0, box_bar);
-      if (p.cin > p.c1) tma_load_5d(box + (size_t)(p.c1 >> 3) * kChunkBytes, &tm2, 0, x0 - 1, y0 - 1, z - 1, 0, box_bar);
-      tma_load_5d(dybox, &tmdy, 0, x0, y0, z, 0, box_bar);
+      tma_load_4d(box, &tm1, 8 * (x0 - 1), y0 - 1, z - 1, 0, box_bar);
+      if (p.cin > p.c1) tma_load_4d(box + (size_t)(p.c1 >> 3) * kChunkBytes, &tm2, 8 * (x0 - 1), y0 - 1, z - 1, 0, box_bar);
+      tma_load_4d(dybox, &tmdy, 8 * x0, y0, z, 0, box_bar);
     }
     bool w = mbar_wait(box_bar, box_phase, p.err, 11);
     box_phase ^= 1;
@@ -663,16 +852,33 @@ __global__ void k_adam(float* __restrict__ p, const float* __restrict__ g, float
 // ---------------------------------------------------------------------------------------------
 // host side
 
-// tensor map of a channel-blocked bf16 tensor: dims (8, n2, n1, n0, C/8), box (8, b2, b1, b0, C/8)
+// tensor map of a channel-blocked bf16 tensor: dims (8 n2, n1, n0, C/8), box (8 b2, b1, b0, C/8).  The eight
+// channels of consecutive voxels are one run of memory, so a box row of b2 voxels is one copy of 16 b2
+// bytes (as five dimensions with an inner one of 8 channels the engine moved 16 bytes at a time).
 bool make_map(CUtensorMap* tm, const void* base, int C, int n0, int n1, int n2, int b0, int b1, int b2) {
   EncodeTiledFn fn = encode_fn();
   if (!fn) return false;
-  const cuuint64_t dims[5] = {8, (cuuint64_t)n2, (cuuint64_t)n1, (cuuint64_t)n0, (cuuint64_t)(C / 8)};
-  const cuuint64_t strides[4] = {16, (cuuint64_t)n2 * 16, (cuuint64_t)n1 * n2 * 16, (cuuint64_t)n0 * n1 * n2 * 16};
-  const cuuint32_t box[5] = {8, (cuuint32_t)b2, (cuuint32_t)b1, (cuuint32_t)b0, (cuuint32_t)(C / 8)};
-  const cuuint32_t es[5] = {1, 1, 1, 1, 1};
-  return fn(tm, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 5, const_cast<void*>(base), dims, strides, box, es,
+  const cuuint64_t dims[4] = {(cuuint64_t)n2 * 8, (cuuint64_t)n1, (cuuint64_t)n0, (cuuint64_t)(C / 8)};
+  const cuuint64_t strides[3] = {(cuuint64_t)n2 * 16, (cuuint64_t)n1 * n2 * 16, (cuuint64_t)n0 * n1 * n2 * 16};
+  const cuuint32_t box[4] = {(cuuint32_t)b2 * 8, (cuuint32_t)b1, (cuuint32_t)b0, (cuuint32_t)(C / 8)};
+  const cuuint32_t es[4] = {1, 1, 1, 1};
+  return fn(tm, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 4, const_cast<void*>(base), dims, strides, box, es,
             CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
+            CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
+
+// tensor map of packed weights [27 = (a, b, c)][cin/8][npad][8]: a box is one (b, c) as [cin/8][a][npad][8],
+// dims (npad rows of 16 bytes as 8-byte elements: at most 256 of a box side), a, cin/8, (b, c)
+bool make_weight_map(CUtensorMap* tm, const void* base, int kc, int npad) {
+  EncodeTiledFn fn = encode_fn();
+  if (!fn) return false;
+  const cuuint64_t block = (cuuint64_t)npad * 16, tap = block * kc;
+  const cuuint64_t dims[4] = {(cuuint64_t)(npad * 2), 3, (cuuint64_t)kc, 9};
+  const cuuint64_t strides[3] = {9 * tap, block, tap};
+  const cuuint32_t box[4] = {(cuuint32_t)(npad * 2), 3, (cuuint32_t)kc, 1};
+  const cuuint32_t es[4] = {1, 1, 1, 1};
+  return fn(tm, CU_TENSOR_MAP_DATA_TYPE_FLOAT64, 4, const_cast<void*>(base), dims, strides, box, es,
+            CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
             CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
@@ -715,13 +921,6 @@ extern "C" int pfm_nn_conv3(const pfm_conv3_args* a, void* stream) {
   if (!aligned16(a->x1) || (a->x2 && !aligned16(a->x2)) || !aligned16(a->w) || (a->y1 && !aligned16(a->y1)) ||
       (a->y2 && !aligned16(a->y2)))
     return PFM_ERR_ARG;
-  CUtensorMap tm1, tm2;
-  if (!make_map(&tm1, a->x1, a->c1, a->d0, a->d1, a->d2, kBoxD0, kBoxD1, kBoxD2)) return PFM_ERR_CUDA;
-  if (a->c2 > 0) {
-    if (!make_map(&tm2, a->x2, a->c2, a->d0, a->d1, a->d2, kBoxD0, kBoxD1, kBoxD2)) return PFM_ERR_CUDA;
-  } else {
-    tm2 = tm1;
-  }
   ConvFwdParams p{};
   p.n0 = a->d0;
   p.n1 = a->d1;
@@ -732,9 +931,6 @@ extern "C" int pfm_nn_conv3(const pfm_conv3_args* a, void* stream) {
   p.c1 = a->c1;
   p.npad = npad;
   p.cout = a->cout;
-  p.ncols = pow2_cols(npad);
-  p.idesc = idesc_bf16(128, npad);
-  p.w = (const __nv_bfloat16*)a->w;
   p.bias = a->bias;
   p.relu = a->relu;
   p.y1 = (__nv_bfloat16*)a->y1;
@@ -743,19 +939,78 @@ extern "C" int pfm_nn_conv3(const pfm_conv3_args* a, void* stream) {
   p.yf = a->yf;
   p.yf_scale = a->yf_scale;
   p.err = a->err;
-  const size_t box = ((size_t)(cin / 8) * kChunkBytes + 127) & ~(size_t)127;
-  // weight ring of 4 taps: deeper rings (up to all 27 taps) remove refill round trips but cost
-  // shared memory, hence CTAs per SM, and concurrent CTAs are what keeps the tensor core busy
-  const size_t stage = (size_t)npad * cin * 2;
-  p.nstage = kStages;
-  const size_t need = 1024 + box + (size_t)p.nstage * stage + 8 * (2 + 2 * p.nstage) + 16;
+  const size_t wtap = (size_t)(cin / 8) * 3 * npad * 16;
+  const size_t fixed = 1024 + 8 * (2 * kPlaneStages + 2 * kTapStages + 2 * kMaxRing + 1) + 8 + 4 * kMaxNpad;
+  size_t need = 0;
+  // Output planes per CTA, TMEM columns and tiles per CTA by the time they should take, in cycles.  An SM's
+  // tensor core works through the seg + 2 input planes of each of its CTAs (34 + N/2 per MMA; two MMAs where
+  // the planes' columns straddle the ring's end or exceed N = 256), a CTA's issuing warp needs some 1000 +
+  // 60 per MMA, and a CTA's start-up and drain of 9000 are hidden where others share its SM.  Weights that
+  // do not fit beside two planes come from L2 once per plane, at some 19 bytes per cycle and SM; two tiles
+  // share them then.  16 -> 16 at 192^3: 331 us with 16 planes in TMEM and 192 per CTA, 207 with rings of 4,
+  // 169 with the 8 this picks; 96 -> 32 at 96^3: 250 us with one tile per CTA, 162 with two.
+  double best = -1.;
+  for (int mt = 1; mt <= 2; ++mt) {
+    const size_t plane = ((size_t)(cin / 8) * (mt * kTileD1 + 2) * kRowBytes + 127) & ~(size_t)127;
+    int nstage = kPlaneStages, wstage = 9;
+    while (nstage > 2 && fixed + nstage * plane + 9 * wtap > (size_t)kMaxDynSmem) --nstage;
+    if (fixed + nstage * plane + 9 * wtap > (size_t)kMaxDynSmem) {
+      wstage = 8;
+      while (wstage > 1 && fixed + nstage * plane + wstage * wtap > (size_t)kMaxDynSmem) --wstage;
+    }
+    const size_t bytes = fixed + nstage * plane + wstage * wtap;
+    if (bytes > (size_t)kMaxDynSmem || (mt == 2 && (wstage == 9 || tiles1 < 2))) continue;
+    const int per_sm = (int)std::max<size_t>(1, (size_t)kSmPerGpuSmem / (bytes + 1024));
+    const long long tiles = (long long)((tiles1 + mt - 1) / mt) * p.tiles2;
+    for (int cols = 512; cols >= 64; cols >>= 1) {
+      const int fit = std::min(cols / (npad * mt), kMaxRing);
+      const int slots = std::min(per_sm, 512 / cols);
+      if (fit < 1) break;
+      for (int ns = 1, last = 0; ns <= a->d0; ++ns) {
+        const int seg = (a->d0 + ns - 1) / ns;
+        if (seg == last) continue;
+        last = seg;
+        if (seg > fit && fit < 4) continue;
+        const double mmas = 9. * (cin / 16) * mt * (3 * npad > 256 ? 2. : 1.) * (seg > fit ? 1. + 2. / fit : 1.);
+        const double tensor = 34. * mmas + 9. * (cin / 16) * mt * 1.5 * npad;
+        double issue = 1000. + 60. * mmas;
+        if (wstage != 9) issue = std::max(issue + 9. * 200., 9. * wtap / 19.);
+        const double alone = (seg + 2) * std::max(issue, tensor) + 9000.;
+        const double work = (seg + 2) * std::max(issue / slots, tensor);
+        const long long ctas = tiles * ((a->d0 + seg - 1) / seg), waves = ctas / ((long long)kSms * slots);
+        const long long rest = ctas - waves * kSms * slots, share = (rest + kSms - 1) / kSms;
+        const double cost = waves * std::max(alone, slots * work + 1000.) +
+                            (rest ? std::max(alone, share * (seg + 2) * tensor) : 0.);
+        if (best < 0 || cost < best) {
+          best = cost;
+          need = bytes;
+          p.mt = mt;
+          p.nstage = nstage;
+          p.wstage = wstage;
+          p.seg = seg;
+          p.ring = std::min(seg, fit);
+          p.ncols = cols;
+        }
+        if (seg == 1) break;
+      }
+    }
+  }
+  if (best < 0) return PFM_ERR_SHAPE;
+  CUtensorMap tm1, tm2, tmw;
+  if (!make_map(&tm1, a->x1, a->c1, a->d0, a->d1, a->d2, 1, p.mt * kTileD1 + 2, kBoxD2)) return PFM_ERR_CUDA;
+  if (a->c2 > 0) {
+    if (!make_map(&tm2, a->x2, a->c2, a->d0, a->d1, a->d2, 1, p.mt * kTileD1 + 2, kBoxD2)) return PFM_ERR_CUDA;
+  } else {
+    tm2 = tm1;
+  }
+  if (!make_weight_map(&tmw, a->w, cin / 8, npad)) return PFM_ERR_CUDA;
   const size_t smem = occupancy_smem(need, p.ncols);
   if (smem > kMaxDynSmem) return PFM_ERR_SHAPE;
   static std::atomic<unsigned long long> attr{0};  // above the default 48 KB: opt in per device
   if (pfm::opt_in_smem(k_conv3_fwd, kMaxDynSmem, attr) != cudaSuccess) return PFM_ERR_CUDA;
-  dim3 grid((unsigned)(tiles1 * p.tiles2), (unsigned)a->d0);
+  dim3 grid((unsigned)((tiles1 + p.mt - 1) / p.mt * p.tiles2), (unsigned)((a->d0 + p.seg - 1) / p.seg));
   if (grid.y > 65535) return PFM_ERR_SHAPE;
-  k_conv3_fwd<<<grid, kThreads, smem, (cudaStream_t)stream>>>(tm1, tm2, p);
+  k_conv3_fwd<<<grid, kFwdThreads, smem, (cudaStream_t)stream>>>(tm1, tm2, tmw, p);
   return cudaGetLastError() == cudaSuccess ? PFM_OK : PFM_ERR_CUDA;
 }
 
