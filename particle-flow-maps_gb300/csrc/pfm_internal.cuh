@@ -609,4 +609,17 @@ int warm_start_init(pfm_handle* h, float* x, const float* p_io, int mode, cudaSt
 // Counting sort of the particle cells (pfm_p2g.cu).
 int sort_particles(pfm_handle* h, const float* pos, cudaStream_t st);
 
+// Per-thread partial sums of the mixed solve: Neumaier-compensated f32 (each thread adds at most a
+// few hundred terms; the block and grid sums are f64).  Per-element f64 arithmetic would run on
+// GB300's narrow FP64 pipe and cost about 0.1 ms per PCG iteration at 256^3.
+struct CompSum {
+  float s = 0.f, c = 0.f;
+  __device__ __forceinline__ void add(float x) {
+    const float t = s + x;
+    c += (fabsf(s) >= fabsf(x)) ? ((s - t) + x) : ((x - t) + s);
+    s = t;
+  }
+  __device__ __forceinline__ double value() const { return (double)s + (double)c; }
+};
+
 }  // namespace pfm

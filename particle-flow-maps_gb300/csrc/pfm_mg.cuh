@@ -88,19 +88,6 @@ __device__ __forceinline__ void decode(const Lvl& L, int64_t e, int& i, int& j, 
   split3((unsigned)e, L.d1, L.d2, i, j, k);
 }
 
-// Per-thread partial sums of the mixed solve: Neumaier-compensated f32 (each thread adds at most a
-// few hundred terms; the block and grid sums are f64).  Per-element f64 arithmetic would run on
-// GB300's narrow FP64 pipe and cost about 0.1 ms per PCG iteration at 256^3.
-struct CompSum {
-  float s = 0.f, c = 0.f;
-  __device__ __forceinline__ void add(float x) {
-    const float t = s + x;
-    c += (fabsf(s) >= fabsf(x)) ? ((s - t) + x) : ((x - t) + s);
-    s = t;
-  }
-  __device__ __forceinline__ double value() const { return (double)s + (double)c; }
-};
-
 // the stopping rule of k_update_xr / k_true_residual; the relative rules accept an exactly zero
 // residual, so a zero right-hand side (a fluid at rest) ends at the first check
 __device__ __forceinline__ bool converged(double rTr, const SolveState* st, double tol, int tol_mode) {

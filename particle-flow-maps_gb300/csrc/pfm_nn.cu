@@ -15,11 +15,10 @@
 //    kind::f16 BF16 x BF16 -> F32) accumulates in TMEM; four warps read it back with tcgen05.ld for the
 //    epilogue (bias, ReLU, BF16 or F32 store).  The data gradient is the same kernel on the output
 //    gradient with the weights flipped and transposed (k_pack_w).
-//  * Weight gradient (k_conv3_wgrad): D[(tap, ci)][co] = sum over voxels X[v + tap][ci] dY[v][co],
-//    K = voxels.  The operands need voxels along the 16-byte rows, so the CTA transposes 8x8 blocks
-//    of the TMA-loaded brick and output-gradient tile into K-major core matrices in shared memory
-//    (one 128-byte core per thread step), then issues M 128 x N npad x K 16 MMAs; each CTA sums a
-//    strided set of voxel tiles for a group of M tiles and a deterministic reduction sums the CTAs.
+//  * Weight gradient (k_conv3_wgrad): D[(b, co)][(a, ci)] for each c = sum over voxels of
+//    dY[v][co] X[v + tap][ci], K = voxels.  With channels along the 16-byte rows the same layout is an
+//    MN-major operand, so TMA loads feed the MMAs here too; each CTA sums a run of voxel tiles for a group
+//    of input channels and a deterministic reduction sums the CTAs.
 //
 // Every wait (TMA, MMA completion) is bounded by wall time; on expiry the kernel raises a flag in
 // device memory, skips its remaining work, frees its TMEM and returns, and later CTAs see the flag
@@ -39,10 +38,8 @@ namespace pfm {
 namespace nn {
 
 constexpr int kTileD1 = 16, kTileD2 = 8;  // 128 output voxels per CTA
-constexpr int kBoxD0 = 3, kBoxD1 = kTileD1 + 2, kBoxD2 = kTileD2 + 2;
-constexpr int kBoxVox = kBoxD0 * kBoxD1 * kBoxD2;  // 540
-constexpr int kChunkBytes = kBoxVox * 16;          // one 8-channel block of the brick: 8640 B
-constexpr int kRowBytes = kBoxD2 * 16;             // one brick row along d2: 160 B
+constexpr int kBoxD2 = kTileD2 + 2;
+constexpr int kRowBytes = kBoxD2 * 16;  // one row of a tile along d2 with its halo: 160 B
 constexpr int kSms = 152;
 constexpr int kMaxCin = 128, kMaxNpad = 128;
 constexpr int kSmPerGpuSmem = 233472;                  // shared memory per SM (228 KB)
@@ -109,6 +106,24 @@ __device__ __forceinline__ void tmem_zero16(uint32_t taddr) {
   asm volatile(
       "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1, %1, %1, %1, %1, %1, %1, %1, %1, %1, %1, %1, %1, %1, %1, %1};"
       ::"r"(taddr), "r"(0)
+      : "memory");
+}
+
+// a + b of two groups of 16 columns into the second
+__device__ __forceinline__ void tmem_add16(uint32_t ta, uint32_t tb) {
+  float a[16], b[16];
+  asm volatile(
+      "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%32];\n\t"
+      "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31}, [%33];\n\t"
+      "tcgen05.wait::ld.sync.aligned;"
+      : "=f"(a[0]), "=f"(a[1]), "=f"(a[2]), "=f"(a[3]), "=f"(a[4]), "=f"(a[5]), "=f"(a[6]), "=f"(a[7]), "=f"(a[8]), "=f"(a[9]), "=f"(a[10]), "=f"(a[11]), "=f"(a[12]), "=f"(a[13]), "=f"(a[14]), "=f"(a[15]),
+        "=f"(b[0]), "=f"(b[1]), "=f"(b[2]), "=f"(b[3]), "=f"(b[4]), "=f"(b[5]), "=f"(b[6]), "=f"(b[7]), "=f"(b[8]), "=f"(b[9]), "=f"(b[10]), "=f"(b[11]), "=f"(b[12]), "=f"(b[13]), "=f"(b[14]), "=f"(b[15])
+      : "r"(ta), "r"(tb)
+      : "memory");
+#pragma unroll
+  for (int i = 0; i < 16; ++i) b[i] += a[i];
+  asm volatile(
+      "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16};" ::"r"(tb), "f"(b[0]), "f"(b[1]), "f"(b[2]), "f"(b[3]), "f"(b[4]), "f"(b[5]), "f"(b[6]), "f"(b[7]), "f"(b[8]), "f"(b[9]), "f"(b[10]), "f"(b[11]), "f"(b[12]), "f"(b[13]), "f"(b[14]), "f"(b[15])
       : "memory");
 }
 
@@ -449,189 +464,266 @@ __global__ void __launch_bounds__(kFwdThreads) k_conv3_fwd(const __grid_constant
 // ---------------------------------------------------------------------------------------------
 // weight gradient
 
+constexpr int kWgThreads = 192;  // warp 0: TMA, warp 1: MMA, warps 2-5: epilogue
+constexpr int kWgStages = 4;
+constexpr int kXChunk = kTileD1 * kRowBytes;  // one 8-channel block of an X plane (16 rows of 10 voxels): 2,560 B
+
 struct ConvWgradParams {
-  int n0, n1, n2, tiles2, ntiles;  // voxel tiles of 1 x 16 x 8
-  int cin, c1, cdy, npad;          // input channels, dY channels (multiple of 8), MMA N
-  int mtiles, mt_per_cta;          // M tiles of 128 (tap, ci) rows; per CTA group (blockIdx.y)
-  int nabuf;                       // operand buffers for A (2: staging overlaps the MMAs; 1: more CTAs per SM)
-  int ncols;
-  uint32_t idesc;
-  float* partial;  // [gridDim.x][mtiles * 128][npad]
+  int n0, n1, n2;
+  int tiles1, tiles2, steps;  // voxel tiles of 16 x 8 along d1, d2; steps = tiles x groups of P G planes
+  int kc, kc1, dc;            // 8-channel blocks of the input, of x1, and of dY
+  int P, G;                   // d0 planes side by side in M; MMA groups per step
+  int nb;                     // input blocks per CTA (even)
+  int mtiles;                 // M tiles of 128; blockIdx.y = M tile + mtiles * input group
+  int N;                      // (P + 2) nb 8 columns per c
+  int rows;                   // rows of a column of `partial`
+  int flush;                  // steps whose sum moves to a second accumulator at a time (0: all of them stay)
+  int nstage, ncols;
+  uint32_t stage_bytes, dy_pitch;
+  float* partial;  // [split][blockIdx.y][c = 3][N][rows]
   int* err;
 };
 
-// 8x8 transpose of 16-bit elements: in[v] holds 8 channels of voxel v, out[e] 8 voxels of channel e
-__device__ __forceinline__ void transpose8x8(const uint4 (&in)[8], uint4 (&out)[8]) {
-  const uint32_t* w = reinterpret_cast<const uint32_t*>(in);  // w[v * 4 + e / 2]
-#pragma unroll
-  for (int e = 0; e < 8; ++e) {
-    const uint32_t sel = (e & 1) ? 0x7632u : 0x5410u;
-    uint32_t o[4];
-#pragma unroll
-    for (int q = 0; q < 4; ++q) o[q] = __byte_perm(w[(2 * q) * 4 + (e >> 1)], w[(2 * q + 1) * 4 + (e >> 1)], sel);
-    out[e] = make_uint4(o[0], o[1], o[2], o[3]);
-  }
-}
-
-__device__ __forceinline__ void copy_core_T(const unsigned char* src, unsigned char* dst) {
-  uint4 in[8], out[8];
-#pragma unroll
-  for (int v = 0; v < 8; ++v) in[v] = *(const uint4*)(src + 16 * v);
-  transpose8x8(in, out);
-#pragma unroll
-  for (int e = 0; e < 8; ++e) *(uint4*)(dst + 16 * e) = out[e];
-}
-
-constexpr int kCoresA = 16 * 16;           // 16 row groups x 16 voxel groups per M tile
-constexpr int kAbufBytes = kCoresA * 128;  // 32 KB
-
-constexpr int kWgThreads = 256;  // 8 warps stage the operand cores; warps 0-3 also drain TMEM
-
+// D[(s, p, co)][(q, ci)] per c, K = voxels.  Both operands keep channels along their 16-byte rows and voxels
+// as rows (MN-major), just as they lie in memory, so TMA's boxes are the MMA's operands: X as
+// [plane][8-channel block][16 rows][10 voxels], and dY as [18 rows][P planes][block][8 voxels].  The row shift
+// s = 2 - b is a shift of the M groups over dY's rows (a K step of two rows starts 2 P dc groups further), the
+// d0 offset a = q - p comes from the planes side by side in N (and, where dY has few channels, in M), and c
+// is a start address in X: a step of P planes of 128 voxels takes 3 c x 8 MMAs for all 27 taps.  X rows
+// belong to one tile and dY's are loaded with a halo row on each side; X planes and columns the other way round.
+// A CTA adds up a run of steps for one group of input channels; the splits are summed with compensation.
+// Bound by the tensor core's reading of A, some 34 + N/2 cycles per MMA.  With its reduction, 16 -> 16 at 96^3
+// 423 -> 35 us, 48 -> 16 at 96^3 1054 -> 71, 96 -> 32 at 48^3 474 -> 57 (operands transposed into shared memory by
+// eight warps before, 592 splits added up by one thread per weight).
 __global__ void __launch_bounds__(kWgThreads) k_conv3_wgrad(const __grid_constant__ CUtensorMap tm1,
                                                           const __grid_constant__ CUtensorMap tm2,
                                                           const __grid_constant__ CUtensorMap tmdy,
                                                           const ConvWgradParams p) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   unsigned char* smem = (unsigned char*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  __shared__ int s_skip;
-  if (tid == 0) s_skip = *(volatile int*)p.err;
-  __syncthreads();
-  if (s_skip) return;
+  const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;
+  const uint32_t x_plane = (uint32_t)p.nb * kXChunk;
+  const int planes = p.P * p.G + 2;
+  uint64_t* full = (uint64_t*)(smem + (size_t)p.nstage * p.stage_bytes);
+  uint64_t *empty = full + kWgStages, *fin = empty + kWgStages, *moved = fin + 1;
+  uint32_t* slot = (uint32_t*)(moved + 1);
+  int* skip = (int*)(slot + 1);
 
-  const int nchunk = p.cin >> 3, dchunk = p.cdy >> 3, ngrp = p.npad >> 3;
-  const uint32_t box_bytes = (uint32_t)nchunk * kChunkBytes;
-  const uint32_t dy_bytes = (uint32_t)dchunk * 2048;
-  unsigned char* box = smem;
-  unsigned char* dybox = box + ((box_bytes + 127) & ~127u);
-  unsigned char* bcore = dybox + dy_bytes;           // [16 voxel groups][npad/8][128 B]
-  unsigned char* abuf = bcore + (size_t)p.npad * 256;  // nabuf x [16 voxel groups][16 row groups][128 B]
-  uint64_t* bars = (uint64_t*)(abuf + p.nabuf * kAbufBytes);
-  uint64_t* box_bar = bars;
-  uint64_t* done = bars + 1;  // [2], one per A buffer
-  uint64_t* final_bar = bars + 3;
-  uint32_t* slot = (uint32_t*)(bars + 4);
+  const int mtile = blockIdx.y % p.mtiles, cb = (int)(blockIdx.y / p.mtiles) * p.nb;
+  const int nblk = min(p.nb, p.kc - cb);
+  const int s0 = (int)((long long)blockIdx.x * p.steps / gridDim.x);
+  const int s1 = (int)((long long)(blockIdx.x + 1) * p.steps / gridDim.x);
 
-  const int mt0 = blockIdx.y * p.mt_per_cta;
-  const int nmt = min(p.mt_per_cta, p.mtiles - mt0);
-
-  if (tid == 0) {
-    mbar_init(box_bar, 1);
-    mbar_init(done, 1);
-    mbar_init(done + 1, 1);
-    mbar_init(final_bar, 1);
+  if (warp == 0) {
+    if (lane < kWgStages) {
+      mbar_init(full + lane, 1);
+      mbar_init(empty + lane, 1);
+    } else if (lane == 31) {
+      mbar_init(fin, 1);
+      mbar_init(moved, 128);
+      *skip = *(volatile int*)p.err;
+    }
     fence_mbar_init();
+  } else if (warp == 1) {
+    tmem_alloc(slot, (uint32_t)p.ncols);
+  } else if (warp == 2 && lane == 0) {
+    prefetch_map(&tm1);
+    prefetch_map(&tmdy);
+    if (p.kc > p.kc1) prefetch_map(&tm2);
   }
-  // B groups beyond the dY channels stay zero
-  for (int i = tid; i < p.npad * 16; i += blockDim.x) ((uint4*)bcore)[i] = make_uint4(0, 0, 0, 0);
-  if (warp == 0) tmem_alloc(slot, (uint32_t)p.ncols);
-  fence_proxy_async();
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem = *slot;
-
-  bool ok = true;
-  bool first = true;
-  unsigned box_phase = 0;
-  int uses[2] = {0, 0};
-  int last = -1;  // A buffer of the last commit
-  const uint32_t idesc = p.idesc;
-  const uint32_t blbo = (uint32_t)ngrp * 128;
-  for (int tile = blockIdx.x; tile < p.ntiles && ok; tile += gridDim.x) {
-    const int pl = tile / ((p.n1 + kTileD1 - 1) / kTileD1 * p.tiles2);
-    const int r = tile - pl * ((p.n1 + kTileD1 - 1) / kTileD1 * p.tiles2);
-    const int t1 = r / p.tiles2, t2 = r - t1 * p.tiles2;
-    const int z = pl, y0 = t1 * kTileD1, x0 = t2 * kTileD2;
-    if (tid == 0) {
-      fence_proxy_async();
-      mbar_expect_tx(box_bar, box_bytes + dy_bytes);
-      tma_load_4d(box, &tm1, 8 * (x0 - 1), y0 - 1, z - 1, 0, box_bar);
-      if (p.cin > p.c1) tma_load_4d(box + (size_t)(p.c1 >> 3) * kChunkBytes, &tm2, 8 * (x0 - 1), y0 - 1, z - 1, 0, box_bar);
-      tma_load_4d(dybox, &tmdy, 8 * x0, y0, z, 0, box_bar);
-    }
-    bool w = mbar_wait(box_bar, box_phase, p.err, 11);
-    box_phase ^= 1;
-    // the previous tile's MMAs read bcore: wait for the last of them before restaging it
-    if (w && last >= 0) w = mbar_wait(done + last, (uses[last] - 1) & 1, p.err, 12);
-    ok = __syncthreads_and(w) != 0;  // every thread takes the same path through the barriers below
-    if (!ok) break;
-    for (int i = tid; i < dchunk * 16; i += blockDim.x) {  // B core (channel group g, voxel group k)
-      const int g = i % dchunk, k = i / dchunk;
-      copy_core_T(dybox + g * 2048 + k * 128, bcore + k * blbo + g * 128);
-    }
-    for (int mi = 0; mi < nmt && ok; ++mi) {
-      const int buf = p.nabuf == 2 ? ((uses[0] + uses[1]) & 1) : 0;
-      bool wb = true;
-      if (uses[buf] > 0) wb = mbar_wait(done + buf, (uses[buf] - 1) & 1, p.err, 13);
-      ok = __syncthreads_and(wb) != 0;
-      if (!ok) break;
-      unsigned char* A = abuf + buf * kAbufBytes;
-      for (int i = tid; i < kCoresA; i += blockDim.x) {  // A core (row group g, voxel group k)
-        const int g = i & 15, k = i >> 4;
-        const int G = (mt0 + mi) * 16 + g;
-        const int tap = G / nchunk, ch = G - tap * nchunk;
-        unsigned char* dst = A + k * 2048 + g * 128;
-        if (tap < 27) {
-          const int a = tap / 9, b = (tap / 3) % 3, c = tap % 3;
-          copy_core_T(box + (size_t)ch * kChunkBytes + ((a * kBoxD1 + k + b) * kBoxD2 + c) * 16, dst);
-        } else {
-#pragma unroll
-          for (int e = 0; e < 8; ++e) *(uint4*)(dst + 16 * e) = make_uint4(0, 0, 0, 0);
-        }
-      }
-      fence_proxy_async();
-      tc_fence_before();
-      __syncthreads();
-      tc_fence_after();
-      if (tid == 0) {
-        const uint32_t a_addr = su32(A), b_addr = su32(bcore);
-        for (int kk = 0; kk < 8; ++kk) {
-          const uint64_t ad = smem_desc(a_addr + (uint32_t)(2 * kk) * 2048, 2048, 128);
-          const uint64_t bd = smem_desc(b_addr + (uint32_t)(2 * kk) * blbo, blbo, 128);
-          mma_bf16(tmem + (uint32_t)(mi * p.npad), ad, bd, idesc, !(first && kk == 0));
-        }
-        mma_commit(done + buf);
-      }
-      uses[buf]++;
-      last = buf;
-    }
-    first = false;
-    __syncthreads();  // the brick and dY tile are consumed: the next TMA may overwrite them
+  if (*skip) {  // an earlier CTA gave up: do nothing (uniform over the CTA)
+    if (warp == 1) tmem_dealloc(tmem, (uint32_t)p.ncols);
+    return;
   }
-  if (tid == 0) mma_commit(final_bar);
-  const bool fin = mbar_wait(final_bar, 0, p.err, 14);
-  tc_fence_after();
 
-  const int rows = p.mtiles * 128;
-  for (int mi = 0; mi < nmt && warp < 4; ++mi) {  // TMEM lanes 32w..32w+31 belong to warp w % 4
-    for (int c0 = 0; c0 < p.npad; c0 += 16) {
-      float v[16];
-      tmem_ld16(tmem + ((uint32_t)(warp * 32) << 16) + (uint32_t)(mi * p.npad + c0), v);
-      if (!fin) continue;
-      const int R = (mt0 + mi) * 128 + warp * 32 + lane;
-      float* dst = p.partial + ((size_t)blockIdx.x * rows + R) * p.npad + c0;
+  if (warp == 0) {
+    if (lane == 0) {
+      bool ok = true;
+      const uint32_t bytes = (uint32_t)planes * (uint32_t)nblk * kXChunk + (uint32_t)(p.G * p.P * p.dc) * 18u * 128u;
+      const int tiles = p.tiles1 * p.tiles2;
+      int i = 0;
+      for (; i < s1 - s0; ++i) {
+        const int s = i % p.nstage;
+        if (i >= p.nstage) ok = mbar_wait(empty + s, (unsigned)(i / p.nstage - 1) & 1u, p.err, 11);
+        if (!ok) break;
+        // steps run along d0 within a tile, so that a CTA's X planes are read again while they are in L2
+        const int zsteps = p.steps / tiles, tile = (s0 + i) / zsteps, z0 = (s0 + i - tile * zsteps) * p.P * p.G;
+        const int t1 = tile / p.tiles2, y0 = t1 * kTileD1, x0 = (tile - t1 * p.tiles2) * kTileD2;
+        unsigned char* dst = smem + (size_t)s * p.stage_bytes;
+        mbar_expect_tx(full + s, bytes);
+        for (int g = 0; g < p.G; ++g)
+          tma_load_4d(dst + (size_t)g * p.dy_pitch, &tmdy, 8 * x0, 0, z0 + g * p.P, y0 - 1, full + s);
+        dst += (size_t)p.G * p.dy_pitch;
+        for (int q = 0; q < planes; ++q)
+          for (int b = 0; b < nblk; b += 2) {
+            const int k = cb + b;
+            tma_load_4d(dst + (size_t)q * x_plane + (size_t)b * kXChunk, k < p.kc1 ? &tm1 : &tm2, 8 * (x0 - 1), y0,
+                        k < p.kc1 ? k : k - p.kc1, z0 + q - 1, full + s);
+          }
+      }
+      if (*(volatile int*)p.err != 0)  // giving up: the copies in flight land before this memory is given back
+        for (int q = max(0, i - p.nstage); q < i; ++q) mbar_drain(full + q % p.nstage, (unsigned)(q / p.nstage) & 1u);
+    }
+  } else if (warp == 1) {
+    const bool lead = elect_one();
+    bool ok = true;
+    int s = 0;
+    unsigned phase = 0;
+    const uint32_t group = (uint32_t)(p.P * p.dc) * 128u;  // one dY row
+    const uint64_t a0 = smem_desc(su32(smem), group, 128) + (uint32_t)mtile * 128u;
+    const uint64_t b0 = smem_desc(su32(smem) + (uint32_t)p.G * p.dy_pitch, kRowBytes, kXChunk);
+    const uint32_t a_k = 2 * group / 16, b_k = 2 * kRowBytes / 16;
+    const uint32_t id = idesc_bf16(128, p.N) | (1u << 15) | (1u << 16);  // both operands MN-major
+    const uint32_t d1 = tmem + (uint32_t)p.N, d2 = d1 + (uint32_t)p.N;
+    bool has = false;
+    int run = 0;  // steps in the accumulator
+    unsigned mphase = 0;
+    for (int i = 0; i < s1 - s0; ++i) {
+      if (!has) ok = mbar_wait(full + s, phase, p.err, 12);
+      if (p.flush && run == p.flush) {
+        if (lead) mma_commit(fin);
+        ok = ok && mbar_wait(moved, mphase, p.err, 14);
+        mphase ^= 1u;
+        run = 0;
+      }
+      ok = __all_sync(0xffffffffu, ok);
+      if (!ok) break;
+      tc_fence_after();
+      const int sn = s + 1 == p.nstage ? 0 : s + 1;
+      const unsigned phase1 = phase ^ (sn == 0);
+      has = mbar_test(full + sn, phase1);
+      uint64_t ad = a0 + (uint32_t)s * (p.stage_bytes / 16), bd = b0 + (uint32_t)s * (p.stage_bytes / 16);
+      for (int g = 0; g < p.G; ++g) {
+        const uint32_t acc = run > 0 || g > 0;
+        if (lead) {
+          mma_bf16(tmem, ad, bd, id, acc);
+          mma_bf16(d1, ad, bd + 1u, id, acc);
+          mma_bf16(d2, ad, bd + 2u, id, acc);
 #pragma unroll
-      for (int e = 0; e < 16; e += 4)
-        *(float4*)(dst + e) = first ? make_float4(0.f, 0.f, 0.f, 0.f) : make_float4(v[e], v[e + 1], v[e + 2], v[e + 3]);
+          for (int k = 1; k < 8; ++k) {
+            const uint64_t ak = ad + (uint32_t)k * a_k, bk = bd + (uint32_t)k * b_k;
+            mma_bf16(tmem, ak, bk, id, 1u);
+            mma_bf16(d1, ak, bk + 1u, id, 1u);
+            mma_bf16(d2, ak, bk + 2u, id, 1u);
+          }
+        }
+        ad += p.dy_pitch / 16;
+        bd += (uint32_t)p.P * (x_plane / 16);
+      }
+      if (lead) mma_commit(empty + s);
+      __syncwarp();
+      ++run;
+      s = sn;
+      phase = phase1;
+    }
+    if (lead) mma_commit(fin);
+    if (*(volatile int*)p.err != 0) mbar_drain(fin, mphase);  // giving up: what was issued ends before its operands go
+    __syncwarp();
+  } else {
+    const int m = (warp & 3) * 32 + lane, grp = mtile * 16 + (m >> 3);
+    const int pl = grp / p.dc % p.P;
+    const bool used = grp < 3 * p.P * p.dc;
+    const uint32_t lanes = tmem + ((uint32_t)((warp & 3) * 32) << 16);
+    float* out = p.partial + ((size_t)blockIdx.x * gridDim.y + blockIdx.y) * 3 * p.N * p.rows + m;
+    const int moves = p.flush ? (s1 - s0 - 1) / p.flush : 0;
+    const uint32_t sums = moves ? 3u * (uint32_t)p.N : 0u;  // columns of the second accumulator
+    bool ok = true;
+    if (moves)
+      for (int c0 = 0; c0 < 3 * p.N; c0 += 16) tmem_zero16(lanes + sums + (uint32_t)c0);
+    for (int f = 0; f < moves && ok; ++f) {
+      ok = mbar_wait(fin, (unsigned)f & 1u, p.err, 13);
+      ok = __all_sync(0xffffffffu, ok);
+      if (!ok) break;
+      tmem_st_wait();
+      tc_fence_after();
+      for (int c0 = 0; c0 < 3 * p.N; c0 += 16) tmem_add16(lanes + (uint32_t)c0, lanes + sums + (uint32_t)c0);
+      tmem_st_wait();
+      tc_fence_before();
+      mbar_arrive(moved);
+    }
+    ok = ok && mbar_wait(fin, (unsigned)moves & 1u, p.err, 13);
+    if (__all_sync(0xffffffffu, ok)) {
+      tc_fence_after();
+      for (int c0 = 0; c0 < 3 * p.N; c0 += 16) {
+        float v[16];
+        if (moves) {
+          tmem_add16(lanes + (uint32_t)c0, lanes + sums + (uint32_t)c0);
+          tmem_st_wait();
+        }
+        tmem_ld16(lanes + sums + (uint32_t)c0, v);
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+          const int blk = (c0 % p.N >> 3) + h, a = blk / p.nb - pl;
+          if (used && a >= 0 && a <= 2 && blk % p.nb < nblk)
+#pragma unroll
+            for (int e = 0; e < 8; ++e) out[(size_t)(c0 + 8 * h + e) * p.rows] = v[8 * h + e];
+        }
+      }
     }
   }
   tc_fence_before();
   __syncthreads();
-  if (warp == 0) tmem_dealloc(tmem, (uint32_t)p.ncols);
+  if (warp == 1) tmem_dealloc(tmem, (uint32_t)p.ncols);
 }
 
-// dW[co][ci][tap] = sum over splits of partial[split][tap * cin + ci][co] (fixed order)
-__global__ void k_wgrad_reduce(const float* __restrict__ partial, int splits, int rows, int npad, int cin, int cout,
-                               float* __restrict__ dw) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  const int total = cout * cin * 27;
-  if (i >= total) return;
-  const int tap = i % 27, ci = (i / 27) % cin, co = i / (27 * cin);
-  const size_t R = (size_t)tap * cin + ci;
-  float s = 0.f;
-  for (int k = 0; k < splits; ++k) s += partial[((size_t)k * rows + R) * npad + co];
-  dw[i] = s;
+// dw[co][ci][(a, b, c)] = sum over splits and planes p of their partial sums, compensated and in a fixed order.
+// A block holds 32 rows (s, co) of one (c, a, ci): 8 lanes of a warp four rows each, its quarters and the block's
+// warps different splits, so that a warp's load is four lines of 128 bytes.
+constexpr int kWrWarps = 8;
+
+__global__ void __launch_bounds__(32 * kWrWarps) k_wgrad_reduce(const ConvWgradParams p, int splits, int gy, int cout,
+                                                                float* __restrict__ dw) {
+  __shared__ float sh[kWrWarps][8][8];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, warps = blockDim.x >> 5;
+  const int cdy = p.dc * 8, i = blockIdx.x * 32 + (lane & 7) * 4;
+  const bool in = i < 3 * cdy;
+  const int s = i / cdy, co = i - s * cdy, ci = blockIdx.y, cin = gridDim.y;
+  const int c = blockIdx.z / 3, a = blockIdx.z - 3 * c;
+  CompSum sum[4];
+  if (in && co < cout) {
+    const int blk = ci >> 3, y0 = p.mtiles * (blk / p.nb);
+    const size_t pitch = (size_t)gy * 3 * p.N * p.rows;
+    for (int q = 0; q < p.P; ++q) {
+      const int row = (s * p.P + q) * cdy + co, col = ((a + q) * p.nb + blk % p.nb) * 8 + (ci & 7);
+      const float* src = p.partial + (((size_t)(y0 + (row >> 7)) * 3 + c) * p.N + col) * p.rows + (row & 127);
+#pragma unroll 4
+      for (int k = warp * 4 + (lane >> 3); k < splits; k += 4 * warps) {
+        const float4 v = *(const float4*)(src + (size_t)k * pitch);
+        sum[0].add(v.x);
+        sum[1].add(v.y);
+        sum[2].add(v.z);
+        sum[3].add(v.w);
+      }
+    }
+  }
+#pragma unroll
+  for (int e = 0; e < 4; ++e)
+#pragma unroll
+    for (int o = 8; o <= 16; o *= 2) {
+      const float hi = __shfl_xor_sync(0xffffffffu, sum[e].s, o), lo = __shfl_xor_sync(0xffffffffu, sum[e].c, o);
+      sum[e].add(hi);
+      sum[e].c += lo;
+    }
+  if (lane < 8)
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+      sh[warp][lane][2 * e] = sum[e].s;
+      sh[warp][lane][2 * e + 1] = sum[e].c;
+    }
+  __syncthreads();
+  if (threadIdx.x < 32) {
+    const int r = blockIdx.x * 32 + lane, sr = r / cdy, cr = r - sr * cdy;
+    CompSum v;
+    for (int k = 0; k < warps; ++k) {
+      v.add(sh[k][lane >> 2][2 * (lane & 3)]);
+      v.c += sh[k][lane >> 2][2 * (lane & 3) + 1];
+    }
+    if (r < 3 * cdy && cr < cout) dw[((size_t)cr * cin + ci) * 27 + a * 9 + (2 - sr) * 3 + c] = v.s + v.c;
+  }
 }
 
 // ---------------------------------------------------------------------------------------------
@@ -898,6 +990,112 @@ size_t occupancy_smem(size_t need, int ncols) {
 
 bool aligned16(const void* p) { return ((uintptr_t)p & 15u) == 0; }
 
+struct WgradPlan {
+  ConvWgradParams p;
+  int gx, gy;
+  size_t smem;
+};
+
+// Planes side by side in M until its 128 rows are used (16 channels: 3 s x 2 planes x 16), two MMA groups per
+// step (X planes are then read (2 P + 2) / 2 P times instead of (P + 2) / P), and as many input channels per CTA
+// as cost least: an MMA takes some 34 + N/2 cycles.  All are cut back until two stages fit.
+bool wgrad_plan(const pfm_conv3_wgrad_args* a, WgradPlan* w) {
+  ConvWgradParams& p = w->p;
+  p = ConvWgradParams{};
+  p.n0 = a->d0;
+  p.n1 = a->d1;
+  p.n2 = a->d2;
+  p.tiles1 = (a->d1 + kTileD1 - 1) / kTileD1;
+  p.tiles2 = (a->d2 + kTileD2 - 1) / kTileD2;
+  p.kc = (a->c1 + a->c2) / 8;
+  p.kc1 = a->c1 / 8;
+  p.dc = a->cdy / 8;
+  p.P = std::max(1, 4 / p.dc);
+  const int groups = 3 * p.P * p.dc;
+  p.mtiles = (groups + 15) / 16;
+  p.rows = std::min(128, groups * 8);
+  p.dy_pitch = (uint32_t)std::max(15 * p.P * p.dc + 16 * p.mtiles, 18 * p.P * p.dc) * 128u;
+  const size_t fixed = 1024 + 8 * (2 * kWgStages + 2) + 8;
+  double best = -1.;
+  for (int nb = 2; nb <= 6; nb += 2) {
+    const int N = (p.P + 2) * nb * 8;
+    if (3 * N > 512) continue;
+    int G = 2;
+    size_t stage = 0;
+    for (; G >= 1; --G) {
+      stage = (size_t)G * p.dy_pitch + (size_t)(p.P * G + 2) * nb * kXChunk;
+      if (fixed + 2 * stage <= (size_t)kMaxDynSmem) break;
+    }
+    if (G == 0) continue;
+    // a tenth more where TMEM has no room for a second accumulator (below)
+    const double cost = (p.kc + nb - 1) / nb * (34. + N / 2.) * (6 * N > 512 ? 1.1 : 1.);
+    if (best < 0 || cost < best) {
+      best = cost;
+      p.nb = nb;
+      p.N = N;
+      p.G = G;
+      p.stage_bytes = (uint32_t)stage;
+    }
+  }
+  if (best < 0) return false;
+  const long long steps = (long long)p.tiles1 * p.tiles2 * ((a->d0 + p.P * p.G - 1) / (p.P * p.G));
+  if (steps > 0x7fffffff) return false;
+  p.steps = (int)steps;
+  w->gy = p.mtiles * ((p.kc + p.nb - 1) / p.nb);
+  // The tensor core rounds its sums towards zero, so their error grows with the number of K steps (16 -> 16 at
+  // 192^3: 7.0e-6 of dW after 736).  A sum is kept to a 640th of the grid's K steps (fewer parts of layers with
+  // many weights), or 48: where TMEM has room its sum then moves to a second accumulator (16 -> 16 at 192^3:
+  // 137 us against 169 with the partial sums of 608 CTAs), else more CTAs share the steps.
+  const long long weights = 27ll * 8 * p.kc * a->cdy, share = 640 / ((weights + 32767) / 32768);
+  const long long chain = std::max<long long>(48, (long long)a->d0 * a->d1 * a->d2 / 16 / share) / (8 * p.G);
+  int per = 1;
+  for (int two = 0; two < 2; ++two) {
+    p.ncols = pow2_cols((two ? 6 : 3) * p.N);
+    const int slots = std::max(1, std::min(512 / p.ncols, (int)((size_t)kSmPerGpuSmem / (fixed + 2 * p.stage_bytes + 1024))));
+    // stages: up to four where they leave as many CTAs on an SM as TMEM allows
+    p.nstage = 2;
+    while (p.nstage < kWgStages && fixed + (p.nstage + 1) * (size_t)p.stage_bytes <= (size_t)kMaxDynSmem &&
+           slots * (fixed + (p.nstage + 1) * (size_t)p.stage_bytes + 1024) <= (size_t)kSmPerGpuSmem)
+      ++p.nstage;
+    w->smem = occupancy_smem(fixed + p.nstage * (size_t)p.stage_bytes, p.ncols);
+    if (w->smem > (size_t)kMaxDynSmem) return false;
+    p.flush = two ? (int)chain : 0;
+    for (int wave = 1;; ++wave) {
+      const long long want = std::max(1, wave * kSms * slots / w->gy);
+      per = (int)((steps + want - 1) / want);
+      if (per == 1 || per <= chain || two) break;
+      if (6 * p.N <= 512) break;
+    }
+    if (per <= chain || 6 * p.N > 512) break;
+  }
+  w->gx = (p.steps + per - 1) / per;
+  return true;
+}
+
+// tensor maps of a channel-blocked bf16 tensor for the weight gradient: X with dims (8 n2, n1, C/8, n0), box one
+// plane of 16 channels; dY with dims (8 n2, C/8, n0, n1), box P planes of 18 rows of 8 voxels
+bool make_wgrad_map(CUtensorMap* tm, const void* base, int C, int n0, int n1, int n2, int P) {
+  EncodeTiledFn fn = encode_fn();
+  if (!fn) return false;
+  const cuuint64_t row = (cuuint64_t)n2 * 16, plane = (cuuint64_t)n1 * row, chunk = (cuuint64_t)n0 * plane;
+  const bool dy = P > 0;
+  const cuuint64_t dims[4] = {(cuuint64_t)n2 * 8, (cuuint64_t)(dy ? C / 8 : n1), (cuuint64_t)(dy ? n0 : C / 8),
+                              (cuuint64_t)(dy ? n1 : n0)};
+  const cuuint64_t strides[3] = {dy ? chunk : row, dy ? plane : chunk, dy ? row : plane};
+  const cuuint32_t box[4] = {(cuuint32_t)(dy ? 64 : 8 * kBoxD2), (cuuint32_t)(dy ? C / 8 : kTileD1),
+                             (cuuint32_t)(dy ? P : 2), (cuuint32_t)(dy ? kTileD1 + 2 : 1)};
+  const cuuint32_t es[4] = {1, 1, 1, 1};
+  return fn(tm, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 4, const_cast<void*>(base), dims, strides, box, es,
+            CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
+            CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
+
+bool wgrad_shape_ok(const pfm_conv3_wgrad_args* a) {
+  const int cin = a->c1 + a->c2;
+  return a->c1 > 0 && a->c1 % 16 == 0 && a->c2 >= 0 && a->c2 % 16 == 0 && cin <= kMaxCin && a->cdy > 0 &&
+         a->cdy % 8 == 0 && a->cdy <= kMaxNpad;
+}
+
 }  // namespace nn
 }  // namespace pfm
 
@@ -1016,68 +1214,43 @@ extern "C" int pfm_nn_conv3(const pfm_conv3_args* a, void* stream) {
 
 extern "C" int pfm_nn_wgrad_workspace(const pfm_conv3_wgrad_args* a, size_t* bytes) {
   if (!a || !bytes) return PFM_ERR_NULL;
-  const int cin = a->c1 + a->c2;
-  const int npad = (a->cdy + 15) / 16 * 16;
-  const int mtiles = (27 * cin + 127) / 128;
-  const int mt_per = std::min(mtiles, std::max(1, 256 / std::max(npad, 16)));
-  const int gy = (mtiles + mt_per - 1) / mt_per;
-  const long long ntiles = (long long)a->d0 * ((a->d1 + kTileD1 - 1) / kTileD1) * ((a->d2 + kTileD2 - 1) / kTileD2);
-  const long long gx = std::min<long long>(ntiles, std::max(1, (4 * 148 + gy - 1) / gy));
-  *bytes = (size_t)gx * mtiles * 128 * npad * sizeof(float);
+  WgradPlan w;
+  *bytes = 0;  // of a shape that pfm_nn_conv3_wgrad refuses
+  if (grid_ok(a->d0, a->d1, a->d2) && wgrad_shape_ok(a) && wgrad_plan(a, &w))
+    *bytes = (size_t)w.gx * w.gy * 3 * w.p.N * w.p.rows * sizeof(float);
   return PFM_OK;
 }
 
 extern "C" int pfm_nn_conv3_wgrad(const pfm_conv3_wgrad_args* a, void* stream) {
   if (!a || !a->x1 || !a->dy || !a->dw || !a->partial || !a->err) return PFM_ERR_NULL;
   if (!grid_ok(a->d0, a->d1, a->d2)) return PFM_ERR_SHAPE;
-  const int cin = a->c1 + a->c2;
-  if (a->c1 <= 0 || a->c1 % 16 || a->c2 < 0 || a->c2 % 16 || cin > kMaxCin || (a->c2 > 0 && !a->x2)) return PFM_ERR_SHAPE;
-  if (a->cdy <= 0 || a->cdy % 8 || a->cdy > kMaxNpad || a->cout <= 0 || a->cout > a->cdy) return PFM_ERR_SHAPE;
+  if (!wgrad_shape_ok(a) || (a->c2 > 0 && !a->x2)) return PFM_ERR_SHAPE;
+  if (a->cout <= 0 || a->cout > a->cdy) return PFM_ERR_SHAPE;
   if (!aligned16(a->x1) || (a->x2 && !aligned16(a->x2)) || !aligned16(a->dy) || !aligned16(a->partial))
     return PFM_ERR_ARG;
-  const int npad = (a->cdy + 15) / 16 * 16;
-  CUtensorMap tm1, tm2, tmdy;
-  if (!make_map(&tm1, a->x1, a->c1, a->d0, a->d1, a->d2, kBoxD0, kBoxD1, kBoxD2)) return PFM_ERR_CUDA;
-  if (a->c2 > 0) {
-    if (!make_map(&tm2, a->x2, a->c2, a->d0, a->d1, a->d2, kBoxD0, kBoxD1, kBoxD2)) return PFM_ERR_CUDA;
-  } else {
-    tm2 = tm1;
-  }
-  if (!make_map(&tmdy, a->dy, a->cdy, a->d0, a->d1, a->d2, 1, kTileD1, kTileD2)) return PFM_ERR_CUDA;
-  ConvWgradParams p{};
-  p.n0 = a->d0;
-  p.n1 = a->d1;
-  p.n2 = a->d2;
-  p.tiles2 = (a->d2 + kTileD2 - 1) / kTileD2;
-  p.ntiles = a->d0 * ((a->d1 + kTileD1 - 1) / kTileD1) * p.tiles2;
-  p.cin = cin;
-  p.c1 = a->c1;
-  p.cdy = a->cdy;
-  p.npad = npad;
-  p.mtiles = (27 * cin + 127) / 128;
-  p.mt_per_cta = std::min(p.mtiles, std::max(1, 256 / npad));
-  p.ncols = pow2_cols(p.mt_per_cta * npad);
-  p.idesc = idesc_bf16(128, npad);
-  p.partial = a->partial;
-  p.err = a->err;
-  const int gy = (p.mtiles + p.mt_per_cta - 1) / p.mt_per_cta;
-  const int gx = std::min(p.ntiles, std::max(1, (4 * 148 + gy - 1) / gy));
+  WgradPlan w;
+  if (!wgrad_plan(a, &w)) return PFM_ERR_SHAPE;
   size_t ws = 0;
   pfm_nn_wgrad_workspace(a, &ws);
   if (a->partial_bytes < ws) return PFM_ERR_WORKSPACE;
-  const size_t box = ((size_t)(cin / 8) * kChunkBytes + 127) & ~(size_t)127;
-  const size_t base = 1024 + box + (size_t)(a->cdy / 8) * 2048 + (size_t)npad * 256 + 8 * 4 + 16;
-  // one A buffer when that lets two CTAs share an SM (their stagings then overlap each other)
-  p.nabuf = (2 * (base + 2 * kAbufBytes + 1024) > (size_t)kSmPerGpuSmem && 2 * (base + kAbufBytes + 1024) <= (size_t)kSmPerGpuSmem) ? 1 : 2;
-  const size_t need = base + (size_t)p.nabuf * kAbufBytes;
-  const size_t smem = occupancy_smem(need, p.ncols);
-  if (smem > kMaxDynSmem) return PFM_ERR_SHAPE;
+  CUtensorMap tm1, tm2, tmdy;
+  if (!make_wgrad_map(&tm1, a->x1, a->c1, a->d0, a->d1, a->d2, 0)) return PFM_ERR_CUDA;
+  if (a->c2 > 0) {
+    if (!make_wgrad_map(&tm2, a->x2, a->c2, a->d0, a->d1, a->d2, 0)) return PFM_ERR_CUDA;
+  } else {
+    tm2 = tm1;
+  }
+  if (!make_wgrad_map(&tmdy, a->dy, a->cdy, a->d0, a->d1, a->d2, w.p.P)) return PFM_ERR_CUDA;
+  w.p.partial = a->partial;
+  w.p.err = a->err;
   static std::atomic<unsigned long long> attr{0};  // above the default 48 KB: opt in per device
   if (pfm::opt_in_smem(k_conv3_wgrad, kMaxDynSmem, attr) != cudaSuccess) return PFM_ERR_CUDA;
   cudaStream_t st = (cudaStream_t)stream;
-  k_conv3_wgrad<<<dim3((unsigned)gx, (unsigned)gy), kWgThreads, smem, st>>>(tm1, tm2, tmdy, p);
-  const int total = a->cout * cin * 27;
-  k_wgrad_reduce<<<(total + 255) / 256, 256, 0, st>>>(a->partial, gx, p.mtiles * 128, npad, cin, a->cout, a->dw);
+  k_conv3_wgrad<<<dim3((unsigned)w.gx, (unsigned)w.gy), kWgThreads, w.smem, st>>>(tm1, tm2, tmdy, w.p);
+  int warps = 1;  // some eight loads per thread
+  while (warps < kWrWarps && warps * 32 < w.gx * w.p.P) warps *= 2;
+  const dim3 rgrid((unsigned)(3 * a->cdy + 31) / 32, (unsigned)(a->c1 + a->c2), 9);
+  k_wgrad_reduce<<<rgrid, 32 * warps, 0, st>>>(w.p, w.gx, w.gy, a->cout, a->dw);
   return cudaGetLastError() == cudaSuccess ? PFM_OK : PFM_ERR_CUDA;
 }
 
