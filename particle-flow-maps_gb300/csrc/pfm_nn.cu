@@ -781,46 +781,52 @@ __device__ __forceinline__ uint4 pack8(const float (&f)[8]) {
 }
 
 // 2x2x2 average pool (mode 0), its backward (mode 1: dx[v] = dy[v / 2] / 8), nearest upsampling
-// (mode 2: y[v] = x[v / 2]) and its backward (mode 3: dx[V] = sum of the 8 children), one
-// 8-channel block of one fine voxel (modes 1, 2) or one coarse voxel (modes 0, 3) per thread.
-__global__ void k_resample(const __nv_bfloat16* __restrict__ in, __nv_bfloat16* __restrict__ out, int chunks, int n0,
-                           int n1, int n2, int mode) {
+// (mode 2: y[v] = x[v / 2]) and its backward (mode 3: dx[V] = sum of the 8 children), on 8-channel blocks:
+// lanes along d2, of coarse voxels (modes 0, 3: eight loads) or of fine ones (modes 1, 2: one load and the
+// stores of the 2 x 2 rows above it).  Bound by memory; the index of a thread comes from the grid (with 64-bit
+// divisions per thread the eight of a 96^3 gradient took 72 us, now 44).
+__global__ void __launch_bounds__(256) k_resample(const __nv_bfloat16* __restrict__ in, __nv_bfloat16* __restrict__ out,
+                                                  int chunks, int n0, int n1, int n2, int mode) {
   const int m0 = n0 >> 1, m1 = n1 >> 1, m2 = n2 >> 1;
   const size_t Vf = (size_t)n0 * n1 * n2, Vc = (size_t)m0 * m1 * m2;
-  const bool coarse = (mode == 0 || mode == 3);
-  const size_t per = coarse ? Vc : Vf;
-  const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= per * chunks) return;
-  const int ch = (int)(i / per);
-  const size_t v = i - (size_t)ch * per;
-  const uint4* src = (const uint4*)in;
-  uint4* dst = (uint4*)out;
-  if (coarse) {
-    const int k = (int)(v % m2), j = (int)((v / m2) % m1), ii = (int)(v / ((size_t)m1 * m2));
-    float acc[8] = {0, 0, 0, 0, 0, 0, 0, 0};
-    for (int a = 0; a < 2; ++a)
-      for (int b = 0; b < 2; ++b)
-        for (int c = 0; c < 2; ++c) {
+  const bool coarse = mode == 0 || mode == 3;
+  const int k = blockIdx.x * 32 + threadIdx.x;
+  if (k >= (coarse ? m2 : n2)) return;
+  for (int z = blockIdx.z; z < m0 * chunks; z += gridDim.z) {
+    const int ch = z / m0, i = z - ch * m0;
+    for (int j = blockIdx.y * 8 + threadIdx.y; j < m1; j += gridDim.y * 8) {
+      const size_t vf = (size_t)ch * Vf + ((size_t)(2 * i) * n1 + 2 * j) * n2, vc = (size_t)ch * Vc + ((size_t)i * m1 + j) * m2;
+      if (coarse) {
+        const uint4* src = (const uint4*)in + vf + 2 * k;
+        uint4 u[8];
+#pragma unroll
+        for (int q = 0; q < 8; ++q) u[q] = src[((size_t)(q >> 2) * n1 + (q >> 1 & 1)) * n2 + (q & 1)];
+        float acc[8] = {0, 0, 0, 0, 0, 0, 0, 0};
+#pragma unroll
+        for (int q = 0; q < 8; ++q) {
           float f[8];
-          unpack8(src[(size_t)ch * Vf + ((size_t)(2 * ii + a) * n1 + 2 * j + b) * n2 + 2 * k + c], f);
+          unpack8(u[q], f);
 #pragma unroll
           for (int e = 0; e < 8; ++e) acc[e] += f[e];
         }
-    if (mode == 0)
+        if (mode == 0)
 #pragma unroll
-      for (int e = 0; e < 8; ++e) acc[e] *= 0.125f;
-    dst[(size_t)ch * Vc + v] = pack8(acc);
-  } else {
-    const int k = (int)(v % n2), j = (int)((v / n2) % n1), ii = (int)(v / ((size_t)n1 * n2));
-    uint4 u = src[(size_t)ch * Vc + ((size_t)(ii >> 1) * m1 + (j >> 1)) * m2 + (k >> 1)];
-    if (mode == 1) {
-      float f[8];
-      unpack8(u, f);
+          for (int e = 0; e < 8; ++e) acc[e] *= 0.125f;
+        ((uint4*)out)[vc + k] = pack8(acc);
+      } else {
+        uint4 u = ((const uint4*)in)[vc + (k >> 1)];
+        if (mode == 1) {
+          float f[8];
+          unpack8(u, f);
 #pragma unroll
-      for (int e = 0; e < 8; ++e) f[e] *= 0.125f;
-      u = pack8(f);
+          for (int e = 0; e < 8; ++e) f[e] *= 0.125f;
+          u = pack8(f);
+        }
+        uint4* dst = (uint4*)out + vf + k;
+#pragma unroll
+        for (int q = 0; q < 4; ++q) dst[((size_t)(q >> 1) * n1 + (q & 1)) * n2] = u;
+      }
     }
-    dst[(size_t)ch * Vf + v] = u;
   }
 }
 
@@ -852,31 +858,51 @@ __device__ __forceinline__ float block_sum(float v, float* sh) {
   return v;
 }
 
-// bias gradient partials: part[block][c] = sum over this block's voxels of dy channel c
-__global__ void k_bias_grad_part(const __nv_bfloat16* __restrict__ dy, int chunks, size_t V, float* __restrict__ part) {
-  __shared__ float sh[32];
-  for (int ch = 0; ch < chunks; ++ch) {
-    float acc[8] = {0, 0, 0, 0, 0, 0, 0, 0};
-    for (size_t v = (size_t)blockIdx.x * blockDim.x + threadIdx.x; v < V; v += (size_t)gridDim.x * blockDim.x) {
+// bias gradient partials: part[block][c] = sum over this block's voxels of dy channel c; blockIdx.y is the
+// 8-channel block
+__global__ void __launch_bounds__(kRedThreads) k_bias_grad_part(const __nv_bfloat16* __restrict__ dy, int chunks,
+                                                                size_t V, float* __restrict__ part) {
+  __shared__ float sh[kRedThreads / 32][8];
+  const uint4* src = (const uint4*)dy + (size_t)blockIdx.y * V;
+  float acc[8] = {0, 0, 0, 0, 0, 0, 0, 0};
+  const size_t step = (size_t)gridDim.x * kRedThreads;
+  for (size_t v = (size_t)blockIdx.x * kRedThreads + threadIdx.x; v < V; v += 4 * step) {
+    uint4 u[4];
+#pragma unroll
+    for (int q = 0; q < 4; ++q) u[q] = v + q * step < V ? src[v + q * step] : make_uint4(0, 0, 0, 0);
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
       float f[8];
-      unpack8(((const uint4*)dy)[(size_t)ch * V + v], f);
+      unpack8(u[q], f);
 #pragma unroll
       for (int e = 0; e < 8; ++e) acc[e] += f[e];
     }
-    for (int e = 0; e < 8; ++e) {
-      const float s = block_sum(acc[e], sh);
-      if (threadIdx.x == 0) part[(size_t)blockIdx.x * chunks * 8 + ch * 8 + e] = s;
-    }
+  }
+#pragma unroll
+  for (int e = 0; e < 8; ++e)
+    for (int o = 16; o > 0; o >>= 1) acc[e] += __shfl_xor_sync(0xffffffffu, acc[e], o);
+  if ((threadIdx.x & 31) == 0)
+#pragma unroll
+    for (int e = 0; e < 8; ++e) sh[threadIdx.x >> 5][e] = acc[e];
+  __syncthreads();
+  if (threadIdx.x < 8) {
+    float s = 0.f;
+    for (int w = 0; w < kRedThreads / 32; ++w) s += sh[w][threadIdx.x];
+    part[(size_t)blockIdx.x * chunks * 8 + blockIdx.y * 8 + threadIdx.x] = s;
   }
 }
 
-// out[c] = sum over parts of part[p][c], fixed order
-__global__ void k_sum_parts(const float* __restrict__ part, int parts, int width, int n, float* __restrict__ out) {
-  const int c = blockIdx.x * blockDim.x + threadIdx.x;
-  if (c >= n) return;
-  float s = 0.f;
-  for (int k = 0; k < parts; ++k) s += part[(size_t)k * width + c];
-  out[c] = s;
+// out[c] = sum over parts of part[p][c], fixed order: a warp per c (one thread each took 11 us)
+__global__ void __launch_bounds__(32) k_sum_parts(const float* __restrict__ part, int parts, int width,
+                                                  float* __restrict__ out) {
+  CompSum s;
+  for (int k = threadIdx.x; k < parts; k += 32) s.add(part[(size_t)k * width + blockIdx.x]);
+  for (int o = 16; o > 0; o >>= 1) {
+    const float hi = __shfl_xor_sync(0xffffffffu, s.s, o), lo = __shfl_xor_sync(0xffffffffu, s.c, o);
+    s.add(hi);
+    s.c += lo;
+  }
+  if (threadIdx.x == 0) out[blockIdx.x] = s.s + s.c;
 }
 
 // partial sums of e = pred - target * (*inv_scale) and e^2; part[block] = (sum e, sum e^2)
@@ -903,12 +929,17 @@ __global__ void k_loss_part(const float* __restrict__ pred, const float* __restr
 // target, the scale of a right-hand side); k_loss_grad writes dL/dpred = 2 (e - mean e) / V as
 // channel 0 of a 16-channel block tensor.
 __global__ void k_loss_final(const float* __restrict__ part, int parts, size_t V, float* __restrict__ out) {
-  if (threadIdx.x != 0 || blockIdx.x != 0) return;
+  // one warp: a chain of 296 FP64 sums in one thread took 47 us
   double a = 0.0, b = 0.0;
-  for (int k = 0; k < parts; ++k) {
+  for (int k = threadIdx.x; k < parts; k += 32) {
     a += part[2 * k];
     b += part[2 * k + 1];
   }
+  for (int o = 16; o > 0; o >>= 1) {
+    a += __shfl_xor_sync(0xffffffffu, a, o);
+    b += __shfl_xor_sync(0xffffffffu, b, o);
+  }
+  if (threadIdx.x != 0) return;
   const double me = a / (double)V, mse = b / (double)V;
   out[0] = (float)(mse - me * me);
   out[1] = (float)me;
@@ -1279,11 +1310,13 @@ extern "C" int pfm_nn_resample(const void* in, void* out, int channels, int d0, 
   if (!in || !out) return PFM_ERR_NULL;
   if (!grid_ok(d0, d1, d2) || d0 % 2 || d1 % 2 || d2 % 2 || channels <= 0 || channels % 8 || mode < 0 || mode > 3)
     return PFM_ERR_SHAPE;
-  const size_t Vf = (size_t)d0 * d1 * d2;
-  const size_t per = (mode == 0 || mode == 3) ? Vf / 8 : Vf;
-  const size_t n = per * (channels / 8);
-  k_resample<<<(unsigned)((n + 255) / 256), 256, 0, (cudaStream_t)stream>>>(
-      (const __nv_bfloat16*)in, (__nv_bfloat16*)out, channels / 8, d0, d1, d2, mode);
+  const int last = (mode == 0 || mode == 3) ? d2 / 2 : d2;
+  const long long planes = (long long)(d0 / 2) * (channels / 8);
+  if (planes > 0x7fffffff) return PFM_ERR_SHAPE;
+  const dim3 grid((unsigned)((last + 31) / 32), (unsigned)std::min((d1 / 2 + 7) / 8, 65535),
+                  (unsigned)std::min<long long>(planes, 65535));
+  k_resample<<<grid, dim3(32, 8), 0, (cudaStream_t)stream>>>((const __nv_bfloat16*)in, (__nv_bfloat16*)out, channels / 8,
+                                                             d0, d1, d2, mode);
   return cudaGetLastError() == cudaSuccess ? PFM_OK : PFM_ERR_CUDA;
 }
 
@@ -1307,8 +1340,8 @@ extern "C" int pfm_nn_bias_grad(const void* dy, int channels, int d0, int d1, in
   if (!grid_ok(d0, d1, d2) || channels <= 0 || channels % 8 || cout <= 0 || cout > channels) return PFM_ERR_SHAPE;
   cudaStream_t st = (cudaStream_t)stream;
   const size_t V = (size_t)d0 * d1 * d2;
-  k_bias_grad_part<<<kRedBlocks, kRedThreads, 0, st>>>((const __nv_bfloat16*)dy, channels / 8, V, scratch);
-  k_sum_parts<<<(cout + 127) / 128, 128, 0, st>>>(scratch, kRedBlocks, channels, cout, db);
+  k_bias_grad_part<<<dim3(kRedBlocks, (unsigned)(channels / 8)), kRedThreads, 0, st>>>((const __nv_bfloat16*)dy, channels / 8, V, scratch);
+  k_sum_parts<<<(unsigned)cout, 32, 0, st>>>(scratch, kRedBlocks, channels, db);
   return cudaGetLastError() == cudaSuccess ? PFM_OK : PFM_ERR_CUDA;
 }
 
