@@ -120,7 +120,7 @@ struct pfm_handle {
   size_t ws_bytes;
   size_t ws_need;
   // workspace offsets
-  size_t o_key, o_slot, o_order, o_count, o_start, o_blocksums, o_payload;
+  size_t o_key, o_slot, o_order, o_count, o_start, o_blocksums, o_payload, o_tilesum;
   size_t o_r[pfm::kMaxLevels], o_z[pfm::kMaxLevels];
   size_t o_x, o_p, o_Ap, o_b, o_partials, o_state, o_maxpart, o_step;
   // warm_start 2: the previous solution of up to two pressure buffers (the caller's pointers name
@@ -520,6 +520,7 @@ __device__ __forceinline__ void write_p2g_record3(const P2GRecords3& R, int64_t 
 // Launches RK4_T_forward (3D); with R non-null the kernel also writes the P2G records and keys
 // of the advected particles, and with Fg non-null it first does the flow-map gradient
 // reinitialisation (init_C = grad u(p) in Fg, update_T, T_gm = I) (defined in pfm_particles.cu).
+size_t tile_sums_bytes3(const int N[3]);
 int launch_rk4_T_forward3(pfm_handle* h, float* pos, float* T, const MacFields3& F, float dt, const P2GRecords3* R,
                           const MacFields3* Fg, cudaStream_t st, const float* dt_dev = nullptr);
 

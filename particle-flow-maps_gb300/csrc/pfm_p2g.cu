@@ -219,20 +219,23 @@ __global__ void __launch_bounds__(kBinThreads) k_payload2(const int* __restrict_
 // of the 4 x 3 x 3 faces they can reach (4 along the family's own axis: faces c-1 .. c+2; 3 along
 // the others: c-1 .. c+1), every thread stores its window in shared memory (36 slots per cell),
 // and after one barrier each face of the region around the tile sums the slots of the cells that
-// reach it, in slot order, and adds the sum into the face grids.  Tiles run in 8 launches by the
-// parity of their tile coordinates: tiles of one parity are a tile apart and their face regions
-// (one face below, two above) never overlap, so no atomics are needed.  Each face sums in a fixed
-// order (launch, pass, particle index): the result is bitwise reproducible (the same sums, in the
-// same order, as merging the windows into a shared copy of the region in 36 passes with a barrier
-// between passes).  Particles outside the grid sit in the clamped edge cell, whose window still
-// holds every in-grid face they reach; their weights come from their real positions.
+// reach it, in slot order, into the tile's region of the workspace.  A second pass (k_tile_faces3)
+// adds, per face, the sums of the up to 8 tiles whose regions hold it (even tiles before odd ones along
+// each axis, x outermost) and divides by the weight.  No atomics, and each face sums in a fixed
+// order: the result is bitwise reproducible.  Particles outside the grid sit in the clamped edge cell,
+// whose window still holds every in-grid face they reach; their weights come from their real positions.
+// (Adding into the face grids from 8 launches by tile parity gives the same sums, but each launch ends
+// in a wave that fills part of the SMs -- 128 of 304 resident blocks at 64^3 -- and reads the faces back.
+// With its zeroing and normalisation passes it took 505 us at 96^3, 8 particles per cell, this 350; 7.11
+// and 6.35 ms at 256^3.)  k_tile3 is bound by latency and by the longest cell of a warp (two blocks of 128
+// registers a thread per SM), k_tile_faces3 by memory.
 //
 // Record staging: a cell's particles are gathered through the sorted order, so each one costs a
 // memory round trip.  Every thread keeps a ring of kRing particle slots in shared memory (pos4 and
 // the family record, 32 B) filled by 16-byte asynchronous copies (cp.async, no registers held), so
 // kRing - 1 particles are in flight while one is summed; the next slot's particle index is read one
 // iteration ahead.  The first kRing copies of the next family are issued before the window merge
-// and face add-back of the current one, so that memory latency overlaps the merge.
+// of the current one, so that memory latency overlaps the merge.
 //
 // Tile of 4 x 4 x 16 cells (256 threads, 128 registers each): 16 along the last axis, the length
 // of the seeding order's cell groups (pfm_seed_jittered), so the records of a group's particles
@@ -266,6 +269,11 @@ constexpr size_t kWinBytes = (size_t)kWinSlots * kTileThreads * sizeof(float2); 
 constexpr size_t kRingBytes = (size_t)kRing * 2 * kTileThreads * sizeof(float4);  // 16,384 B
 constexpr size_t kTileSmem = kWinBytes + kRingBytes;                              // 92,160 B
 static_assert(kTileSmem <= 227 * 1024, "k_tile3 exceeds the 227 KB of shared memory of a block");
+
+// faces in the region of a tile, per family: one face below the tile, two (along the family's axis) or one above
+__host__ __device__ constexpr int tile_region(int fam) {
+  return (kTX + (fam == 0 ? 3 : 2)) * (kTY + (fam == 1 ? 3 : 2)) * (kTZ + (fam == 2 ? 3 : 2));
+}
 
 struct FaceOut3 {
   float* u[3];
@@ -344,15 +352,14 @@ __device__ __forceinline__ void tile_axis(float p, int c, float* w, float* d) {
 
 // One family: the particle loop from the ring (whose prologue was issued earlier; qn is the index
 // of slot sb + kRing), the window store, and -- after the barrier -- the next family's ring
-// prologue (NEXT >= 0), the window merge and the face add-back.
+// prologue (NEXT >= 0), the window merge and the store of the region's sums.
 template <int FAM, int NEXT, bool APIC>
 __device__ __forceinline__ int tile_family(float2* __restrict__ win, float4* ring, const float4* __restrict__ pos4,
                                            const float4* __restrict__ rec, const float4* __restrict__ rec_next,
                                            const int* __restrict__ order, int sb, int se, int qn, int ci, int cj,
-                                           int ck, int x0, int y0, int z0, const MacGeom& g,
-                                           float* __restrict__ u, float* __restrict__ w) {
+                                           int ck, float2* __restrict__ sums) {
   constexpr int W0 = FAM == 0 ? 4 : 3, W1 = FAM == 1 ? 4 : 3, W2 = FAM == 2 ? 4 : 3;
-  constexpr int E0 = kTX + W0 - 1, E1 = kTY + W1 - 1, E2 = kTZ + W2 - 1, NE = E0 * E1 * E2;
+  constexpr int E1 = kTY + W1 - 1, E2 = kTZ + W2 - 1, NE = tile_region(FAM);
   static_assert(W0 * W1 * W2 <= kWinSlots, "window exceeds the shared buffer");
   float2 acc[W0][W1][W2];  // (numerator, weight sum) of each window face
 #pragma unroll
@@ -419,80 +426,122 @@ __device__ __forceinline__ int tile_family(float2* __restrict__ win, float4* rin
   if (NEXT >= 0) qnext = ring_prologue(ring, pos4, rec_next, order, sb, se);
   // Face e of the tile's region (origin one face below the tile) takes window slot (a, b, k) of
   // the cell e - (a, b, k), summed from zero in slot order (a, then b, then k)
-  const int n0 = g.n[FAM][0], n1 = g.n[FAM][1], n2 = g.n[FAM][2];
-  constexpr int NPT = (NE + kTileThreads - 1) / kTileThreads;
-  int64_t qs[NPT];
-  float2 vs[NPT];
 #pragma unroll
-  for (int j = 0; j < NPT; ++j) {
+  for (int j = 0; j < (NE + kTileThreads - 1) / kTileThreads; ++j) {
     const int e = threadIdx.x + j * kTileThreads;
+    if (e >= NE) break;
     const int ez = e % E2, r = e / E2, ey = r % E1, ex = r / E1;
-    const int gi = x0 - 1 + ex, gj = y0 - 1 + ey, gk = z0 - 1 + ez;
-    qs[j] = -1;
-    if (e < NE && gi >= 0 && gi < n0 && gj >= 0 && gj < n1 && gk >= 0 && gk < n2) {
-      qs[j] = ((int64_t)gi * n1 + gj) * n2 + gk;
-      float2 v = make_float2(0.f, 0.f);
+    float2 v = make_float2(0.f, 0.f);
 #pragma unroll
-      for (int a = 0; a < W0; ++a) {
-        const int sx = ex - a;
-        if (sx < 0 || sx >= kTX) continue;
+    for (int a = 0; a < W0; ++a) {
+      const int sx = ex - a;
+      if (sx < 0 || sx >= kTX) continue;
 #pragma unroll
-        for (int b = 0; b < W1; ++b) {
-          const int sy = ey - b;
-          if (sy < 0 || sy >= kTY) continue;
+      for (int b = 0; b < W1; ++b) {
+        const int sy = ey - b;
+        if (sy < 0 || sy >= kTY) continue;
 #pragma unroll
-          for (int k = 0; k < W2; ++k) {
-            const int sz = ez - k;
-            if (sz < 0 || sz >= kTZ) continue;
-            v = __fadd2_rn(v, win[((a * W1 + b) * W2 + k) * kTileThreads + (sx * kTY + sy) * kTZ + sz]);
-          }
+        for (int k = 0; k < W2; ++k) {
+          const int sz = ez - k;
+          if (sz < 0 || sz >= kTZ) continue;
+          v = __fadd2_rn(v, win[((a * W1 + b) * W2 + k) * kTileThreads + (sx * kTY + sy) * kTZ + sz]);
         }
       }
-      vs[j] = make_float2(v.x + u[qs[j]], v.y + w[qs[j]]);
     }
-  }
-#pragma unroll
-  for (int j = 0; j < NPT; ++j) {
-    if (qs[j] >= 0) {
-      u[qs[j]] = vs[j].x;
-      w[qs[j]] = vs[j].y;
-    }
+    sums[e] = v;
   }
   __syncthreads();
   return qnext;
 }
 
-// One parity class (px, py, pz) of tiles; grid = (tiles along z, y, x of that parity).
+// grid = (tiles along z, y, x); tile_sums holds the regions' sums, family by family
 template <bool APIC>
 __global__ void __launch_bounds__(kTileThreads, kTileBlocksPerSM) k_tile3(const float4* __restrict__ pos4,
                                                            const float4* __restrict__ famrec,
                                                            const int* __restrict__ order,
                                                            const int* __restrict__ start, MacGeom g,
-                                                           int64_t P, int px, int py, int pz, FaceOut3 out) {
+                                                           int64_t P, float2* __restrict__ tile_sums) {
   extern __shared__ __align__(16) unsigned char tile_smem[];
   float2* win = reinterpret_cast<float2*>(tile_smem);  // kWinSlots x kTileThreads window values (num, den)
   float4* ring = reinterpret_cast<float4*>(tile_smem + kWinBytes);
-  const int x0 = (2 * (int)blockIdx.z + px) * kTX, y0 = (2 * (int)blockIdx.y + py) * kTY;
-  const int z0 = (2 * (int)blockIdx.x + pz) * kTZ;
   const int lz = threadIdx.x % kTZ, ly = (threadIdx.x / kTZ) % kTY, lx = threadIdx.x / (kTZ * kTY);
-  const int ci = x0 + lx, cj = y0 + ly, ck = z0 + lz;
+  const int ci = (int)blockIdx.z * kTX + lx, cj = (int)blockIdx.y * kTY + ly, ck = (int)blockIdx.x * kTZ + lz;
   int sb = 0, se = 0;
   if (ci < g.N[0] && cj < g.N[1] && ck < g.N[2]) {
     const int c = (ci * g.N[1] + cj) * g.N[2] + ck;
     sb = __ldg(start + c);
     se = __ldg(start + c + 1);
   }
+  const int64_t nt = (int64_t)gridDim.x * gridDim.y * gridDim.z;
+  const int64_t tile = ((int64_t)blockIdx.z * gridDim.y + blockIdx.y) * gridDim.x + blockIdx.x;
+  float2* s0 = tile_sums + tile * tile_region(0);
+  float2* s1 = tile_sums + nt * tile_region(0) + tile * tile_region(1);
+  float2* s2 = tile_sums + nt * (tile_region(0) + tile_region(1)) + tile * tile_region(2);
   const float4* r0 = famrec;
   const float4* r1 = famrec + P;
   const float4* r2 = famrec + 2 * P;
   int qn = ring_prologue(ring, pos4, r0, order, sb, se);
-  qn = tile_family<0, 1, APIC>(win, ring, pos4, r0, r1, order, sb, se, qn, ci, cj, ck, x0, y0, z0, g, out.u[0],
-                               out.w[0]);
-  qn = tile_family<1, 2, APIC>(win, ring, pos4, r1, r2, order, sb, se, qn, ci, cj, ck, x0, y0, z0, g, out.u[1],
-                               out.w[1]);
-  tile_family<2, -1, APIC>(win, ring, pos4, r2, r2, order, sb, se, qn, ci, cj, ck, x0, y0, z0, g, out.u[2],
-                           out.w[2]);
+  qn = tile_family<0, 1, APIC>(win, ring, pos4, r0, r1, order, sb, se, qn, ci, cj, ck, s0);
+  qn = tile_family<1, 2, APIC>(win, ring, pos4, r1, r2, order, sb, se, qn, ci, cj, ck, s1);
+  tile_family<2, -1, APIC>(win, ring, pos4, r2, r2, order, sb, se, qn, ci, cj, ck, s2);
   cp_async_wait<0>();
+}
+
+// The tiles whose regions hold face index f along one axis (tiles of T cells, regions of E faces from one
+// below the tile): n of them, the even tile first; tile t[i], position e[i] in its region.
+template <int T, int E>
+__device__ __forceinline__ int axis_tiles(int f, int nt, int (&t)[2], int (&e)[2]) {
+  const int hi = (f + 1) / T, r = f + 1 - hi * T;  // region of tile hi starts at face T hi - 1
+  const bool a = hi < nt, b = hi > 0 && r + T < E;
+  const bool swap = a && b && (hi & 1);
+  t[0] = a && !swap ? hi : hi - 1;
+  e[0] = a && !swap ? r : r + T;
+  t[1] = swap ? hi : hi - 1;
+  e[1] = swap ? r : r + T;
+  return (a ? 1 : 0) + (b ? 1 : 0);
+}
+
+// Faces of family FAM from the tiles' sums: u = sum num / sum den where den > 0 (3D/run_3D.py:530-552), w = sum den.
+template <int FAM>
+__device__ __forceinline__ void tile_face(unsigned f, const float2* __restrict__ sums, const MacGeom& g, int nt0, int nt1,
+                                          int nt2, float* __restrict__ u, float* __restrict__ w) {
+  constexpr int E0 = kTX + (FAM == 0 ? 3 : 2), E1 = kTY + (FAM == 1 ? 3 : 2), E2 = kTZ + (FAM == 2 ? 3 : 2);
+  int i, j, k;
+  split3(f, g.dn[FAM][1], g.dn[FAM][2], i, j, k);
+  int t0[2], e0[2], t1[2], e1[2], t2[2], e2[2];
+  const int c0 = axis_tiles<kTX, E0>(i, nt0, t0, e0), c1 = axis_tiles<kTY, E1>(j, nt1, t1, e1);
+  const int c2 = axis_tiles<kTZ, E2>(k, nt2, t2, e2);
+  float2 s[8];
+#pragma unroll
+  for (int q = 0; q < 8; ++q) {
+    const int a = q >> 2, b = q >> 1 & 1, c = q & 1;
+    s[q] = make_float2(0.f, 0.f);
+    if (a < c0 && b < c1 && c < c2)
+      s[q] = __ldcs(sums + (((int64_t)t0[a] * nt1 + t1[b]) * nt2 + t2[c]) * tile_region(FAM) + (e0[a] * E1 + e1[b]) * E2 + e2[c]);
+  }
+  float2 v = s[0];
+#pragma unroll
+  for (int q = 1; q < 8; ++q) v = __fadd2_rn(v, s[q]);
+  w[f] = v.y;
+  u[f] = v.y > 0.f ? v.x / v.y : v.x;
+}
+
+__global__ void __launch_bounds__(kBinThreads) k_tile_faces3(const float2* __restrict__ sums, MacGeom g, int nt0, int nt1,
+                                                             int nt2, int64_t F0, int64_t F1, int64_t F2, FaceOut3 out) {
+  int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  const int64_t nt = (int64_t)nt0 * nt1 * nt2;
+  if (e < F0) {
+    tile_face<0>((unsigned)e, sums, g, nt0, nt1, nt2, out.u[0], out.w[0]);
+  } else if ((e -= F0) < F1) {
+    tile_face<1>((unsigned)e, sums + nt * tile_region(0), g, nt0, nt1, nt2, out.u[1], out.w[1]);
+  } else if ((e -= F1) < F2) {
+    tile_face<2>((unsigned)e, sums + nt * (tile_region(0) + tile_region(1)), g, nt0, nt1, nt2, out.u[2], out.w[2]);
+  }
+}
+
+size_t tile_sums_bytes3(const int N[3]) {
+  const size_t nt = (size_t)((N[0] + kTX - 1) / kTX) * ((N[1] + kTY - 1) / kTY) * ((N[2] + kTZ - 1) / kTZ);
+  return nt * (tile_region(0) + tile_region(1) + tile_region(2)) * sizeof(float2);
 }
 
 // ---------------------------------------------------------------------------------------------
@@ -699,50 +748,6 @@ __global__ void __launch_bounds__(kBinThreads) k_normalize_smoke3(float4* __rest
   smoke[e] = s;
 }
 
-// u = u / w where w > 0 (3D/run_3D.py:530-552), all three families in one pass
-__global__ void __launch_bounds__(kBinThreads) k_normalize3(FaceOut3 out, int64_t F0, int64_t F1, int64_t F2) {
-  int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  int f = 0;
-  if (e >= F0) {
-    e -= F0;
-    f = 1;
-    if (e >= F1) {
-      e -= F1;
-      f = 2;
-      if (e >= F2) return;
-    }
-  }
-  float* u = f == 0 ? out.u[0] : (f == 1 ? out.u[1] : out.u[2]);
-  const float* w = f == 0 ? out.w[0] : (f == 1 ? out.w[1] : out.w[2]);
-  const float wv = w[e];
-  if (wv > 0.f) u[e] = u[e] / wv;
-}
-
-// The same division four faces at a time (16-byte vectors of u and w; every family's face count a
-// multiple of 4 and the six arrays 16-byte aligned): element for element k_normalize3.
-__global__ void __launch_bounds__(kBinThreads) k_normalize3v(FaceOut3 out, int64_t Q0, int64_t Q1, int64_t Q2) {
-  int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  int f = 0;
-  if (e >= Q0) {
-    e -= Q0;
-    f = 1;
-    if (e >= Q1) {
-      e -= Q1;
-      f = 2;
-      if (e >= Q2) return;
-    }
-  }
-  float4* u = reinterpret_cast<float4*>(f == 0 ? out.u[0] : (f == 1 ? out.u[1] : out.u[2]));
-  const float4* w = reinterpret_cast<const float4*>(f == 0 ? out.w[0] : (f == 1 ? out.w[1] : out.w[2]));
-  const float4 wv = w[e];
-  float4 uv = u[e];
-  if (wv.x > 0.f) uv.x = uv.x / wv.x;
-  if (wv.y > 0.f) uv.y = uv.y / wv.y;
-  if (wv.z > 0.f) uv.z = uv.z / wv.z;
-  if (wv.w > 0.f) uv.w = uv.w / wv.w;
-  u[e] = uv;
-}
-
 // Column gather (2D): columns along j; 2D normalises with scale = 1/w (run_2D.py:599-611) and
 // also carries the reference map psi.
 template <int fam>
@@ -914,35 +919,24 @@ int p2g3_from_records(pfm_handle* h, float* const* us, float* const* ws, cudaStr
   const int* order = ws_ptr<int>(h, h->o_order);
   FaceOut3 out{{us[0], us[1], us[2]}, {ws[0], ws[1], ws[2]}};
   int64_t F[3];
-  for (int f = 0; f < 3; ++f) {
-    F[f] = (int64_t)h->geom.n[f][0] * h->geom.n[f][1] * h->geom.n[f][2];
-    rc = check_cuda(h, cudaMemsetAsync(us[f], 0, F[f] * 4, st), "zero u");
-    if (!rc) rc = check_cuda(h, cudaMemsetAsync(ws[f], 0, F[f] * 4, st), "zero w");
-    if (rc) return rc;
+  for (int f = 0; f < 3; ++f) F[f] = (int64_t)h->geom.n[f][0] * h->geom.n[f][1] * h->geom.n[f][2];
+  if (h->P == 0) {
+    for (int f = 0; f < 3; ++f) {
+      rc = check_cuda(h, cudaMemsetAsync(us[f], 0, F[f] * 4, st), "zero u");
+      if (!rc) rc = check_cuda(h, cudaMemsetAsync(ws[f], 0, F[f] * 4, st), "zero w");
+      if (rc) return rc;
+    }
+    return launch_check(h, "p2g3");
   }
-  if (h->P > 0) {
-    static std::atomic<unsigned long long> attr{0};  // above the default 48 KB: opt in per device
-    auto tile = h->cfg.use_apic ? k_tile3<true> : k_tile3<false>;
-    rc = check_cuda(h, opt_in_smem(tile, (int)kTileSmem, attr), "k_tile3 shared-memory attribute");
-    if (rc) return rc;
-    const int nt[3] = {(h->geom.N[0] + kTX - 1) / kTX, (h->geom.N[1] + kTY - 1) / kTY, (h->geom.N[2] + kTZ - 1) / kTZ};
-    for (int px = 0; px < 2; ++px)
-      for (int py = 0; py < 2; ++py)
-        for (int pz = 0; pz < 2; ++pz) {
-          const unsigned bx = (nt[0] - px + 1) / 2, by = (nt[1] - py + 1) / 2, bz = (nt[2] - pz + 1) / 2;
-          if (!bx || !by || !bz) continue;
-          launch(h, tile, dim3(bz, by, bx), kTileThreads, kTileSmem, st, pos4, famrec, order, start, h->geom, h->P,
-                 px, py, pz, out);
-        }
-    bool vec = true;
-    for (int f = 0; f < 3; ++f)
-      vec = vec && F[f] % 4 == 0 && ((uintptr_t)us[f] | (uintptr_t)ws[f]) % 16 == 0;
-    if (vec)
-      launch(h, k_normalize3v, grid_for((F[0] + F[1] + F[2]) / 4, kBinThreads), kBinThreads, 0, st, out, F[0] / 4,
-             F[1] / 4, F[2] / 4);
-    else
-      launch(h, k_normalize3, grid_for(F[0] + F[1] + F[2], kBinThreads), kBinThreads, 0, st, out, F[0], F[1], F[2]);
-  }
+  static std::atomic<unsigned long long> attr[2];  // above the default 48 KB: opt in per kernel and device
+  auto tile = h->cfg.use_apic ? k_tile3<true> : k_tile3<false>;
+  rc = check_cuda(h, opt_in_smem(tile, (int)kTileSmem, attr[h->cfg.use_apic ? 1 : 0]), "k_tile3 shared-memory attribute");
+  if (rc) return rc;
+  const int nt[3] = {(h->geom.N[0] + kTX - 1) / kTX, (h->geom.N[1] + kTY - 1) / kTY, (h->geom.N[2] + kTZ - 1) / kTZ};
+  float2* sums = ws_ptr<float2>(h, h->o_tilesum);
+  launch(h, tile, dim3(nt[2], nt[1], nt[0]), kTileThreads, kTileSmem, st, pos4, famrec, order, start, h->geom, h->P, sums);
+  launch(h, k_tile_faces3, grid_for(F[0] + F[1] + F[2], kBinThreads), kBinThreads, 0, st, (const float2*)sums, h->geom,
+         nt[0], nt[1], nt[2], F[0], F[1], F[2], out);
   return launch_check(h, "p2g3");
 }
 
