@@ -138,7 +138,7 @@ int pfm_measure_fp32_peak(float* sink, int blocks_per_sm, int iters, int reps, i
  * their order); they only change how the work maps to the GPU.  Setting one drops the handle's
  * captured graphs (they are rebuilt on next use); a batch that holds the handle must be rebuilt
  * (a new pfm_batch).  pfm.tune.autotune picks them by timing on a scene's own data. */
-#define PFM_TUNE_P2G2_COLUMN 1    /* faces per thread of the 2D P2G column gather, 1..64 (8) */
+#define PFM_TUNE_P2G2_COLUMN 1    /* 1..64 (8): kept and read back; the 2D P2G picks its faces per thread by size */
 #define PFM_TUNE_MG_TAIL_CELLS 2  /* MGPCG levels with at most this many cells run the rest of the
                                      V-cycle in one thread block; 0 = none (4096) */
 #define PFM_TUNE_SMOOTH_TMA 3     /* 1: 3D 16-bit MGPCG levels are smoothed from tiles the TMA stages

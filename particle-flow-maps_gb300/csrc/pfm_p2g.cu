@@ -8,8 +8,8 @@
 //  2. a payload pass evaluates each particle's impulse m = T_gm^T-composed init_imp and affine
 //     matrix T_gm^T C T_gm once, in sorted order (float4 records);
 //  3. 3D: one thread per cell sums its particles into the window of faces they reach and cell
-//     tiles merge the windows in shared memory in a fixed order (k_tile3); 2D: one thread per
-//     face column gathers the particles of the cells that reach it (k_gather2).
+//     tiles merge the windows in shared memory in a fixed order (k_tile3); 2D: a thread gathers
+//     the particles of the cells that reach its faces (k_face2).
 //     Particles outside the grid keep a clamped key, which stays inside every neighbourhood they
 //     can reach, and their weights come from their real positions, exactly as the reference's
 //     bounds-checked scatter.
@@ -748,100 +748,97 @@ __global__ void __launch_bounds__(kBinThreads) k_normalize_smoke3(float4* __rest
   smoke[e] = s;
 }
 
-// Column gather (2D): columns along j; 2D normalises with scale = 1/w (run_2D.py:599-611) and
-// also carries the reference map psi.
-template <int fam>
-__global__ void __launch_bounds__(128) k_gather2(const float4* __restrict__ pos4, const float4* __restrict__ famrec,
-                                                 const int* __restrict__ start, MacGeom g, int K, int use_apic,
-                                                 int64_t P, float* __restrict__ u, float* __restrict__ w,
-                                                 float* __restrict__ psig) {
-  constexpr int WIN = (fam == 1) ? 4 : 3;
-  const int n0 = g.n[fam][0], n1 = g.n[fam][1];
-  const int nseg = (n1 + K - 1) / K;
-  const int64_t ncol = (int64_t)n0 * nseg;
-  const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= ncol) return;
-  const int i = (int)(t % n0);
-  const int seg = (int)(t / n0);
-  const int j0 = seg * K, j1 = min(j0 + K, n1);
-  const int G0 = g.N[0], G1 = g.N[1];
-  const int ci_lo = max(i - (fam == 0 ? 2 : 1), 0), ci_hi = min(i + 1, G0 - 1);
-  const int cj_lo = max(j0 - (fam == 1 ? 2 : 1), 0), cj_hi = min(j1, G1 - 1);
-  const float fi = (float)i, dx = g.dx;
-  float num[WIN], den[WIN], s0[WIN], s1[WIN];
+// Face gather (2D): a thread sums NF faces next to each other along i from the particles of the cells that reach
+// them, each face's in the order of the cells (cj, then ci) and of the particles, loading NB particles of a cell
+// ahead of their sums; 2D normalises with scale = 1/w (run_2D.py:599-611) and also carries the reference map
+// psi.  The rounding of every term is spelled out, so that a face's sum does not depend on NF and NB.
+// Bound by the latency of the dependent loads on small grids (start, then particles: a face visits 12 cells)
+// and by the L1 wavefronts of 32 cells' records on large ones.
+template <int fam, int NF, int NB>
+__device__ __forceinline__ void face2(const float4* __restrict__ pos4, const float4* __restrict__ rec,
+                                      const int* __restrict__ start, const MacGeom& g, int use_apic,
+                                      float* __restrict__ u, float* __restrict__ w, float* __restrict__ psig) {
+  constexpr int NI = NF + (fam == 0 ? 3 : 2), NJ = fam == 1 ? 4 : 3;  // cells that reach the faces along i and j
+  const int n0 = g.n[fam][0], n1 = g.n[fam][1], G0 = g.N[0], G1 = g.N[1];
+  const int j = blockIdx.x * 32 + (threadIdx.x & 31), i0 = (blockIdx.y * 4 + (threadIdx.x >> 5)) * NF;
+  if (i0 >= n0 || j >= n1) return;
+  const int ci0 = i0 - (fam == 0 ? 2 : 1), cj0 = j - (NJ - 2);
+  int st[NI][NJ + 1];
 #pragma unroll
-  for (int q = 0; q < WIN; ++q) num[q] = den[q] = s0[q] = s1[q] = 0.f;
-  auto flush = [&](int jf, int q) {
-    if (jf >= j0 && jf < j1) {
-      const int64_t e = (int64_t)i * n1 + jf;
-      float a = num[q], b0 = s0[q], b1 = s1[q];
-      if (den[q] > 0.f) {
-        float scale = 1.f / den[q];
-        a *= scale;
-        b0 *= scale;
-        b1 *= scale;
-      }
-      w[e] = den[q];
-      u[e] = a;
-      if (psig) {
-        psig[e * 2] = b0;
-        psig[e * 2 + 1] = b1;
-      }
+  for (int a = 0; a < NI; ++a) {
+    const int ci = ci0 + a;
+#pragma unroll
+    for (int b = 0; b <= NJ; ++b) {
+      const int cj = min(max(cj0 + b, 0), G1);
+      st[a][b] = ci >= 0 && ci < G0 ? __ldg(start + ci * G1 + cj) : 0;
     }
-  };
-  int jb = cj_lo - 1;
-  for (int cj = cj_lo; cj <= cj_hi; ++cj) {
-    while (jb < cj - 1) {
-      flush(jb, 0);
+  }
+  const float fj = (float)j, dx = g.dx;
+  float num[NF], den[NF], s0[NF], s1[NF];
 #pragma unroll
-      for (int q = 0; q < WIN - 1; ++q) {
-        num[q] = num[q + 1];
-        den[q] = den[q + 1];
-        s0[q] = s0[q + 1];
-        s1[q] = s1[q + 1];
-      }
-      num[WIN - 1] = den[WIN - 1] = s0[WIN - 1] = s1[WIN - 1] = 0.f;
-      ++jb;
-    }
-    const float fj0 = (float)(cj - 1);
-    for (int ci = ci_lo; ci <= ci_hi; ++ci) {
-      const int c = ci * G1 + cj;
-      const int sb = __ldg(start + c), se = __ldg(start + c + 1);
-      for (int s = sb; s < se; ++s) {
-        const float4 p = __ldg(pos4 + s);
-        float wi, di;
-        if (fam == 0) {
-          wi = N2(p.x - fi);
-          di = (fi - p.x) * dx;
-        } else {
-          wi = N2((p.x - fi) - 0.5f);
-          di = ((fi + 0.5f) - p.x) * dx;
-        }
-        if (wi == 0.f) continue;
-        const float4 fr = __ldg(famrec + (int64_t)fam * P + s);
+  for (int q = 0; q < NF; ++q) num[q] = den[q] = s0[q] = s1[q] = 0.f;
 #pragma unroll
-        for (int q = 0; q < WIN; ++q) {
-          const float fj = fj0 + (float)q;
-          float wj, dj;
-          if (fam == 1) {
-            wj = N2(p.y - fj);
-            dj = (fj - p.y) * dx;
-          } else {
-            wj = N2((p.y - fj) - 0.5f);
-            dj = ((fj + 0.5f) - p.y) * dx;
+  for (int b = 0; b < NJ; ++b) {
+#pragma unroll
+    for (int a = 0; a < NI; ++a) {
+      for (int s = st[a][b]; s < st[a][b + 1]; s += NB) {
+        float4 pp[NB], ff[NB];
+#pragma unroll
+        for (int k = 0; k < NB; ++k)
+          if (s + k < st[a][b + 1]) {
+            pp[k] = __ldg(pos4 + s + k);
+            ff[k] = __ldg(rec + s + k);
           }
-          const float wt = wi * wj;
-          const float delta = fr.y * di + fr.z * dj;
-          num[q] += (use_apic ? (fr.x + delta) : fr.x) * wt;
-          den[q] += wt;
-          s0[q] += p.z * wt;
-          s1[q] += p.w * wt;
+#pragma unroll
+        for (int k = 0; k < NB; ++k) {
+          if (s + k >= st[a][b + 1]) break;
+          const float4 p = pp[k], fr = ff[k];
+          const float wj = fam == 1 ? N2(p.y - fj) : N2((p.y - fj) - 0.5f);
+          const float dj = fam == 1 ? (fj - p.y) * dx : ((fj + 0.5f) - p.y) * dx;
+#pragma unroll
+          for (int q = 0; q < NF; ++q) {
+            if (a < q || a > q + (fam == 0 ? 3 : 2)) continue;
+            const float fi = (float)(i0 + q);
+            const float wi = fam == 0 ? N2(p.x - fi) : N2((p.x - fi) - 0.5f);
+            const float di = fam == 0 ? (fi - p.x) * dx : ((fi + 0.5f) - p.x) * dx;
+            if (wi == 0.f) continue;
+            const float wt = __fmul_rn(wi, wj);
+            const float v = use_apic ? __fadd_rn(fr.x, __fmaf_rn(fr.z, dj, __fmul_rn(fr.y, di))) : fr.x;
+            num[q] = __fmaf_rn(v, wt, num[q]);
+            den[q] = __fadd_rn(den[q], wt);
+            s0[q] = __fmaf_rn(p.z, wt, s0[q]);
+            s1[q] = __fmaf_rn(p.w, wt, s1[q]);
+          }
         }
       }
     }
   }
 #pragma unroll
-  for (int q = 0; q < WIN; ++q) flush(jb + q, q);
+  for (int q = 0; q < NF; ++q) {
+    if (i0 + q >= n0) break;
+    const int64_t e = (int64_t)(i0 + q) * n1 + j;
+    const float scale = den[q] > 0.f ? 1.f / den[q] : 1.f;
+    w[e] = den[q];
+    u[e] = num[q] * scale;
+    if (psig) {
+      psig[e * 2] = s0[q] * scale;
+      psig[e * 2 + 1] = s1[q] * scale;
+    }
+  }
+}
+
+struct FaceOut2 {
+  float *u[2], *w[2], *psi[2];
+};
+
+template <int NF, int NB>
+__global__ void __launch_bounds__(128) k_face2(const float4* __restrict__ pos4, const float4* __restrict__ famrec,
+                                               const int* __restrict__ start, MacGeom g, int use_apic, int64_t P,
+                                               FaceOut2 out) {
+  if (blockIdx.z == 0)
+    face2<0, NF, NB>(pos4, famrec, start, g, use_apic, out.u[0], out.w[0], out.psi[0]);
+  else
+    face2<1, NF, NB>(pos4, famrec + P, start, g, use_apic, out.u[1], out.w[1], out.psi[1]);
 }
 
 // Bins with counted keys/slots -> bin starts and the stable order (scan, scatter, per-bin sort).
@@ -1117,19 +1114,17 @@ int pfm2_p2g(pfm_handle* h, const float* imp, const float* pos, const float* C, 
   if (h->P > 0)
     launch(h, k_payload2, grid_for(h->P, kBinThreads), kBinThreads, 0, st, ws_ptr<int>(h, h->o_order), h->P, h->geom,
            pos, imp, C, psi, pos4, famrec);
-  float* us[2] = {u_x, u_y};
-  float* ws[2] = {w_x, w_y};
-  float* ps[2] = {psi_x, psi_y};
+  // One face per thread with four loads in flight while that leaves SMs short of warps, two faces and two loads
+  // beyond (both families, 4 particles per cell, one launch: 128^2 20.6 against 34.1 us, 256^2 30.4 against 40.5,
+  // 512^2 105.8 against 95.9, 1024^2 416 against 348; columns of 8 faces per thread, a launch per family, took
+  // 235, 250, 334 and 493).
+  const FaceOut2 out{{u_x, u_y}, {w_x, w_y}, {psi_x, psi_y}};
   const int* start = ws_ptr<int>(h, h->o_start);
-  for (int f = 0; f < 2; ++f) {
-    const int n1 = h->geom.n[f][1];
-    const int K = n1 < h->p2g2_column ? n1 : h->p2g2_column;
-    const int64_t ncol = (int64_t)h->geom.n[f][0] * ((n1 + K - 1) / K);
-    if (f == 0) launch(h, k_gather2<0>, grid_for(ncol, 128), 128, 0, st, pos4, famrec, start, h->geom, K,
-                       h->cfg.use_apic, h->P, us[f], ws[f], ps[f]);
-    if (f == 1) launch(h, k_gather2<1>, grid_for(ncol, 128), 128, 0, st, pos4, famrec, start, h->geom, K,
-                       h->cfg.use_apic, h->P, us[f], ws[f], ps[f]);
-  }
+  const int NF = h->cells < 160000 ? 1 : 2;
+  const dim3 gr((unsigned)(h->geom.N[1] / 32 + 1), (unsigned)(h->geom.N[0] / (4 * NF) + 1), 2);
+  auto gather = NF == 1 ? k_face2<1, 4> : k_face2<2, 2>;
+  launch(h, gather, gr, 128, 0, st, (const float4*)pos4, (const float4*)famrec, start, h->geom, h->cfg.use_apic, h->P,
+         out);
   return launch_check(h, "pfm2_p2g");
 }
 

@@ -6,8 +6,7 @@ simulation; it is done once per scene size, before the step or batch graphs are 
   * ``mg_tail_cells``: the MGPCG levels with at most this many cells run the rest of the V-cycle
     in one thread block (fewer launches, one SM) instead of grid-wide kernels; timed on a solve of
     the scene's current divergence (into a scratch pressure);
-  * ``p2g2_column`` (2D): faces per thread of the P2G column gather; timed on the scene's P2G into
-    its scratch grids;
+  * ``p2g2_column`` (2D): kept for callers; the P2G picks its faces per thread by size;
   * ``smooth_tma`` (3D, 16-bit MGPCG levels): smoothing from tiles the TMA stages in shared memory
     (1) or from global memory (0); timed on the same solve.
 """
