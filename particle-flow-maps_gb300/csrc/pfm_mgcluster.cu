@@ -747,36 +747,6 @@ __global__ void __launch_bounds__(kT, 1) k_cluster_tail(S* __restrict__ zg, cons
 // ---------------------------------------------------------------------------------------------
 // cluster-wide sums
 // ---------------------------------------------------------------------------------------------
-// GB300 issues one FP64 warp instruction per 16 cycles and SM, with 63 cycles of latency for an addition
-// and 670 for a division, so the sums of compensated f32 terms are trees of f32 pairs (Knuth's TwoSum,
-// about 48 bits: far below the rounding of the f32 terms themselves).
-struct Pair {
-  float s, c;
-};
-
-// s is the chain of plain additions, c collects their exact errors
-__device__ __forceinline__ Pair pair_add(Pair a, Pair b) {
-  const float t = a.s + b.s;
-  const float bb = t - a.s;
-  return Pair{t, ((a.s - (t - bb)) + (b.s - bb)) + (a.c + b.c)};
-}
-
-__device__ __forceinline__ double pair_value(Pair a) { return (double)a.s + (double)a.c; }
-__device__ __forceinline__ Pair to_pair(double x) {
-  const float s = (float)x;
-  return Pair{s, (float)(x - (double)s)};
-}
-
-template <int WIDTH>
-__device__ __forceinline__ Pair pair_reduce(Pair v) {
-#pragma unroll
-  for (int o = WIDTH / 2; o > 0; o >>= 1) {
-    const Pair w{__shfl_xor_sync(0xffffffffu, v.s, o), __shfl_xor_sync(0xffffffffu, v.c, o)};
-    v = pair_add(v, w);
-  }
-  return v;
-}
-
 constexpr int kWarps = kT / 32;
 
 struct ClusterRed {  // in shared memory

@@ -125,6 +125,114 @@ __device__ bool grid_sum2(double v0, double v1, double* partials, unsigned* tick
   return true;
 }
 
+// The same for compensated f32 sums, by trees of f32 pairs (48 bits): in FP64, at one warp instruction per 16 cycles and SM, the two trees of
+// 64 resident warps took some 6000 cycles per sum.
+__device__ __forceinline__ bool grid_sum(const CompSum& v, double* partials, unsigned* ticket, double* total,
+                                         unsigned bid, unsigned nb) {
+  __shared__ Pair ws[32];
+  __shared__ bool last;
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = blockDim.x >> 5;
+  const Pair w = pair_reduce<32>(Pair{v.s, v.c});
+  if (lane == 0) ws[wid] = w;
+  __syncthreads();
+  if (wid == 0) {
+    const Pair b = pair_reduce<32>(lane < nw ? ws[lane] : Pair{0.f, 0.f});
+    if (lane == 0) {
+      partials[bid] = pair_value(b);
+      __threadfence();
+      last = atomicAdd(ticket, 1u) == nb - 1;
+    }
+  }
+  __syncthreads();
+  if (!last) return false;
+  __threadfence();
+  Pair s{0.f, 0.f};
+  for (int b = threadIdx.x; b < (int)nb; b += blockDim.x) s = pair_add(s, to_pair(((volatile double*)partials)[b]));
+  s = pair_reduce<32>(s);
+  if (lane == 0) ws[wid] = s;
+  __syncthreads();
+  if (wid == 0) {
+    s = pair_reduce<32>(lane < nw ? ws[lane] : Pair{0.f, 0.f});
+    if (lane == 0) {
+      *total = pair_value(s);
+      *ticket = 0u;
+    }
+  }
+  __syncthreads();
+  return true;
+}
+
+// Blocks of 64 threads that stand for the 256-thread blocks of grid_sum, each thread for four of the lanes:
+// d[s] are the lanes' values of sum s, and every sum is grid_sum's, bit for bit (the trees of a warp's 32
+// lanes over 8 threads).  True in thread 0 of the last block, with the totals.
+constexpr int kLaneThreads = 64;
+
+// warp_sum of the 32 lanes of 8 threads, in all of them.  Partners split the additions of a level between
+// them (6 FP64 instructions; 15 when each thread adds all its lanes), at 16 cycles of an SM's FP64 pipe each.
+__device__ __forceinline__ double lanes_tree(const double (&d)[4]) {
+  const bool h4 = threadIdx.x & 4, h2 = threadIdx.x & 2;
+  const double a0 = (h4 ? d[2] : d[0]) + __shfl_xor_sync(0xffffffffu, h4 ? d[0] : d[2], 4);
+  const double a1 = (h4 ? d[3] : d[1]) + __shfl_xor_sync(0xffffffffu, h4 ? d[1] : d[3], 4);
+  double v = (h2 ? a1 : a0) + __shfl_xor_sync(0xffffffffu, h2 ? a0 : a1, 2);
+  v += __shfl_xor_sync(0xffffffffu, v, 1);
+  v += __shfl_xor_sync(0xffffffffu, v, 4);
+  return v + __shfl_xor_sync(0xffffffffu, v, 2);
+}
+
+template <int N>
+__device__ __forceinline__ bool lanes_sum(double (&d)[N][4], int sums, double* partials, unsigned* ticket,
+                                          double (&total)[N]) {
+  __shared__ double ws[N][8];
+  __shared__ bool last;
+  const unsigned nb = gridDim.x, t = threadIdx.x;
+#pragma unroll
+  for (int s = 0; s < N; ++s) {
+    if (s >= sums) break;
+    const double v = lanes_tree(d[s]);
+    if ((t & 7) == 0) ws[s][t >> 3] = v;
+  }
+  __syncthreads();
+  if (t < 32) {
+#pragma unroll
+    for (int s = 0; s < N; ++s) {
+      if (s >= sums) break;
+      double b = t < 8 ? ws[s][t] : 0.0;  // the block's other warps add zeros in warp_sum
+#pragma unroll
+      for (int o = 4; o > 0; o >>= 1) b += __shfl_down_sync(0xffffffffu, b, o);
+      if (t == 0) partials[s * nb + blockIdx.x] = b;
+    }
+    if (t == 0) {
+      __threadfence();
+      last = atomicAdd(ticket, 1u) == nb - 1;
+    }
+  }
+  __syncthreads();
+  if (!last) return false;
+  __threadfence();
+#pragma unroll
+  for (int s = 0; s < N; ++s) {
+    if (s >= sums) break;
+    double e[4];
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      e[q] = 0.0;
+      for (unsigned b = 4 * t + q; b < nb; b += 4 * kLaneThreads) e[q] += ((volatile double*)partials)[s * nb + b];
+    }
+    const double v = lanes_tree(e);
+    if ((t & 7) == 0) ws[s][t >> 3] = v;
+  }
+  __syncthreads();
+  if (t != 0) return false;
+#pragma unroll
+  for (int s = 0; s < N; ++s) {
+    if (s >= sums) break;
+    total[s] = 0.0;
+    for (int w = 0; w < 8; ++w) total[s] += ws[s][w];
+  }
+  *ticket = 0u;
+  return true;
+}
+
 struct RedBuf {
   double* partials;  // 2 x kReduceBlocks
   SolveState* st;
@@ -877,31 +985,74 @@ __global__ void __launch_bounds__(256) k_zero(S* __restrict__ a, int64_t n, cons
 // ---------------------------------------------------------------------------------------------
 // PCG kernels with fused reductions and device-side scalar updates
 // ---------------------------------------------------------------------------------------------
+// The passes over whole vectors of the finest level (dots, x and r updates, A p, true residual) read 16-byte
+// vectors where the grid allows: one 4-byte load per thread and array left too few bytes in flight.  The mixed
+// solve's dots, A p and true residual take runs of eight elements per thread and f32 pair trees (four blocks of
+// 64 registers a thread per SM instead of eight of 32); the sums that its 16-bit rounding or the plain FP32
+// solve depend on keep the order of one element per thread, bit for bit (lanes_sum).  256^3, FP16 levels: x/r
+// update 104 -> 69 us, A p 69 -> 44, r . z 31 -> 23, true residual 23 -> 12, recentring 34 -> 23, p update
+// 34 -> 20; 160 x 96 x 72, FP32: x/r update 22 -> 13 us, A p 13 -> 9.6, dots 10 -> 8.4.  Small grids, where
+// latency counts, keep one element per thread.
+constexpr int64_t kRunsMin = 65536;
+constexpr int kRunBlocks = 608;  // 4 per SM
+__host__ __device__ __forceinline__ bool use_runs(int64_t n) { return n % 8 == 0 && n >= kRunsMin; }
+__host__ __device__ __forceinline__ bool use_lanes(int64_t n) { return n % 4 == 0 && n >= kRunsMin; }
+template <int D>
+__host__ __device__ __forceinline__ bool use_runs(const Lvl& L) {
+  return D == 3 && L.n2 % 8 == 0 && L.count >= kRunsMin;
+}
+
+// f(q, centre, neighbour sum, mult) for the W cells of run e (e = index / W) of field x, with stencil<3>'s sums in
+// stencil<3>'s order; returns the run's first index.
+__device__ __forceinline__ void ld_run(const float* p, float (&v)[8]) { ld8(p, v); }
+__device__ __forceinline__ void ld_run(const float* p, float (&v)[4]) { ld4(p, v); }
+
+template <int W, class F>
+__device__ __forceinline__ int64_t stencil_run(const float* __restrict__ x, const Lvl& L, const BC& bc, unsigned e, F&& f) {
+  const int runs = L.n2 / W;
+  const unsigned row = e / (unsigned)runs;
+  const int k0 = (int)(e - row * (unsigned)runs) * W;
+  const unsigned i_ = udiv(row, L.d1);
+  const int i = (int)i_, j = (int)(row - i_ * (unsigned)L.n1);
+  const int64_t sx = (int64_t)L.n1 * L.n2, sy = L.n2;
+  const int64_t c0 = ((int64_t)i * L.n1 + j) * L.n2 + k0;
+  float xc[W], xp[W], xm[W], yp[W], ym[W];
+  ld_run(x + c0, xc);
+  const bool hx = i < L.n0 - 1, lx = i > 0, hy = j < L.n1 - 1, ly = j > 0;
+  if (hx) ld_run(x + c0 + sx, xp);
+  if (lx) ld_run(x + c0 - sx, xm);
+  if (hy) ld_run(x + c0 + sy, yp);
+  if (ly) ld_run(x + c0 - sy, ym);
+  const float zl = k0 > 0 ? x[c0 - 1] : 0.f;
+  const float zr = k0 + W < L.n2 ? x[c0 + W] : 0.f;
+  float base = 6.f;
+  if (i <= 0 && bc.lo[0] == 2) base -= 1.f;
+  if (i >= L.n0 - 1 && bc.hi[0] == 2) base -= 1.f;
+  if (j <= 0 && bc.lo[1] == 2) base -= 1.f;
+  if (j >= L.n1 - 1 && bc.hi[1] == 2) base -= 1.f;
+#pragma unroll
+  for (int q = 0; q < W; ++q) {
+    const int k = k0 + q;
+    float nb = 0.f;
+    if (hx) nb += xp[q];
+    if (lx) nb += xm[q];
+    if (hy) nb += yp[q];
+    if (ly) nb += ym[q];
+    if (k < L.n2 - 1) nb += (q < W - 1) ? xc[q + 1] : zr;
+    if (k > 0) nb += (q > 0) ? xc[q - 1] : zl;
+    float mult = base;
+    if (k <= 0 && bc.lo[2] == 2) mult -= 1.f;
+    if (k >= L.n2 - 1 && bc.hi[2] == 2) mult -= 1.f;
+    f(q, xc[q], nb, mult);
+  }
+  return c0;
+}
+
 enum RedKind { RED_ZTR_INIT = 0, RED_ZTR = 1, RED_RTR0 = 2, RED_MEAN = 3, RED_BTB = 4 };
 
-// sum(a*b) (or sum(a) for RED_MEAN) with a finalizer that updates the solve state.  Per-thread
-// partials accumulate in f32 (the reference solve) or f64 (f64 != 0, the mixed solve).
-template <typename SA>
-__device__ __forceinline__ void dot_blk(const SA* __restrict__ a, const float* __restrict__ b, int64_t n, RedBuf rb,
-                                        int kind, double eps, double inv_n, int max_iters, int f64, unsigned bid,
-                                        unsigned nb) {
-  SolveState* st = rb.st;
-  if (st->done) return;
-  double total;
-  if (f64) {
-    // a 16-bit level vector (z) holds the scaled values: undo the scale of the residual it answers
-    const double us = (sizeof(SA) == 2) ? 1.0 / (double)st->hscale : 1.0;
-    CompSum acc;
-    for (int64_t e = (int64_t)bid * blockDim.x + threadIdx.x; e < n; e += (int64_t)nb * blockDim.x)
-      acc.add((kind == RED_MEAN) ? ldv(a + e) : ldv(a + e) * b[e]);
-    if (!grid_sum(acc.value() * us, rb.partials, &st->ticket, &total, bid, nb)) return;
-  } else {
-    float acc = 0.f;
-    for (int64_t e = (int64_t)bid * blockDim.x + threadIdx.x; e < n; e += (int64_t)nb * blockDim.x)
-      acc += (kind == RED_MEAN) ? ldv(a + e) : ldv(a + e) * b[e];
-    if (!grid_sum((double)acc, rb.partials, &st->ticket, &total, bid, nb)) return;
-  }
-  if (threadIdx.x != 0) return;
+// what the thread with the total of a dot does
+__device__ __forceinline__ void dot_done(SolveState* st, double total, int kind, double eps, double inv_n,
+                                         int max_iters) {
   if (kind == RED_ZTR_INIT) {
     st->zTr_old = total;
     if (max_iters == 0) {  // for i in range(0): no iteration at all
@@ -928,6 +1079,76 @@ __device__ __forceinline__ void dot_blk(const SA* __restrict__ a, const float* _
   }
 }
 
+// sum(a*b) (or sum(a) for RED_MEAN) with a finalizer that updates the solve state.  Per-thread
+// partials accumulate in f32 (the reference solve) or f64 (f64 != 0, the mixed solve).
+template <typename SA, bool RUNS>
+__device__ __forceinline__ void dot_blk(const SA* __restrict__ a, const float* __restrict__ b, int64_t n, RedBuf rb,
+                                        int kind, double eps, double inv_n, int max_iters, int f64, unsigned bid,
+                                        unsigned nb) {
+  SolveState* st = rb.st;
+  if (st->done) return;
+  CompSum acc;
+  const int64_t first = (int64_t)bid * blockDim.x + threadIdx.x, step = (int64_t)nb * blockDim.x;
+  if (RUNS) {
+    for (int64_t e = first * 8; e < n; e += step * 8) {
+      float va[8], vb[8];
+      ld8(a + e, va);
+      if (kind != RED_MEAN) ld8(b + e, vb);
+#pragma unroll
+      for (int q = 0; q < 8; ++q) acc.add(kind == RED_MEAN ? va[q] : va[q] * vb[q]);
+    }
+  } else if (f64) {
+    for (int64_t e = first; e < n; e += step) acc.add((kind == RED_MEAN) ? ldv(a + e) : ldv(a + e) * b[e]);
+  } else {
+    for (int64_t e = first; e < n; e += step) acc.s += (kind == RED_MEAN) ? ldv(a + e) : ldv(a + e) * b[e];
+  }
+  // a 16-bit level vector (z) holds the scaled values: undo the scale of the residual it answers
+  const double us = (f64 && sizeof(SA) == 2) ? 1.0 / (double)st->hscale : 1.0;
+  double total;
+  if (RUNS) {
+    if (!grid_sum(acc, rb.partials, &st->ticket, &total, bid, nb)) return;
+    total *= us;
+  } else if (!grid_sum(acc.value() * us, rb.partials, &st->ticket, &total, bid, nb)) {
+    return;
+  }
+  if (threadIdx.x != 0) return;
+  dot_done(st, total, kind, eps, inv_n, max_iters);
+}
+
+// dot_blk of f32 partials from 16-byte vectors: the same sums, bit for bit (lanes_sum).
+template <bool MEAN>
+__global__ void __launch_bounds__(kLaneThreads) k_dot4(const float* __restrict__ a, const float* __restrict__ b, int64_t n,
+                                                       RedBuf rb, int kind, double eps, double inv_n, int max_iters) {
+  SolveState* st = rb.st;
+  if (st->done) return;
+  constexpr int kDeep = 4;
+  float acc[4] = {0.f, 0.f, 0.f, 0.f};
+  const int64_t step = (int64_t)gridDim.x * kLaneThreads * 4;
+  for (int64_t e0 = ((int64_t)blockIdx.x * kLaneThreads + threadIdx.x) * 4; e0 < n; e0 += kDeep * step) {
+    float av[kDeep][4], bv[kDeep][4];
+#pragma unroll
+    for (int k = 0; k < kDeep; ++k)
+      if (e0 + k * step < n) {
+        ld4(a + e0 + k * step, av[k]);
+        if (!MEAN) ld4(b + e0 + k * step, bv[k]);
+      }
+#pragma unroll
+    for (int k = 0; k < kDeep; ++k) {
+      if (e0 + k * step >= n) break;
+#pragma unroll
+      for (int q = 0; q < 4; ++q) acc[q] = MEAN ? acc[q] + av[k][q] : __fmaf_rn(av[k][q], bv[k][q], acc[q]);
+    }
+  }
+  double d[1][4], total[1];
+#pragma unroll
+  for (int q = 0; q < 4; ++q) d[0][q] = (double)acc[q];
+  if (lanes_sum<1>(d, 1, rb.partials, &st->ticket, total)) dot_done(st, total[0], kind, eps, inv_n, max_iters);
+}
+
+__host__ __device__ __forceinline__ bool dot_runs(int64_t n, int kind, int f64) {
+  return f64 && kind != RED_MEAN && use_runs(n);
+}
+
 template <typename SA>
 struct OpDot {
   const SA* a;
@@ -938,15 +1159,20 @@ struct OpDot {
   double eps, inv_n;
   int max_iters, f64;
   __device__ __forceinline__ void run(unsigned bid, unsigned nb) const {
-    dot_blk<SA>(a, b, n, rb, kind, eps, inv_n, max_iters, f64, bid, nb);
+    if (dot_runs(n, kind, f64))
+      dot_blk<SA, true>(a, b, n, rb, kind, eps, inv_n, max_iters, f64, bid, nb);
+    else
+      dot_blk<SA, false>(a, b, n, rb, kind, eps, inv_n, max_iters, f64, bid, nb);
   }
 };
 
-template <typename SA>
-__global__ void __launch_bounds__(kReduceThreads, kReduceResident) k_dot(const SA* __restrict__ a, const float* __restrict__ b,
+constexpr int red_resident(bool runs) { return runs ? kRunBlocks / 152 : kReduceResident; }
+
+template <typename SA, bool RUNS>
+__global__ void __launch_bounds__(kReduceThreads, red_resident(RUNS)) k_dot(const SA* __restrict__ a, const float* __restrict__ b,
                                                         int64_t n, RedBuf rb, int kind, double eps, double inv_n,
                                                         int max_iters, int f64) {
-  dot_blk<SA>(a, b, n, rb, kind, eps, inv_n, max_iters, f64, blockIdx.x, gridDim.x);
+  dot_blk<SA, RUNS>(a, b, n, rb, kind, eps, inv_n, max_iters, f64, blockIdx.x, gridDim.x);
 }
 
 // recenter (3D/mgpcg.py:174-180): r -= mean; with rh, also the level-storage copy of r that the
@@ -979,6 +1205,24 @@ __global__ void __launch_bounds__(256) k_sub_mean(float* __restrict__ r, S* __re
   sub_mean_blk<S>(r, rh, n, st, blockIdx.x, gridDim.x);
 }
 
+template <typename S>
+__global__ void __launch_bounds__(256) k_sub_mean8(float* __restrict__ r, S* __restrict__ rh, int64_t n,
+                                                   const SolveState* st) {
+  const int64_t e = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) * 8;
+  if (st->done || e >= n) return;
+  const float m = st->mean;
+  const float hs = (sizeof(S) == 2) ? st->hscale : 1.f;
+  float v[8], w[8];
+  ld8(r + e, v);
+#pragma unroll
+  for (int q = 0; q < 8; ++q) {
+    v[q] = v[q] - m;
+    w[q] = v[q] * hs;
+  }
+  st8(r + e, v);
+  if (rh) st8(rh + e, w);
+}
+
 // the level-storage copy of r (mixed solve without recentring)
 template <typename S>
 __device__ __forceinline__ void to_storage_blk(S* __restrict__ out, const float* __restrict__ in, int64_t n,
@@ -1005,29 +1249,66 @@ __global__ void __launch_bounds__(256) k_to_storage(S* __restrict__ out, const f
 }
 
 // compute_Ap + reduce(p, Ap) + alpha = zTr / (pAp + eps)   (3D/mgpcg.py:237-240)
-template <int D>
+template <int D, bool RUNS>
 __device__ __forceinline__ void Ap_dot_blk(const float* __restrict__ p, float* __restrict__ Ap, const Lvl& L,
                                            const BC& bc, RedBuf rb, double eps, int f64, unsigned bid, unsigned nb) {
   SolveState* st = rb.st;
   if (st->done) return;
-  float acc = 0.f;
-  CompSum cacc;
-  for (int64_t e = (int64_t)bid * blockDim.x + threadIdx.x; e < L.count; e += (int64_t)nb * blockDim.x) {
-    int i, j, k;
-    decode(L, e, i, j, k);
-    float nbs, mult;
-    stencil<D>(p, L, bc, i, j, k, e, nbs, mult);
-    float pe = p[e];
-    float ap = mult * pe - nbs;
-    Ap[e] = ap;
-    if (f64) cacc.add(pe * ap);
-    else acc += pe * ap;
+  CompSum acc;
+  const int64_t first = (int64_t)bid * blockDim.x + threadIdx.x, step = (int64_t)nb * blockDim.x;
+  if (RUNS) {
+    for (int64_t e = first; e < L.count / 8; e += step) {
+      float out[8];
+      const int64_t c0 = stencil_run<8>(p, L, bc, (unsigned)e, [&](int q, float pe, float nbs, float mult) {
+        out[q] = mult * pe - nbs;
+        acc.add(pe * out[q]);
+      });
+      st8(Ap + c0, out);
+    }
+  } else {
+    for (int64_t e = first; e < L.count; e += step) {
+      int i, j, k;
+      decode(L, e, i, j, k);
+      float nbs, mult;
+      stencil<D>(p, L, bc, i, j, k, e, nbs, mult);
+      float pe = p[e];
+      float ap = mult * pe - nbs;
+      Ap[e] = ap;
+      if (f64) acc.add(pe * ap);
+      else acc.s += pe * ap;
+    }
   }
   double total;
-  if (!grid_sum(f64 ? cacc.value() : (double)acc, rb.partials, &st->ticket, &total, bid, nb)) return;
+  if (RUNS ? !grid_sum(acc, rb.partials, &st->ticket, &total, bid, nb)
+           : !grid_sum(f64 ? acc.value() : (double)acc.s, rb.partials, &st->ticket, &total, bid, nb))
+    return;
   if (threadIdx.x == 0) {
     st->pAp = total;
     st->alpha = (float)(st->zTr_old / (total + eps));
+  }
+}
+
+// Ap_dot_blk of f32 partials in 3D from 16-byte vectors (n2 % 4 == 0): the same sums, bit for bit (lanes_sum).
+__global__ void __launch_bounds__(kLaneThreads) k_Ap_dot4(const float* __restrict__ p, float* __restrict__ Ap, Lvl L,
+                                                          BC bc, RedBuf rb, double eps) {
+  SolveState* st = rb.st;
+  if (st->done) return;
+  float acc[4] = {0.f, 0.f, 0.f, 0.f};
+  const int64_t step = (int64_t)gridDim.x * kLaneThreads * 4;
+  for (int64_t e = ((int64_t)blockIdx.x * kLaneThreads + threadIdx.x) * 4; e < L.count; e += step) {
+    float out[4];
+    stencil_run<4>(p, L, bc, (unsigned)(e >> 2), [&](int q, float pe, float nbs, float mult) {
+      out[q] = mult * pe - nbs;
+      acc[q] = __fmaf_rn(pe, out[q], acc[q]);
+    });
+    *reinterpret_cast<float4*>(Ap + e) = make_float4(out[0], out[1], out[2], out[3]);
+  }
+  double d[1][4], total[1];
+#pragma unroll
+  for (int q = 0; q < 4; ++q) d[0][q] = (double)acc[q];
+  if (lanes_sum<1>(d, 1, rb.partials, &st->ticket, total)) {
+    st->pAp = total[0];
+    st->alpha = (float)(st->zTr_old / (total[0] + eps));
   }
 }
 
@@ -1040,13 +1321,18 @@ struct OpApDot {
   RedBuf rb;
   double eps;
   int f64;
-  __device__ __forceinline__ void run(unsigned bid, unsigned nb) const { Ap_dot_blk<D>(p, Ap, L, bc, rb, eps, f64, bid, nb); }
+  __device__ __forceinline__ void run(unsigned bid, unsigned nb) const {
+    if (f64 && use_runs<D>(L))
+      Ap_dot_blk<D, D == 3>(p, Ap, L, bc, rb, eps, f64, bid, nb);
+    else
+      Ap_dot_blk<D, false>(p, Ap, L, bc, rb, eps, f64, bid, nb);
+  }
 };
 
-template <int D>
-__global__ void __launch_bounds__(kReduceThreads, kReduceResident) k_Ap_dot(const float* __restrict__ p, float* __restrict__ Ap,
+template <int D, bool RUNS>
+__global__ void __launch_bounds__(kReduceThreads, red_resident(RUNS)) k_Ap_dot(const float* __restrict__ p, float* __restrict__ Ap,
                                                            Lvl L, BC bc, RedBuf rb, double eps, int f64) {
-  Ap_dot_blk<D>(p, Ap, L, bc, rb, eps, f64, blockIdx.x, gridDim.x);
+  Ap_dot_blk<D, RUNS>(p, Ap, L, bc, rb, eps, f64, blockIdx.x, gridDim.x);
 }
 
 // update_x, update_r, reduce(r, r) and the convergence test (3D/mgpcg.py:243-258).  With x64
@@ -1054,6 +1340,20 @@ __global__ void __launch_bounds__(kReduceThreads, kReduceResident) k_Ap_dot(cons
 // for verification (done = 5): k_true_residual, next in the iteration, decides on the true residual.
 // With want_mean the pass also sums the new r for the next recenter (sum(r) / n into st->mean),
 // accumulated and reduced exactly as dot_blk's RED_MEAN pass over the same r would: the same mean.
+__device__ __forceinline__ void update_xr_done(SolveState* st, double total, double tmean, bool want_mean, double tol,
+                                               int tol_mode, double inv_n, bool verify) {
+  if (want_mean) st->mean = (float)(tmean * inv_n);
+  st->rTr = total;
+  if (total > 0.0) st->hscale = (float)(1.0 / sqrt(total * inv_n));
+  if (!isfinite(total)) {
+    st->done = 3;
+    st->conv_it = st->it;
+  } else if (converged(total, st, tol, tol_mode)) {
+    st->done = verify ? 5 : 1;
+    st->conv_it = st->it;
+  }
+}
+
 __device__ __forceinline__ void update_xr_blk(float* __restrict__ x, const float* __restrict__ p, float* __restrict__ r,
                                               const float* __restrict__ Ap, int64_t n, RedBuf rb, double tol,
                                               int tol_mode, int f64, double inv_n, unsigned bid, unsigned nb,
@@ -1086,18 +1386,63 @@ __device__ __forceinline__ void update_xr_blk(float* __restrict__ x, const float
   } else if (!grid_sum(f64 ? cacc.value() : (double)acc, rb.partials, &st->ticket, &total, bid, nb)) {
     return;
   }
-  if (threadIdx.x == 0) {
-    if (want_mean) st->mean = (float)(tmean * inv_n);
-    st->rTr = total;
-    if (total > 0.0) st->hscale = (float)(1.0 / sqrt(total * inv_n));
-    if (!isfinite(total)) {
-      st->done = 3;
-      st->conv_it = st->it;
-    } else if (converged(total, st, tol, tol_mode)) {
-      st->done = x64 ? 5 : 1;
-      st->conv_it = st->it;
+  if (threadIdx.x == 0) update_xr_done(st, total, tmean, want_mean, tol, tol_mode, inv_n, x64 != nullptr);
+}
+
+// update_xr_blk from 16-byte vectors, kAhead of each array in flight: the same sums, bit for bit (lanes_sum).
+constexpr int kAhead = 2;
+
+template <bool F64>
+__global__ void __launch_bounds__(kLaneThreads) k_update_xr4(float* __restrict__ x, const float* __restrict__ p,
+                                                             float* __restrict__ r, const float* __restrict__ Ap,
+                                                             int64_t n, RedBuf rb, double tol, int tol_mode, double inv_n,
+                                                             int want_mean) {
+  SolveState* st = rb.st;
+  if (st->done) return;
+  const float alpha = st->alpha;
+  CompSum acc[4], macc[4];
+  const int64_t step = (int64_t)gridDim.x * kLaneThreads * 4;
+  for (int64_t e0 = ((int64_t)blockIdx.x * kLaneThreads + threadIdx.x) * 4; e0 < n; e0 += kAhead * step) {
+    float pv[kAhead][4], av[kAhead][4], rv[kAhead][4], xv[kAhead][4];
+#pragma unroll
+    for (int a = 0; a < kAhead; ++a) {
+      const int64_t e = e0 + a * step;
+      if (e < n) {
+        ld4(p + e, pv[a]);
+        ld4(Ap + e, av[a]);
+        ld4(r + e, rv[a]);
+        ld4(x + e, xv[a]);
+      }
+    }
+#pragma unroll
+    for (int a = 0; a < kAhead; ++a) {
+      const int64_t e = e0 + a * step;
+      if (e >= n) break;
+#pragma unroll
+      for (int q = 0; q < 4; ++q) {
+        xv[a][q] += alpha * pv[a][q];
+        const float re = rv[a][q] - alpha * av[a][q];
+        rv[a][q] = re;
+        if (F64) {
+          acc[q].add(re * re);
+          if (want_mean) macc[q].add(re);
+        } else {
+          acc[q].s += re * re;
+          if (want_mean) macc[q].s += re;
+        }
+      }
+      *reinterpret_cast<float4*>(x + e) = make_float4(xv[a][0], xv[a][1], xv[a][2], xv[a][3]);
+      *reinterpret_cast<float4*>(r + e) = make_float4(rv[a][0], rv[a][1], rv[a][2], rv[a][3]);
     }
   }
+  double d[2][4], total[2] = {0.0, 0.0};
+#pragma unroll
+  for (int q = 0; q < 4; ++q) {
+    d[0][q] = F64 ? acc[q].value() : (double)acc[q].s;
+    d[1][q] = F64 ? macc[q].value() : (double)macc[q].s;
+  }
+  if (lanes_sum<2>(d, want_mean ? 2 : 1, rb.partials, &st->ticket, total))
+    update_xr_done(st, total[0], total[1], want_mean != 0, tol, tol_mode, inv_n, false);
 }
 
 struct OpUpdateXr {
@@ -1201,23 +1546,37 @@ __device__ __forceinline__ void true_residual_replace_blk(const float* __restric
   }
 }
 
-template <int D>
+template <int D, bool RUNS>
 __device__ __forceinline__ void true_residual_blk(const float* __restrict__ b, const float* __restrict__ x,
                                                   const Lvl& L, const BC& bc, RedBuf rb, int every, unsigned bid,
                                                   unsigned nb) {
   SolveState* st = rb.st;
   if (every > 0 && (st->done != 0 || (st->it + 1) % every != 0)) return;
   CompSum acc;
-  for (int64_t e = (int64_t)bid * blockDim.x + threadIdx.x; e < L.count; e += (int64_t)nb * blockDim.x) {
-    int i, j, k;
-    decode(L, e, i, j, k);
-    float nbs, mult;
-    stencil<D>(x, L, bc, i, j, k, e, nbs, mult);
-    const float re = b[e] - (mult * x[e] - nbs);
-    acc.add(re * re);
+  const int64_t first = (int64_t)bid * blockDim.x + threadIdx.x, step = (int64_t)nb * blockDim.x;
+  if (RUNS) {
+    for (int64_t e = first; e < L.count / 8; e += step) {
+      float bb[8];
+      ld8(b + e * 8, bb);
+      stencil_run<8>(x, L, bc, (unsigned)e, [&](int q, float xe, float nbs, float mult) {
+        const float re = bb[q] - (mult * xe - nbs);
+        acc.add(re * re);
+      });
+    }
+  } else {
+    for (int64_t e = first; e < L.count; e += step) {
+      int i, j, k;
+      decode(L, e, i, j, k);
+      float nbs, mult;
+      stencil<D>(x, L, bc, i, j, k, e, nbs, mult);
+      const float re = b[e] - (mult * x[e] - nbs);
+      acc.add(re * re);
+    }
   }
   double total;
-  if (!grid_sum(acc.value(), rb.partials, &st->ticket, &total, bid, nb)) return;
+  if (RUNS ? !grid_sum(acc, rb.partials, &st->ticket, &total, bid, nb)
+           : !grid_sum(acc.value(), rb.partials, &st->ticket, &total, bid, nb))
+    return;
   if (threadIdx.x == 0) st->rTr_true = total;
 }
 
@@ -1237,16 +1596,18 @@ struct OpTrueResidual {
   __device__ __forceinline__ void run(unsigned bid, unsigned nb) const {
     if (x64)
       true_residual_replace_blk<D>(b, x64, r, L, bc, rb, every, tol, tol_mode, inv_n, bid, nb);
+    else if (use_runs<D>(L))
+      true_residual_blk<D, D == 3>(b, x, L, bc, rb, every, bid, nb);
     else
-      true_residual_blk<D>(b, x, L, bc, rb, every, bid, nb);
+      true_residual_blk<D, false>(b, x, L, bc, rb, every, bid, nb);
   }
 };
 
-template <int D>
-__global__ void __launch_bounds__(kReduceThreads, kReduceResident) k_true_residual(const float* __restrict__ b,
+template <int D, bool RUNS>
+__global__ void __launch_bounds__(kReduceThreads, red_resident(RUNS)) k_true_residual(const float* __restrict__ b,
                                                                   const float* __restrict__ x, Lvl L, BC bc,
                                                                   RedBuf rb, int every) {
-  true_residual_blk<D>(b, x, L, bc, rb, every, blockIdx.x, gridDim.x);
+  true_residual_blk<D, RUNS>(b, x, L, bc, rb, every, blockIdx.x, gridDim.x);
 }
 
 template <int D>
@@ -1287,6 +1648,20 @@ template <typename SZ>
 __global__ void __launch_bounds__(256) k_update_p(float* __restrict__ p, const SZ* __restrict__ z, int64_t n,
                                                   const SolveState* st) {
   update_p_blk<SZ>(p, z, n, st, blockIdx.x, gridDim.x);
+}
+
+template <typename SZ>
+__global__ void __launch_bounds__(256) k_update_p8(float* __restrict__ p, const SZ* __restrict__ z, int64_t n,
+                                                   const SolveState* st) {
+  const int64_t e = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) * 8;
+  if (st->done || e >= n) return;
+  const float beta = st->beta, us = sizeof(SZ) == 2 ? 1.f / st->hscale : 1.f;
+  float v[8], w[8];
+  ld8(p + e, v);
+  ld8(z + e, w);
+#pragma unroll
+  for (int q = 0; q < 8; ++q) v[q] = sizeof(SZ) == 2 ? w[q] * us + beta * v[q] : w[q] + beta * v[q];
+  st8(p + e, v);
 }
 
 // Device loop control.  The loop body is the second half of iteration k (recenter, V-cycle, beta,
@@ -1496,9 +1871,24 @@ struct OpTail {
 // ---------------------------------------------------------------------------------------------
 // host orchestration
 // ---------------------------------------------------------------------------------------------
-static unsigned red_blocks(int64_t n) {
-  unsigned b = grid_for(n, kReduceThreads);
-  return b > (unsigned)kReduceBlocks ? (unsigned)kReduceBlocks : b;
+static unsigned red_blocks(int64_t n, bool runs) {
+  const unsigned b = grid_for(runs ? n / 8 : n, kReduceThreads), most = runs ? kRunBlocks : kReduceBlocks;
+  return b > most ? most : b;
+}
+template <int D>
+static unsigned red_blocks(const Lvl& L) { return red_blocks(L.count, use_runs<D>(L)); }
+
+template <typename SA>
+static void launch_dot(pfm_handle* h, cudaStream_t q, const SA* a, const float* b, int64_t n, RedBuf rb, int kind,
+                       double eps, double inv_n, int max_iters, int f64) {
+  const bool runs = dot_runs(n, kind, f64);
+  if (!f64 && use_lanes(n) && std::is_same<SA, float>::value) {
+    launch(h, kind == RED_MEAN ? k_dot4<true> : k_dot4<false>, red_blocks(n, false), kLaneThreads, 0, q, (const float*)a, b,
+           n, rb, kind, eps, inv_n, max_iters);
+    return;
+  }
+  launch(h, runs ? k_dot<SA, true> : k_dot<SA, false>, red_blocks(n, runs), kReduceThreads, 0, q, a, b, n, rb, kind, eps,
+         inv_n, max_iters, f64);
 }
 
 // Elementwise kernels: one wave of 8 resident 256-thread blocks per SM (every block loops over an
@@ -1790,23 +2180,42 @@ struct SolveKernels {
     S* out = (mixed && storage) ? rh : nullptr;
     if (neu) {
       if (!mean_ready)
-        launch(h, k_dot<float>, red_blocks(n), kReduceThreads, 0, q, (const float*)r0, (const float*)nullptr, n, rb,
-               (int)RED_MEAN, o.eps, inv_n, mi, f64);
-      launch(h, k_sub_mean<S>, stream_blocks(n), 256, 0, q, r0, out, n, (const SolveState*)st);
+        launch_dot<float>(h, q, r0, nullptr, n, rb, (int)RED_MEAN, o.eps, inv_n, mi, f64);
+      if (use_runs(n))
+        launch(h, k_sub_mean8<S>, grid_for(n / 8, 256), 256, 0, q, r0, out, n, (const SolveState*)st);
+      else
+        launch(h, k_sub_mean<S>, stream_blocks(n), 256, 0, q, r0, out, n, (const SolveState*)st);
     } else if (out) {
       launch(h, k_to_storage<S>, stream_blocks(n), 256, 0, q, out, (const float*)r0, n, (const SolveState*)st);
     }
   }
   void first_half(cudaStream_t q) {
-    launch(h, k_Ap_dot<D>, red_blocks(n), kReduceThreads, 0, q, (const float*)p, Ap, L0, bc, rb, o.eps, f64);
-    launch(h, k_update_xr, red_blocks(n), kReduceThreads, 0, q, x, (const float*)p, r0, (const float*)Ap, n, rb, o.tol,
-           o.tol_mode, f64, inv_n, x64, fuse_mean ? 1 : 0);
+    if (D == 3 && !f64 && L0.n2 % 4 == 0 && use_lanes(n))
+      launch(h, k_Ap_dot4, red_blocks(n, false), kLaneThreads, 0, q, (const float*)p, Ap, L0, bc, rb, o.eps);
+    else
+      launch(h, f64 && use_runs<D>(L0) ? k_Ap_dot<D, D == 3> : k_Ap_dot<D, false>,
+             red_blocks(n, f64 && use_runs<D>(L0)), kReduceThreads, 0, q, (const float*)p, Ap, L0, bc, rb, o.eps, f64);
+    if (!x64 && use_lanes(n))
+      launch(h, f64 ? k_update_xr4<true> : k_update_xr4<false>, red_blocks(n, false), kLaneThreads, 0, q, x, (const float*)p, r0, (const float*)Ap, n, rb,
+             o.tol, o.tol_mode, inv_n, fuse_mean ? 1 : 0);
+    else
+      launch(h, k_update_xr, red_blocks(n, false), kReduceThreads, 0, q, x, (const float*)p, r0, (const float*)Ap, n, rb,
+             o.tol, o.tol_mode, f64, inv_n, x64, fuse_mean ? 1 : 0);
     if (replace)
-      launch(h, k_true_residual_replace<D>, red_blocks(n), kReduceThreads, 0, q, (const float*)bvec,
+      launch(h, k_true_residual_replace<D>, red_blocks(n, false), kReduceThreads, 0, q, (const float*)bvec,
              (const double*)x64, r0, L0, bc, rb, o.true_residual_every, o.tol, o.tol_mode, inv_n);
     else if (true_res)
-      launch(h, k_true_residual<D>, red_blocks(n), kReduceThreads, 0, q, (const float*)bvec, (const float*)x, L0, bc, rb,
-             o.true_residual_every);
+      launch_true_residual(q, o.true_residual_every);
+  }
+  void launch_true_residual(cudaStream_t q, int every) {
+    launch(h, use_runs<D>(L0) ? k_true_residual<D, D == 3> : k_true_residual<D, false>, red_blocks<D>(L0), kReduceThreads, 0,
+           q, (const float*)bvec, (const float*)x, L0, bc, rb, every);
+  }
+  void update_p(cudaStream_t q) {
+    if (use_runs(n))
+      launch(h, k_update_p8<S>, grid_for(n / 8, 256), 256, 0, q, p, (const S*)z0, n, (const SolveState*)st);
+    else
+      launch(h, k_update_p<S>, stream_blocks(n), 256, 0, q, p, (const S*)z0, n, (const SolveState*)st);
   }
   void setup(cudaStream_t q) {
     // init(): x = p = Ap = 0 (3D/mgpcg.py:63-79); z0 is zeroed by the V-cycle, and Ap needs no
@@ -1817,8 +2226,7 @@ struct SolveKernels {
     recenter(q, false);
     if (keep_b) {
       cudaMemcpyAsync(bvec, r0, n * 4, cudaMemcpyDeviceToDevice, q);
-      launch(h, k_dot<float>, red_blocks(n), kReduceThreads, 0, q, (const float*)bvec, (const float*)bvec, n, rb,
-             (int)RED_BTB, o.eps, inv_n, mi, 1);
+      launch_dot<float>(h, q, bvec, bvec, n, rb, (int)RED_BTB, o.eps, inv_n, mi, 1);
     }
     if (warm) {
       if (D == 3 && L0.n2 % 8 == 0)
@@ -1827,22 +2235,19 @@ struct SolveKernels {
         launch(h, k_residual<D>, stream_blocks(n), 256, 0, q, r0, (const float*)bvec, (const float*)x, L0, bc);
     }
     if (replace) launch(h, k_x_to64, stream_blocks(n), 256, 0, q, x64, (const float*)x, n, (const SolveState*)st);
-    launch(h, k_dot<float>, red_blocks(n), kReduceThreads, 0, q, (const float*)r0, (const float*)r0, n, rb,
-           (int)RED_RTR0, o.eps, inv_n, mi, f64);
+    launch_dot<float>(h, q, r0, r0, n, rb, (int)RED_RTR0, o.eps, inv_n, mi, f64);
     // the scaled level-storage copy of r0, once r0.r0 (and so the scale) is known
     if (mixed) launch(h, k_to_storage<S>, stream_blocks(n), 256, 0, q, rh, (const float*)r0, n, (const SolveState*)st);
     vcycle<D, S>(h, st, q);
-    launch(h, k_update_p<S>, stream_blocks(n), 256, 0, q, p, (const S*)z0, n, (const SolveState*)st);
-    launch(h, k_dot<S>, red_blocks(n), kReduceThreads, 0, q, (const S*)z0, (const float*)r0, n, rb, (int)RED_ZTR_INIT,
-           o.eps, inv_n, mi, f64);
+    update_p(q);
+    launch_dot<S>(h, q, z0, r0, n, rb, (int)RED_ZTR_INIT, o.eps, inv_n, mi, f64);
     first_half(q);
   }
   void body(cudaStream_t q, cudaGraphConditionalHandle cond) {
     recenter(q, true, fuse_mean);
     vcycle<D, S>(h, st, q);
-    launch(h, k_dot<S>, red_blocks(n), kReduceThreads, 0, q, (const S*)z0, (const float*)r0, n, rb, (int)RED_ZTR, o.eps,
-           inv_n, mi, f64);
-    launch(h, k_update_p<S>, stream_blocks(n), 256, 0, q, p, (const S*)z0, n, (const SolveState*)st);
+    launch_dot<S>(h, q, z0, r0, n, rb, (int)RED_ZTR, o.eps, inv_n, mi, f64);
+    update_p(q);
     first_half(q);
     launch(h, k_loop_cond, 1, 1, 0, q, (const SolveState*)st, cond);
   }
@@ -1850,8 +2255,7 @@ struct SolveKernels {
     if (replace)  // the FP32 pressure the caller receives
       launch(h, k_x_from64, stream_blocks(n), 256, 0, q, x, (const double*)x64, n);
     if (true_res)  // the final true residual of the solve (of the FP32 pressure)
-      launch(h, k_true_residual<D>, red_blocks(n), kReduceThreads, 0, q, (const float*)bvec, (const float*)x, L0, bc, rb,
-             -1);
+      launch_true_residual(q, -1);
   }
 };
 
@@ -2393,7 +2797,8 @@ static void batched_body(std::vector<BatchScene<D, S>>& B, cudaStream_t q) {
     for (auto& b : B) {
       auto& K = b.K;
       if (K.neu) {
-        mean.add(OpDot<float>{K.r0, nullptr, K.n, K.rb, (int)RED_MEAN, K.o.eps, K.inv_n, K.mi, K.f64}, red_blocks(K.n));
+        mean.add(OpDot<float>{K.r0, nullptr, K.n, K.rb, (int)RED_MEAN, K.o.eps, K.inv_n, K.mi, K.f64},
+                 red_blocks(K.n, dot_runs(K.n, RED_MEAN, K.f64)));
         sub.add(OpSubMean<S>{K.r0, K.mixed ? K.rh : nullptr, K.n, K.st}, stream_blocks(K.n));
       } else if (K.mixed) {
         sto.add(OpToStorage<S>{K.rh, K.r0, K.n, K.st}, stream_blocks(K.n));
@@ -2411,14 +2816,17 @@ static void batched_body(std::vector<BatchScene<D, S>>& B, cudaStream_t q) {
   WorkItems<OpTrueResidual<D>> tr;
   for (auto& b : B) {
     auto& K = b.K;
-    ztr.add(OpDot<S>{K.z0, K.r0, K.n, K.rb, (int)RED_ZTR, K.o.eps, K.inv_n, K.mi, K.f64}, red_blocks(K.n));
+    ztr.add(OpDot<S>{K.z0, K.r0, K.n, K.rb, (int)RED_ZTR, K.o.eps, K.inv_n, K.mi, K.f64},
+            red_blocks(K.n, dot_runs(K.n, RED_ZTR, K.f64)));
     up.add(OpUpdateP<S>{K.p, K.z0, K.n, K.st}, stream_blocks(K.n));
-    ap.add(OpApDot<D>{K.p, K.Ap, K.L0, K.bc, K.rb, K.o.eps, K.f64}, red_blocks(K.n));
-    xr.add(OpUpdateXr{K.x, K.p, K.r0, K.Ap, K.n, K.rb, K.o.tol, K.o.tol_mode, K.f64, K.inv_n, K.x64}, red_blocks(K.n));
+    ap.add(OpApDot<D>{K.p, K.Ap, K.L0, K.bc, K.rb, K.o.eps, K.f64},
+           red_blocks(K.n, K.f64 && use_runs<D>(K.L0)));
+    xr.add(OpUpdateXr{K.x, K.p, K.r0, K.Ap, K.n, K.rb, K.o.tol, K.o.tol_mode, K.f64, K.inv_n, K.x64},
+           red_blocks(K.n, false));
     if (K.true_res)
       tr.add(OpTrueResidual<D>{K.bvec, K.x, K.L0, K.bc, K.rb, K.o.true_residual_every, K.x64, K.r0, K.o.tol,
                                K.o.tol_mode, K.inv_n},
-             red_blocks(K.n));
+             K.x64 ? red_blocks(K.n, false) : red_blocks<D>(K.L0));
   }
   launch_worklist<OpDot<S>, kReduceThreads>(h0, q, ztr);
   launch_worklist<OpUpdateP<S>, 256>(h0, q, up);

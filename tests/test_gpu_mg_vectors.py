@@ -1,0 +1,41 @@
+"""The solver's vector passes over grids just above the size from which they use 16-byte vectors: a scene stepped
+alone (vectors; sums over lanes in FP32, runs of eight in the mixed solve) against the same scene in a work-list
+batch, whose FP32 passes take one element per thread -- bitwise, as the sums keep their order -- with rows of a
+multiple of 8, of 4 and of neither."""
+import pytest
+
+torch = pytest.importorskip("torch")
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("opts", [dict(tol=1e-6, tol_mode=1, max_iters=60),
+                                  dict(tol=1e-6, tol_mode=2, max_iters=60, precision="fp16", warm_start=3,
+                                       true_residual_every=2)])
+def test_vector_passes_equal_worklist(opts):
+    import pfm
+    from pfm import _lib
+
+    def make(res, graph):
+        dx = 1.0 / res[1]
+        g = torch.Generator(device="cuda").manual_seed(sum(res))
+        u = [torch.randn([n + (a == f) for a, n in enumerate(res)], device="cuda", generator=g) for f in range(3)]
+        for f in range(3):
+            u[f].select(f, 0).zero_()
+            u[f].select(f, res[f]).zero_()
+        sim = pfm.Sim3D(u, pfm.jittered(res, dx, 8, seed=2), res, dx, reinit_every=4, poisson_opts=opts, graph=graph)
+        sim.scene.set_tuning(_lib.TUNE_MG_CLUSTER, 0)
+        return sim
+
+    specs = [(48, 40, 40), (48, 48, 36), (48, 40, 42)]
+    alone = [make(s, False) for s in specs]
+    together = [make(s, True) for s in specs]
+    batch = pfm.Batch(together, worklist=True)
+    for _ in range(2):
+        for sim in alone:
+            sim.step()
+        batch.step()
+    torch.cuda.synchronize()
+    for a, b in zip(alone, together):
+        assert torch.equal(a.p, b.p)
+        for f in range(3):
+            assert torch.equal(a.u[f], b.u[f])
