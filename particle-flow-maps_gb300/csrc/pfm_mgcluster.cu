@@ -27,8 +27,8 @@
 // cluster or block barriers that all threads reach the same number of times: the branches around them
 // depend only on values every CTA computes alike.
 //
-// Measured (one PCG iteration, FP32, GB300): 128^2 103 -> 26 us, 256^2 125 -> 35 us, 512^2 165 -> 59 us,
-// 32^3 107 -> 32 us, 64^3 155 -> 63 us; the coarse levels of 128^3 and 1024^2 as one launch: 210 -> 185 and
+// Measured (one PCG iteration, FP32, GB300): 128^2 103 -> 23 us, 256^2 125 -> 31 us, 512^2 165 -> 54 us,
+// 32^3 107 -> 28 us, 64^3 155 -> 60 us; the coarse levels of 128^3 and 1024^2 as one launch: 210 -> 185 and
 // 180 -> 141 us per iteration.  What bounds it: the chain of half-sweeps -- about 850 cycles each on the
 // distributed levels (a row's flight through the cluster is some 400 of them), 60 to 200 on the solo ones.
 #include <cooperative_groups.h>
@@ -267,6 +267,7 @@ __device__ __forceinline__ void update_spot(const F* __restrict__ zo, const F* _
 // half-sweep early overwrites nothing that is still to be read: it has the colour not read.
 struct Exchange {
   uint64_t full[2];  // in shared memory, one arrival (the expected bytes) per half-sweep
+  uint64_t up, down;  // per V-cycle: the solo level's r is complete (rank 0); its z rows are here (the others)
   int lost;          // a row did not arrive in time: later waits return at once
 };
 
@@ -497,11 +498,12 @@ __device__ __forceinline__ void sweeps_planes(const CLev& v, const BC& bc, float
 // The restriction of the fine rows under the coarse rows [c_lo, c_lo + c_rows) into rc (its row 0 the
 // coarse row c_base): restrict_blk's sums in its order, four coarse cells along the last axis at a time
 // (the four cells of either colour of the fine rows under them).  zf, rf: the fine level's vectors with
-// the fine row f_lo first (zf past its ghost row).
+// the fine row f_lo first (zf past its ghost row).  With `push` rc is that shared address of another CTA, and the
+// cells go there by st.async on its `bar` (16 bytes per vector, the cells beyond the last axis included).
 template <int D, typename R, typename F, typename C>
 __device__ __forceinline__ void restrict_rows(const CLev& vf, const CLev& vc, const BC& bc, const F* __restrict__ zf,
                                               const F* __restrict__ rf, int f_lo, C* __restrict__ rc, int c_base,
-                                              int c_lo, int c_rows) {
+                                              int c_lo, int c_rows, uint32_t push = 0, uint32_t bar = 0) {
   const int hv = vf.hs >> 2, T = c_rows * vc.n1 * hv, pad = (vf.rmax + 1) * vf.plane;
 #pragma unroll 1
   for (int t = threadIdx.x; t < T; t += kT) {
@@ -514,7 +516,7 @@ __device__ __forceinline__ void restrict_rows(const CLev& vf, const CLev& vc, co
     }
     const int I = c_lo + il;
     float acc[4] = {0.f, 0.f, 0.f, 0.f};
-#pragma unroll 1
+#pragma unroll(D == 3 ? 1 : 2)
     for (int ab = 0; ab < (D == 3 ? 4 : 2); ++ab) {
       const int i = 2 * I + (D == 3 ? ab >> 1 : ab), j = D == 3 ? 2 * J + (ab & 1) : 0;
       const int fc = (i + j) & 1;  // colour of the even cells (a = 0); the odd ones have the other
@@ -542,7 +544,15 @@ __device__ __forceinline__ void restrict_rows(const CLev& vf, const CLev& vc, co
         acc[q] += e1 * 1.0f / ((float)D - 1.0f);
       }
     }
-    C* dst = rc + (I - c_base) * vc.plane + J * vc.hs;
+    const int at = (I - c_base) * vc.plane + J * vc.hs;
+    if (sizeof(C) == 4 && push) {
+      const float even[2] = {through<R>(acc[0]), through<R>(acc[2])}, odd[2] = {through<R>(acc[1]), through<R>(acc[3])};
+      const int c0 = (I + J) & 1;  // K is a multiple of 4
+      push_async<8>(push + 4u * (uint32_t)(c0 * vc.cr + at + (K >> 1)), even, bar);
+      push_async<8>(push + 4u * (uint32_t)((1 - c0) * vc.cr + at + (K >> 1)), odd, bar);
+      continue;
+    }
+    C* dst = rc + at;
 #pragma unroll
     for (int q = 0; q < 4; ++q)
       if (K + q < vc.nk) stv(dst + ((I + J + K + q) & 1) * vc.cr + ((K + q) >> 1), through<R>(acc[q]));
@@ -550,10 +560,11 @@ __device__ __forceinline__ void restrict_rows(const CLev& vf, const CLev& vc, co
 }
 
 // z_l += z_{l+1}[I//2] on the fine rows [i0, i1) (row f_lo first in zf); zc holds the coarse row
-// c_lo first.  Both cells of a pair (2h, 2h + 1) lie under the coarse cell h.
+// c_lo first.  Both cells of a pair (2h, 2h + 1) lie under the coarse cell h.  Of the rows outside [o0, o1), the
+// ghost rows, only colour 0 is updated.
 template <int D, typename R, typename F, typename C>
 __device__ __forceinline__ void prolong_rows(const CLev& vf, const CLev& vc, F* __restrict__ zf, int f_lo, int i0,
-                                             int i1, const C* __restrict__ zc, int c_lo) {
+                                             int i1, int o0, int o1, const C* __restrict__ zc, int c_lo) {
   const int T = (i1 - i0) * vf.plane / 4;
 #pragma unroll 1
   for (int t = threadIdx.x; t < T; t += kT) {
@@ -566,10 +577,11 @@ __device__ __forceinline__ void prolong_rows(const CLev& vf, const CLev& vc, F* 
     ldvec<2>(src + even, p);
     ldvec<2>(src + odd, s);
     const float add[4] = {p[0], s[0], p[1], s[1]};
-    float f[4], g[4];
+    float f[4], g[4] = {0.f, 0.f, 0.f, 0.f};
     F* a = zf + (i - f_lo) * vf.plane + j * vf.hs + h;
+    const bool own = i >= o0 && i < o1;
     ldvec<4>(a, f);
-    ldvec<4>(a + vf.cz, g);
+    if (own) ldvec<4>(a + vf.cz, g);
 #pragma unroll
     for (int q = 0; q < 4; ++q)
       if (h + q < vf.half) {
@@ -577,7 +589,7 @@ __device__ __forceinline__ void prolong_rows(const CLev& vf, const CLev& vc, F* 
         g[q] += through<R>(add[q]);
       }
     *reinterpret_cast<Vec<4, F>*>(a) = pack<4, F>(f);
-    *reinterpret_cast<Vec<4, F>*>(a + vf.cz) = pack<4, F>(g);
+    if (own) *reinterpret_cast<Vec<4, F>*>(a + vf.cz) = pack<4, F>(g);
   }
 }
 
@@ -595,7 +607,7 @@ __device__ __forceinline__ void solo_vcycle(const CPlan& P, unsigned char* sm, c
     const CLev v = P.lv[l];
     if (t > n) {
       const CLev c = P.lv[l + 1];
-      prolong_rows<D, float, float, float>(v, c, Z(l) + v.plane, 0, 0, v.n0, Z(l + 1) + c.plane, 0);
+      prolong_rows<D, float, float, float>(v, c, Z(l) + v.plane, 0, 0, v.n0, 0, v.n0, Z(l + 1) + c.plane, 0);
       __syncthreads();
     }
     if (t == n && fits_planes<D>(v))
@@ -610,18 +622,54 @@ __device__ __forceinline__ void solo_vcycle(const CPlan& P, unsigned char* sm, c
   }
 }
 
+// The coarse rows under the fine rows [lo - 1, lo + rows] of a share (its own and the ghost rows inside the grid).
+struct Under {
+  int first, rows;
+};
+__device__ __forceinline__ Under rows_under(const CLev& v, int lo, int rows) {
+  const int i0 = lo > 0 ? lo - 1 : 0, i1 = lo + rows < v.n0 ? lo + rows + 1 : v.n0;
+  return Under{i0 >> 1, ((i1 - 1) >> 1) - (i0 >> 1) + 1};
+}
+
+// Rank 0's z of the solo level into the other CTAs, each the rows under its share, at their place in its own
+// (otherwise unused) memory of that level: a warp per CTA.
+__device__ __forceinline__ void push_solo(const CPlan& P, const CLev& v, const CLev& c, unsigned char* sm, Exchange* ex) {
+  const int rank = (int)threadIdx.x >> 5;
+  if (rank == 0 || rank >= P.nc) return;
+  const int b0 = rank * P.nbase / P.nc, b1 = (rank + 1) * P.nbase / P.nc;
+  const Under u = rows_under(v, b0 << v.shift, (b1 - b0) << v.shift);
+  const float* z = reinterpret_cast<const float*>(sm + c.z);
+  const uint32_t dst = remote_addr(su32(z), rank), bar = remote_addr(su32(&ex->down), rank);
+  const int n = u.rows * c.plane, base = (u.first + 1) * c.plane;
+  for (int e = (int)(threadIdx.x & 31) * 4; e < 2 * n; e += 128) {
+    const int at = base + (e < n ? e : e - n + c.cz);
+    const float4 q = *reinterpret_cast<const float4*>(z + at);
+    push_async<16>(dst + 4u * (uint32_t)at, &q, bar);
+  }
+}
+
 // apply_preconditioner (3D/mgpcg.py:182-200) from r of level l0 to its z.  Every thread of the
-// cluster calls it; r of level l0 must be visible to its own CTA.
+// cluster calls it; r of level l0 must be visible to its own CTA.  `cycles` numbers the calls.
+// Between the distributed levels and the solo ones the rows travel by st.async, and a CTA waits for what it
+// reads only (remote stores and loads between cluster barriers took 4400 cycles down and 5000 up at 64^2 solo
+// cells; an iteration at 128^2 went from 26.0 to 23.1 us, at 32^3 from 32 to 28.4).  A ghost row takes its coarse rows in colour 0 only (the other is pushed by
+// the first half-sweep up before anything reads it), so that no barrier parts the prolongation from that push.
 template <int D, typename S>
 __device__ __forceinline__ void cluster_vcycle(const CPlan& P, unsigned char* sm, const float2* inv, Exchange* ex,
-                                               const Me& me, unsigned& count) {
+                                               const Me& me, unsigned& count, unsigned& cycles) {
   const int bottom = P.L - 1, n = (P.lg < P.L ? P.lg : bottom) - P.l0;  // distributed levels that restrict
+  const unsigned parity = cycles++ & 1u;
   // down: t = 0 .. n-1; the solo levels or the distributed bottom: t = n; up: t = n+1 .. 2n
 #pragma unroll 1
   for (int t = 0; t <= 2 * n; ++t) {
     if (t == n && P.lg < P.L) {
-      if (me.rank == 0) solo_vcycle<D>(P, sm, inv);
-      cluster_barrier();
+      if (me.rank == 0) {
+        const CLev v = P.lv[P.lg - 1], c = P.lv[P.lg];
+        if (threadIdx.x == 0) mbar_expect_tx(&ex->up, (unsigned)(c.n0 * c.n1 * (v.hs >> 2) * 16));
+        wait_rows(ex, &ex->up, parity);
+        solo_vcycle<D>(P, sm, inv);
+        push_solo(P, v, c, sm, ex);
+      }
       continue;
     }
     const int l = P.l0 + (t <= n ? t : 2 * n - t);
@@ -630,13 +678,19 @@ __device__ __forceinline__ void cluster_vcycle(const CPlan& P, unsigned char* sm
     S* z = reinterpret_cast<S*>(sm + v.z) + v.plane;
     if (t > n) {
       const CLev c = P.lv[l + 1];
-      // the ghost rows take their coarse rows too: no exchange before the next half-sweep
       const int i0 = s.lo > 0 ? s.lo - 1 : 0, i1 = s.lo + s.rows < v.n0 ? s.lo + s.rows + 1 : v.n0;
-      if (l + 1 < P.lg)
-        prolong_rows<D, S, S, S>(v, c, z, s.lo, i0, i1, reinterpret_cast<const S*>(sm + c.z) + c.plane, s.lo >> 1);
-      else
-        prolong_rows<D, S, S, float>(v, c, z, s.lo, i0, i1, remote(reinterpret_cast<float*>(sm + c.z), 0) + c.plane, 0);
-      cluster_barrier();
+      if (l + 1 < P.lg) {
+        prolong_rows<D, S, S, S>(v, c, z, s.lo, i0, i1, s.lo, s.lo + s.rows, reinterpret_cast<const S*>(sm + c.z) + c.plane,
+                                 s.lo >> 1);
+      } else {
+        if (me.rank > 0) {
+          if (threadIdx.x == 0) mbar_expect_tx(&ex->down, (unsigned)(rows_under(v, s.lo, s.rows).rows * c.plane * 8));
+          wait_rows(ex, &ex->down, parity);
+        }
+        prolong_rows<D, S, S, float>(v, c, z, s.lo, i0, i1, s.lo, s.lo + s.rows,
+                                     reinterpret_cast<const float*>(sm + c.z) + c.plane, 0);
+      }
+      __syncthreads();
     }
     const int iters = t == n ? P.bottom : P.pre_post, first = t > n ? 1 : 0;
     sweeps_dist<D, S>(P, v, sm, inv, ex, me, 2 * iters, first, t <= n, count);
@@ -648,9 +702,9 @@ __device__ __forceinline__ void cluster_vcycle(const CPlan& P, unsigned char* sm
                                s.rows >> 1);
         __syncthreads();
       } else {
-        restrict_rows<D, S, S, float>(v, c, P.bc, z, r, s.lo, remote(reinterpret_cast<float*>(sm + c.r), 0), 0, s.lo >> 1,
-                                   s.rows >> 1);
-        cluster_barrier();
+        float* rc = reinterpret_cast<float*>(sm + c.r);
+        restrict_rows<D, S, S, float>(v, c, P.bc, z, r, s.lo, rc, 0, s.lo >> 1, s.rows >> 1, remote_addr(su32(rc), 0),
+                                   remote_addr(su32(&ex->up), 0));
       }
     }
   }
@@ -669,6 +723,8 @@ __device__ __forceinline__ void init_exchange(Exchange* ex) {
   if (threadIdx.x == 0) {
     mbar_init(&ex->full[0], 1);
     mbar_init(&ex->full[1], 1);
+    mbar_init(&ex->up, 1);
+    mbar_init(&ex->down, 1);
     ex->lost = 0;
     fence_mbar_init();
   }
@@ -706,7 +762,7 @@ __global__ void __launch_bounds__(kT, 1) k_cluster_tail(S* __restrict__ zg, cons
   __shared__ Exchange ex;
   if (st && st->done) return;  // the same for the whole cluster
   const Me me = who_am_i(P);
-  unsigned count = 0;
+  unsigned count = 0, cycles = 0;
   init_exchange(&ex);
   fill_inverses(inv);
   zero_z<S>(P, me, sm);
@@ -731,7 +787,7 @@ __global__ void __launch_bounds__(kT, 1) k_cluster_tail(S* __restrict__ zg, cons
     if (both) r[(1 - c) * v.cr + e] = rg[g + 1];
   }
   cluster_barrier();  // every CTA of the cluster runs before the first remote store
-  cluster_vcycle<D, S>(P, sm, inv, &ex, me, count);
+  cluster_vcycle<D, S>(P, sm, inv, &ex, me, count, cycles);
   const S* z = reinterpret_cast<const S*>(sm + v.z) + v.plane;
   for (int t = threadIdx.x; t < T; t += kT) {
     int e, c;
@@ -822,7 +878,7 @@ __global__ void __launch_bounds__(kT, 1) k_cluster_solve(const __grid_constant__
   constexpr bool MIXED = sizeof(S) == 2;
   const Me me = who_am_i(P);
   const int rank = me.rank, tid = threadIdx.x;
-  unsigned count = 0;
+  unsigned count = 0, cycles = 0;
   init_exchange(&ex);
   fill_inverses(inv);
   zero_z<S>(P, me, sm);
@@ -998,7 +1054,7 @@ __global__ void __launch_bounds__(kT, 1) k_cluster_solve(const __grid_constant__
 #pragma unroll 1
   while (true) {
     // ---- V-cycle, z.r, beta, p
-    cluster_vcycle<D, S>(P, sm, inv, &ex, me, count);
+    cluster_vcycle<D, S>(P, sm, inv, &ex, me, count, cycles);
     {
       CompSum q;
       for_groups([&](int e, int, int, int, int, int c) {
