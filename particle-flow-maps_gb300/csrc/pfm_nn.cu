@@ -179,8 +179,8 @@ struct ConvFwdParams {
 // plane's terms arrive in the order of its 27 taps: the planes below, beside and above it in turn, each by
 // (b, c) and channel block.  Three roles overlap: TMA (a ring of planes, the weights once or as a ring of
 // taps), MMA (one lane), epilogue of finished planes.  Bound by the tensor core for 48 channels and more
-// (MMAs at 58 of 57 cycles), by the issuing warp (some 1000 cycles per plane beside its MMAs) for 16.
-// 16 -> 16 at 192^3 684 -> 169 us, 48 -> 16 at 192^3 2359 -> 374 us, 96 -> 32 at 96^3 1094 -> 162 us
+// and for 16, at four CTAs per SM, where the issuing warp (some 600 cycles per plane beside its MMAs) is next.
+// 16 -> 16 at 192^3 684 -> 117 us, 48 -> 16 at 192^3 2359 -> 296 us, 96 -> 32 at 96^3 1094 -> 157 us
 // (one tile per CTA, all 27 taps in turn, before).
 __global__ void __launch_bounds__(kFwdThreads) k_conv3_fwd(const __grid_constant__ CUtensorMap tm1,
                                                            const __grid_constant__ CUtensorMap tm2,
@@ -302,7 +302,6 @@ __global__ void __launch_bounds__(kFwdThreads) k_conv3_fwd(const __grid_constant
     // a plane's input and its new accumulator are looked for while the plane before is issued
     bool has_in = false, has_acc = false;
     for (int z = in0; z <= in1; ++z) {
-      const int lo = max(z - 1, zs), hi = min(z + 1, ze - 1);
       if (!has_acc) ok = ok && mbar_wait(pfree + at, lap & 1u, p.err, 6);
       if (!has_in) ok = ok && mbar_wait(full + s, phase, p.err, 3);
       ok = __all_sync(0xffffffffu, ok);
@@ -313,36 +312,59 @@ __global__ void __launch_bounds__(kFwdThreads) k_conv3_fwd(const __grid_constant
       has_in = mbar_test(full + s1, phase1);
       has_acc = at1 == at || mbar_test(pfree + at1, lap1 & 1u);
       const uint64_t ad0 = a_first + (uint32_t)s * (plane_pitch / 16);
+      const uint32_t d1 = tmem + (uint32_t)((p.ring - 1 - at) * p.npad);
+      const int lo = max(z - 1, zs), hi = min(z + 1, ze - 1), n = hi - lo + 1;
       const uint64_t bdz = bd0 + (uint32_t)((z + 1 - hi) * p.npad);  // rows of the planes that are not there left out
-      // the planes' columns in runs: cut at the ring's end and at N = 256
-      const int n = hi - lo + 1, r1 = min(min(n, at + 1), gmax);
-      const int at2 = r1 > at ? p.ring - 1 : at - r1, r2 = min(min(n - r1, at2 + 1), gmax);
-      const int at3 = r2 > at2 ? p.ring - 1 : at2 - r2, r3 = n - r1 - r2;
-      const uint32_t d1 = tmem + (uint32_t)((p.ring - 1 - at) * p.npad), id1 = idesc_bf16(128, r1 * p.npad);
-      const uint32_t d2 = tmem + (uint32_t)((p.ring - 1 - at2) * p.npad), id2 = idesc_bf16(128, r2 * p.npad);
-      const uint32_t d3 = tmem + (uint32_t)((p.ring - 1 - at3) * p.npad), id3 = idesc_bf16(128, r3 * p.npad);
-      const uint32_t b2 = (uint32_t)(r1 * p.npad), b3 = (uint32_t)((r1 + r2) * p.npad);
-      auto step = [&](uint64_t ad, uint64_t bd) {
-        mma_bf16(d1, ad, bd, id1, 1u);
-        if (r2) mma_bf16(d2, ad, bd + b2, id2, 1u);
-        if (r3) mma_bf16(d3, ad, bd + b3, id3, 1u);
-        if (p.mt == 2) {
-          mma_bf16(d1 + d_tile, ad + a_tile, bd, id1, 1u);
-          if (r2) mma_bf16(d2 + d_tile, ad + a_tile, bd + b2, id2, 1u);
-          if (r3) mma_bf16(d3 + d_tile, ad + a_tile, bd + b3, id3, 1u);
-        }
-      };
-      if (resident && r2 == 0) {
+      if (resident && n <= at + 1 && n <= gmax) {  // the planes' columns are one run
+        const uint32_t id = idesc_bf16(128, n * p.npad);
         if (lead) {
+          uint64_t adb = ad0, bdb = bdz;
+#pragma unroll 1
+          for (int b = 0; b < 3; ++b, adb += kBoxD2, bdb += 3 * w_step) {
 #pragma unroll
-          for (int bc = 0; bc < 9; ++bc) {
-            const uint64_t ad = ad0 + (uint32_t)((bc / 3) * kBoxD2 + bc % 3);
-            const uint64_t bd = bdz + (uint32_t)bc * w_step;
-            mma_bf16(d1, ad, bd, id1, 1u);
-            for (int j = 1; j < nj; ++j) mma_bf16(d1, ad + (uint32_t)j * a_step, bd + (uint32_t)j * b_step, id1, 1u);
+            for (int c = 0; c < 3; ++c) {
+              const uint64_t ad = adb + (uint32_t)c, bd = bdb + (uint32_t)c * w_step;
+              mma_bf16(d1, ad, bd, id, 1u);
+              for (int j = 1; j < nj; ++j) mma_bf16(d1, ad + (uint32_t)j * a_step, bd + (uint32_t)j * b_step, id, 1u);
+            }
+          }
+        }
+      } else if (resident && n <= gmax) {  // two runs, cut at the ring's end
+        const uint32_t id1 = idesc_bf16(128, (at + 1) * p.npad), id2 = idesc_bf16(128, (n - at - 1) * p.npad);
+        const uint32_t b2 = (uint32_t)((at + 1) * p.npad);
+        if (lead) {
+          uint64_t adb = ad0, bdb = bdz;
+#pragma unroll 1
+          for (int b = 0; b < 3; ++b, adb += kBoxD2, bdb += 3 * w_step) {
+#pragma unroll
+            for (int c = 0; c < 3; ++c) {
+              const uint64_t ad = adb + (uint32_t)c, bd = bdb + (uint32_t)c * w_step;
+              for (int j = 0; j < nj; ++j) {
+                mma_bf16(d1, ad + (uint32_t)j * a_step, bd + (uint32_t)j * b_step, id1, 1u);
+                mma_bf16(tmem, ad + (uint32_t)j * a_step, bd + b2 + (uint32_t)j * b_step, id2, 1u);
+              }
+            }
           }
         }
       } else {
+        // runs of columns, cut at the ring's end and at N = 256
+        const int r1 = min(min(n, at + 1), gmax);
+        const int at2 = r1 > at ? p.ring - 1 : at - r1, r2 = min(min(n - r1, at2 + 1), gmax);
+        const int at3 = r2 > at2 ? p.ring - 1 : at2 - r2, r3 = n - r1 - r2;
+        const uint32_t id1 = idesc_bf16(128, r1 * p.npad);
+        const uint32_t d2 = tmem + (uint32_t)((p.ring - 1 - at2) * p.npad), id2 = idesc_bf16(128, r2 * p.npad);
+        const uint32_t d3 = tmem + (uint32_t)((p.ring - 1 - at3) * p.npad), id3 = idesc_bf16(128, r3 * p.npad);
+        const uint32_t b2 = (uint32_t)(r1 * p.npad), b3 = (uint32_t)((r1 + r2) * p.npad);
+        auto step = [&](uint64_t ad, uint64_t bd) {
+          mma_bf16(d1, ad, bd, id1, 1u);
+          if (r2) mma_bf16(d2, ad, bd + b2, id2, 1u);
+          if (r3) mma_bf16(d3, ad, bd + b3, id3, 1u);
+          if (p.mt == 2) {
+            mma_bf16(d1 + d_tile, ad + a_tile, bd, id1, 1u);
+            if (r2) mma_bf16(d2 + d_tile, ad + a_tile, bd + b2, id2, 1u);
+            if (r3) mma_bf16(d3 + d_tile, ad + a_tile, bd + b3, id3, 1u);
+          }
+        };
         uint64_t adr = ad0;
         bool has_tap = false;
         for (int b = 0; b < 3 && ok; ++b, adr += kBoxD2) {
@@ -1173,11 +1195,11 @@ extern "C" int pfm_nn_conv3(const pfm_conv3_args* a, void* stream) {
   size_t need = 0;
   // Output planes per CTA, TMEM columns and tiles per CTA by the time they should take, in cycles.  An SM's
   // tensor core works through the seg + 2 input planes of each of its CTAs (34 + N/2 per MMA; two MMAs where
-  // the planes' columns straddle the ring's end or exceed N = 256), a CTA's issuing warp needs some 1000 +
+  // the planes' columns straddle the ring's end or exceed N = 256), a CTA's issuing warp needs some 600 +
   // 60 per MMA, and a CTA's start-up and drain of 9000 are hidden where others share its SM.  Weights that
   // do not fit beside two planes come from L2 once per plane, at some 19 bytes per cycle and SM; two tiles
-  // share them then.  16 -> 16 at 192^3: 331 us with 16 planes in TMEM and 192 per CTA, 207 with rings of 4,
-  // 169 with the 8 this picks; 96 -> 32 at 96^3: 250 us with one tile per CTA, 162 with two.
+  // share them then.  16 -> 16 at 192^3: 147 us with rings of 16 planes (two CTAs per SM), 117
+  // with the 8 this picks; 96 -> 32 at 96^3: 250 us with one tile per CTA, 157 with two.
   double best = -1.;
   for (int mt = 1; mt <= 2; ++mt) {
     const size_t plane = ((size_t)(cin / 8) * (mt * kTileD1 + 2) * kRowBytes + 127) & ~(size_t)127;
@@ -1202,7 +1224,7 @@ extern "C" int pfm_nn_conv3(const pfm_conv3_args* a, void* stream) {
         if (seg > fit && fit < 4) continue;
         const double mmas = 9. * (cin / 16) * mt * (3 * npad > 256 ? 2. : 1.) * (seg > fit ? 1. + 2. / fit : 1.);
         const double tensor = 34. * mmas + 9. * (cin / 16) * mt * 1.5 * npad;
-        double issue = 1000. + 60. * mmas;
+        double issue = 600. + 60. * mmas;
         if (wstage != 9) issue = std::max(issue + 9. * 200., 9. * wtap / 19.);
         const double alone = (seg + 2) * std::max(issue, tensor) + 9000.;
         const double work = (seg + 2) * std::max(issue / slots, tensor);
