@@ -220,6 +220,14 @@ int pfm_create(const pfm_config* cfg, pfm_handle** out) {
   h->o_hist = take(4 * C * 4);  // per pressure buffer: its last two solutions
   h->o_hist_flag = take(2 * sizeof(int));
   h->hist_ptr[0] = h->hist_ptr[1] = nullptr;
+  h->pad_pitch = pad_pitch_of(h->geom);
+  h->pad_done = nullptr;
+  if (h->pad_pitch && cudaEventCreateWithFlags(&h->pad_done, cudaEventDisableTiming) != cudaSuccess) {
+    cudaGetLastError();
+    h->pad_pitch = 0;
+  }
+  h->pad_sets = h->pad_pitch ? (P > 0 ? 2 : 1) : 0;  // the RK4 with the gradient's reinitialisation reads two fields
+  h->o_pad = h->pad_sets ? take(h->pad_sets * pad_set_bytes(h->geom, h->pad_pitch)) : 0;
 
   h->ws_need = off;
   h->p2g2_column = 8;
@@ -230,6 +238,7 @@ int pfm_create(const pfm_config* cfg, pfm_handle** out) {
   h->mg_cluster = 1;
   if (cudaHostAlloc((void**)&h->h_state, sizeof(SolveState), cudaHostAllocDefault) != cudaSuccess) {
     cudaGetLastError();
+    if (h->pad_done) cudaEventDestroy(h->pad_done);
     delete h;
     return PFM_ERR_CUDA;
   }
@@ -245,6 +254,7 @@ int pfm_destroy(pfm_handle* h) {
   if (h->g_step) cudaGraphExecDestroy(h->g_step);
   if (h->cap_stream) cudaStreamDestroy(h->cap_stream);
   if (h->h_state) cudaFreeHost(h->h_state);
+  if (h->pad_done) cudaEventDestroy(h->pad_done);
   delete h;
   return PFM_OK;
 }

@@ -149,7 +149,8 @@ __device__ __forceinline__ bool interp_face_centre(const MacFields3& F, const Ma
     int first[3];
 #pragma unroll
     for (int a = 0; a < 3; ++a) first[a] = (a == fam || a != c) ? I[a] - 1 : I[a];
-    const int m1 = NC ? (c == 1 ? NC + 1 : NC) : g.n[c][1], m2 = NC ? (c == 2 ? NC + 1 : NC) : g.n[c][2];
+    const int m1 = NC > 0 ? (c == 1 ? NC + 1 : NC) : NC ? -NC : g.n[c][1];
+    const int m2 = NC > 0 ? (c == 2 ? NC + 1 : NC) : NC ? -NC : g.n[c][2];
     const float* __restrict__ base = F.u[c] + ((first[0] * m1 + first[1]) * m2 + first[2]);
     const int sx = m1 * m2;
     float v, gx, gy, gz;
@@ -303,18 +304,47 @@ __global__ void __launch_bounds__(kGThreads) k_midpoint2(MacFields2 F, MacGeom g
   u1[e] = Tf[0] * ua[0] + Tf[1] * ua[1];
 }
 
-// k_midpoint3 of face family fam, instantiated for the grid's cube extent when there is one.
-static void launch_midpoint3(pfm_handle* h, int fam, dim3 gr, cudaStream_t st, const MacFields3& F, float dt_half,
-                             float* u1, float* psi_out, float* T_out, const float* dt_half_dev) {
-  with_cube(h, [&](auto nc) {
+// The three components of F into the padded set (z = component): one row per warp.
+__global__ void __launch_bounds__(256) k_pad_fields(MacFields3 F, MacGeom g, float* __restrict__ out, int pitch) {
+  const int c = blockIdx.z, n1 = g.n[c][1], n2 = g.n[c][2], lane = threadIdx.x & 31;
+  const int j = blockIdx.x * 8 + (threadIdx.x >> 5), i = blockIdx.y;
+  if (i >= g.n[c][0] || j >= n1) return;
+  const float* src = F.u[c] + ((int64_t)i * n1 + j) * n2;
+  float* dst = out + ((((int64_t)c * (g.N[0] + 1) + i) * pitch) + j) * pitch;
+  for (int k = lane; k < n2; k += 128) {
+    float v[4];
+#pragma unroll
+    for (int q = 0; q < 4; ++q)
+      if (k + 32 * q < n2) v[q] = __ldg(src + k + 32 * q);
+#pragma unroll
+    for (int q = 0; q < 4; ++q)
+      if (k + 32 * q < n2) dst[k + 32 * q] = v[q];
+  }
+}
+
+MacFields3 pad_fields(pfm_handle* h, const MacFields3& F, int set, cudaStream_t st) {
+  const MacGeom& g = h->geom;
+  const int p = h->pad_pitch;
+  float* out = ws_ptr<float>(h, h->o_pad) + set * (pad_set_bytes(g, p) / sizeof(float));
+  launch(h, k_pad_fields, dim3((unsigned)(g.N[1] / 8 + 1), (unsigned)(g.N[0] + 1), 3), 256, 0, st, F, g, out, p);
+  const size_t comp = (size_t)(g.N[0] + 1) * p * p;
+  return MacFields3{{out, out + comp, out + 2 * comp}};
+}
+
+// k_midpoint3 of the face families, instantiated for the grid's cube extent or padded pitch when there is one.
+static void launch_midpoint3(pfm_handle* h, cudaStream_t st, const MacFields3& F, float dt_half, float* const* u1,
+                             float* const* psi_out, float* const* T_out, const float* dt_half_dev) {
+  const MacFields3 fields[1] = {F};
+  with_strides<1>(h, fields, true, st, [&](auto nc, const MacFields3 (&G)[1]) {
     constexpr int NC = decltype(nc)::value;
     const int c = h->mid_centre;
-    if (fam == 0)
-      launch(h, k_midpoint3<0, NC>, gr, kGThreads, 0, st, F, h->geom, dt_half, u1, psi_out, T_out, dt_half_dev, c);
-    if (fam == 1)
-      launch(h, k_midpoint3<1, NC>, gr, kGThreads, 0, st, F, h->geom, dt_half, u1, psi_out, T_out, dt_half_dev, c);
-    if (fam == 2)
-      launch(h, k_midpoint3<2, NC>, gr, kGThreads, 0, st, F, h->geom, dt_half, u1, psi_out, T_out, dt_half_dev, c);
+    for (int fam = 0; fam < 3; ++fam) {
+      const int64_t nf = (int64_t)h->geom.n[fam][0] * h->geom.n[fam][1] * h->geom.n[fam][2];
+      const dim3 gr(grid_for(nf, kGThreads));
+      auto kernel = fam == 0 ? k_midpoint3<0, NC> : fam == 1 ? k_midpoint3<1, NC> : k_midpoint3<2, NC>;
+      launch(h, kernel, gr, kGThreads, 0, st, G[0], h->geom, dt_half, u1[fam], psi_out ? psi_out[fam] : nullptr,
+             T_out ? T_out[fam] : nullptr, dt_half_dev, c);
+    }
   });
 }
 
@@ -322,20 +352,15 @@ static void launch_midpoint3(pfm_handle* h, int fam, dim3 gr, cudaStream_t st, c
 // from device memory.
 int launch_midpoint(pfm_handle* h, const float* const* u0, float* const* u1, float dt_half, const float* dt_half_dev,
                     cudaStream_t st) {
-  const int D = h->cfg.dim;
-  for (int fam = 0; fam < D; ++fam) {
-    const int64_t nf = (int64_t)h->geom.n[fam][0] * h->geom.n[fam][1] * h->geom.n[fam][2];
-    const dim3 gr(grid_for(nf, kGThreads));
-    if (D == 3) {
-      const MacFields3 F{{u0[0], u0[1], u0[2]}};
-      launch_midpoint3(h, fam, gr, st, F, dt_half, u1[fam], nullptr, nullptr, dt_half_dev);
-    } else {
-      const MacFields2 F{{u0[0], u0[1]}};
-      if (fam == 0) launch(h, k_midpoint2<0>, gr, kGThreads, 0, st, F, h->geom, dt_half, u1[0], (float*)nullptr,
-                           (float*)nullptr, dt_half_dev);
-      if (fam == 1) launch(h, k_midpoint2<1>, gr, kGThreads, 0, st, F, h->geom, dt_half, u1[1], (float*)nullptr,
-                           (float*)nullptr, dt_half_dev);
-    }
+  if (h->cfg.dim == 3) {
+    launch_midpoint3(h, st, MacFields3{{u0[0], u0[1], u0[2]}}, dt_half, u1, nullptr, nullptr, dt_half_dev);
+    return launch_check(h, "midpoint");
+  }
+  const MacFields2 F{{u0[0], u0[1]}};
+  for (int fam = 0; fam < 2; ++fam) {
+    const dim3 gr(grid_for((int64_t)h->geom.n[fam][0] * h->geom.n[fam][1], kGThreads));
+    launch(h, fam == 0 ? k_midpoint2<0> : k_midpoint2<1>, gr, kGThreads, 0, st, F, h->geom, dt_half, u1[fam],
+           (float*)nullptr, (float*)nullptr, dt_half_dev);
   }
   return launch_check(h, "midpoint");
 }
@@ -386,18 +411,9 @@ int pfm3_midpoint(pfm_handle* h, const float* u0_x, const float* u0_y, const flo
     return set_error(h, PFM_ERR_NULL, "pfm3_midpoint: null input");
   if (u0_x == u1_x || u0_y == u1_y || u0_z == u1_z)
     return set_error(h, PFM_ERR_ARG, "pfm3_midpoint: u0 and u1 must not alias");
-  MacFields3 F{{u0_x, u0_y, u0_z}};
   float* outs[3] = {u1_x, u1_y, u1_z};
-  for (int fam = 0; fam < 3; ++fam) {
-    int64_t nf = (int64_t)h->geom.n[fam][0] * h->geom.n[fam][1] * h->geom.n[fam][2];
-    float* po = psi_out ? psi_out[fam] : nullptr;
-    float* to = T_out ? T_out[fam] : nullptr;
-    dim3 gr(grid_for(nf, kGThreads));
-    launch_midpoint3(h, fam, gr, (cudaStream_t)stream, F, dt_half, outs[fam], po, to, nullptr);
-    int s = launch_check(h, "k_midpoint3");
-    if (s) return s;
-  }
-  return PFM_OK;
+  launch_midpoint3(h, (cudaStream_t)stream, MacFields3{{u0_x, u0_y, u0_z}}, dt_half, outs, psi_out, T_out, nullptr);
+  return launch_check(h, "k_midpoint3");
 }
 
 int pfm2_midpoint(pfm_handle* h, const float* u0_x, const float* u0_y, float* u1_x, float* u1_y, float dt_half,

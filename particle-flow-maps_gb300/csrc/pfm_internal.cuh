@@ -127,6 +127,11 @@ struct pfm_handle {
   // the slots) and a device flag per slot saying whether it holds one
   size_t o_hist, o_hist_flag;
   size_t o_x64;
+  // 3D grids without an instance of their extent: copies of velocity fields with rows and planes of pad_pitch
+  // (pad_sets of three components from o_pad), or 0
+  size_t o_pad;
+  int pad_pitch, pad_sets;
+  cudaEvent_t pad_done;  // after the last reader of the copies (they are shared by the callers' streams)
   const float* hist_ptr[2];
 
   // pinned host mirror of the solve state
@@ -317,7 +322,10 @@ __device__ __forceinline__ void mac_taps3(const MacGeom& g, const float p[3], Ax
 // The tap sums of interp_mac3 for taps already computed (two fields of the same shape sampled at
 // one position share them).  NC > 0: the grid is NC^3 cells, so the face fields' strides are
 // compile-time constants and every row of a field is its base pointer plus a load immediate (the
-// same loads and sums as NC = 0, which reads the strides from g).
+// same loads and sums as NC = 0, which reads the strides from g).  NC < 0: the fields are copies with
+// rows of -NC elements and planes of -NC rows (k_pad_fields), so that any grid has such strides.
+constexpr int abs_of(int n) { return n < 0 ? -n : n; }
+
 template <int NC = 0>
 __device__ __forceinline__ void interp_mac3_taps(const MacFields3& F, const MacGeom& g, const Axis3 A0[3],
                                                  const Axis3 A1[3], float uo[3], float G[3][3], bool want_grad);
@@ -338,8 +346,8 @@ __device__ __forceinline__ void interp_mac3_taps(const MacFields3& F, const MacG
   {
     const float* __restrict__ f0 = F.u[0];
     const float* __restrict__ f1 = F.u[1];
-    const int m01 = NC ? NC : g.n[0][1], m02 = NC ? NC : g.n[0][2];
-    const int m11 = NC ? NC + 1 : g.n[1][1], m12 = NC ? NC : g.n[1][2];
+    const int m01 = NC ? abs_of(NC) : g.n[0][1], m02 = NC ? abs_of(NC) : g.n[0][2];
+    const int m11 = NC > 0 ? NC + 1 : NC ? -NC : g.n[1][1], m12 = NC ? abs_of(NC) : g.n[1][2];
     const Axis3& Z = A1[2];
     const float* __restrict__ b0 = f0 + ((A0[0].first * m01 + A1[1].first) * m02 + Z.first);
     const float* __restrict__ b1 = f1 + ((A1[0].first * m11 + A0[1].first) * m12 + Z.first);
@@ -392,7 +400,7 @@ __device__ __forceinline__ void interp_mac3_taps(const MacFields3& F, const MacG
   // ---- component z: (A1x, A1y, A0z)
   {
     const float* __restrict__ f = F.u[2];
-    const int m1 = NC ? NC : g.n[2][1], m2 = NC ? NC + 1 : g.n[2][2];
+    const int m1 = NC ? abs_of(NC) : g.n[2][1], m2 = NC > 0 ? NC + 1 : NC ? -NC : g.n[2][2];
     const Axis3 &X = A1[0], &Y = A1[1], &Z = A0[2];
     const float* __restrict__ base = f + ((X.first * m1 + Y.first) * m2 + Z.first);
     const int sx = m1 * m2;
@@ -447,6 +455,50 @@ inline void with_cube(const pfm_handle* h, Fn&& f) {
     case 512: f(std::integral_constant<int, 512>()); break;
     default: f(std::integral_constant<int, 0>()); break;
   }
+}
+
+// The pitch of the padded copies of a grid's fields: the smallest of 128, 256 and 512 that holds its rows and
+// planes, where that is at most four times the fields; 0 (no copies) for cubes with an instance of their own and
+// for grids below 64^3 cells, where a copy takes as long as it saves (3 us of a midpoint's 77).
+inline int pad_pitch_of(const MacGeom& g) {
+  if (g.dim != 3 || cube_extent(g) || (int64_t)g.N[0] * g.N[1] * g.N[2] < 262144) return 0;
+  const int n = (g.N[1] > g.N[2] ? g.N[1] : g.N[2]) + 1;
+  const int p = n <= 128 ? 128 : n <= 256 ? 256 : n <= 512 ? 512 : 0;
+  return p && (int64_t)p * p <= 4ll * (g.N[1] + 1) * (g.N[2] + 1) ? p : 0;
+}
+inline size_t pad_set_bytes(const MacGeom& g, int pitch) {
+  return 3 * (size_t)(g.N[0] + 1) * pitch * pitch * sizeof(float);
+}
+// Copies the components of F into set `set` of the padded copies; returns them.
+MacFields3 pad_fields(pfm_handle* h, const MacFields3& F, int set, cudaStream_t st);
+
+// with_cube for kernels that read N velocity fields: f(integral_constant<NC>(), fields), the fields replaced by
+// their padded copies where the grid has these and the caller asks for them.  With the strides as load immediates
+// a row costs no 64-bit add: the midpoint of 192^3 took 1931 us with run-time strides, 1780 with padded ones and
+// 28 for the copies; the RK4 of 7.1M particles at 96^3 586, 526 and 8.  Calls on different streams wait for each
+// other's copies; in a caller's capture there are none, since they would tie its graph to work outside it.
+template <int N, class Fn>
+inline void with_strides(pfm_handle* h, const MacFields3 (&F)[N], bool ask, cudaStream_t st, Fn&& f) {
+  if (ask && h->ws && h->cube_kernels && h->pad_pitch && N <= h->pad_sets) {
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(st, &cap) != cudaSuccess) {
+      cudaGetLastError();
+      cap = cudaStreamCaptureStatusActive;
+    }
+    const bool own = cap != cudaStreamCaptureStatusNone && st && st == h->cap_stream;  // the whole-step graph
+    if (own || (cap == cudaStreamCaptureStatusNone && cudaStreamWaitEvent(st, h->pad_done, 0) == cudaSuccess)) {
+      MacFields3 G[N];
+      for (int i = 0; i < N; ++i) G[i] = pad_fields(h, F[i], i, st);
+      switch (h->pad_pitch) {
+        case 128: f(std::integral_constant<int, -128>(), G); break;
+        case 256: f(std::integral_constant<int, -256>(), G); break;
+        default: f(std::integral_constant<int, -512>(), G); break;
+      }
+      if (!own) cudaEventRecord(h->pad_done, st);
+      return;
+    }
+  }
+  with_cube(h, [&](auto nc) { f(nc, F); });
 }
 
 // Loads and stores of particle state that a thread touches once (the RK4's inputs and outputs):

@@ -343,18 +343,21 @@ int launch_rk4_T_forward3(pfm_handle* h, float* pos, float* T, const MacFields3&
                           const MacFields3* Fg, cudaStream_t st, const float* dt_dev) {
   if (h->P == 0) return PFM_OK;
   const unsigned nb = grid_for(h->P, kRK4Threads);
-  with_cube(h, [&](auto nc) {
-    constexpr int NC = decltype(nc)::value;
-    if (R && Fg)
-      launch(h, k_rk4_T_forward3<true, true, NC>, nb, kRK4Threads, 0, st, pos, T, h->P, F, h->geom, dt, *R, *Fg,
-             dt_dev);
-    else if (R)
-      launch(h, k_rk4_T_forward3<true, false, NC>, nb, kRK4Threads, 0, st, pos, T, h->P, F, h->geom, dt, *R,
-             MacFields3{}, dt_dev);
-    else
-      launch(h, k_rk4_T_forward3<false, false, NC>, nb, kRK4Threads, 0, st, pos, T, h->P, F, h->geom, dt,
-             P2GRecords3{}, MacFields3{}, dt_dev);
-  });
+  const bool pad = h->P >= 2 * h->cells;  // fewer particles do not pay for the copies
+  if (R && Fg) {
+    const MacFields3 two[2] = {F, *Fg};
+    with_strides<2>(h, two, pad, st, [&](auto nc, const MacFields3 (&G)[2]) {
+      launch(h, k_rk4_T_forward3<true, true, decltype(nc)::value>, nb, kRK4Threads, 0, st, pos, T, h->P, G[0], h->geom, dt,
+             *R, G[1], dt_dev);
+    });
+  } else {
+    const MacFields3 one[1] = {F};
+    with_strides<1>(h, one, pad, st, [&](auto nc, const MacFields3 (&G)[1]) {
+      constexpr int NC = decltype(nc)::value;
+      launch(h, R ? k_rk4_T_forward3<true, false, NC> : k_rk4_T_forward3<false, false, NC>, nb, kRK4Threads, 0, st, pos, T,
+             h->P, G[0], h->geom, dt, R ? *R : P2GRecords3{}, MacFields3{}, dt_dev);
+    });
+  }
   return launch_check(h, "k_rk4_T_forward3");
 }
 
