@@ -596,6 +596,8 @@ typedef struct pfm_conv3_wgrad_args {
 int pfm_nn_conv3(const pfm_conv3_args* a, void* stream);
 /* Weight gradient dW = sum over voxels of x(v + tap) dy(v); deterministic. */
 int pfm_nn_conv3_wgrad(const pfm_conv3_wgrad_args* a, void* stream);
+/* The same with the bias gradient db[cout] beside it (pfm_nn_bias_grad in one pass over dy); scratch as there. */
+int pfm_nn_conv3_wgrad_bias(const pfm_conv3_wgrad_args* a, float* db, float* scratch, void* stream);
 int pfm_nn_wgrad_workspace(const pfm_conv3_wgrad_args* a, size_t* bytes);
 /* Packs W [cout][cin][27] into [27][kin/8][npad][8] BF16 for the forward (flip 0: rows = cout,
  * K = cin) or the data gradient (flip 1: rows = cin, K = cout, taps mirrored). */

@@ -486,6 +486,16 @@ __global__ void __launch_bounds__(kFwdThreads) k_conv3_fwd(const __grid_constant
 // ---------------------------------------------------------------------------------------------
 // weight gradient
 
+__device__ __forceinline__ void unpack8(uint4 u, float (&f)[8]) {
+  const __nv_bfloat162* h = reinterpret_cast<const __nv_bfloat162*>(&u);
+#pragma unroll
+  for (int q = 0; q < 4; ++q) {
+    float2 t = __bfloat1622float2(h[q]);
+    f[2 * q] = t.x;
+    f[2 * q + 1] = t.y;
+  }
+}
+
 constexpr int kWgThreads = 192;  // warp 0: TMA, warp 1: MMA, warps 2-5: epilogue
 constexpr int kWgStages = 4;
 constexpr int kXChunk = kTileD1 * kRowBytes;  // one 8-channel block of an X plane (16 rows of 10 voxels): 2,560 B
@@ -503,6 +513,7 @@ struct ConvWgradParams {
   int nstage, ncols;
   uint32_t stage_bytes, dy_pitch;
   float* partial;  // [split][blockIdx.y][c = 3][N][rows]
+  float* bias;     // [split][16][8]: sums of dY over groups of eight voxels, by the CTAs of blockIdx.y = 0 (or null)
   int* err;
 };
 
@@ -514,6 +525,8 @@ struct ConvWgradParams {
 // is a start address in X: a step of P planes of 128 voxels takes 3 c x 8 MMAs for all 27 taps.  X rows
 // belong to one tile and dY's are loaded with a halo row on each side; X planes and columns the other way round.
 // A CTA adds up a run of steps for one group of input channels; the splits are summed with compensation.
+// The epilogue warps, idle until then, add up dY's channels for the bias gradient from the stages they find it in
+// (its own pass and sum took 80 us of a 96^3 gradient).
 // Bound by the tensor core's reading of A, some 34 + N/2 cycles per MMA.  With its reduction, 16 -> 16 at 96^3
 // 423 -> 35 us, 48 -> 16 at 96^3 1054 -> 71, 96 -> 32 at 48^3 474 -> 57 (operands transposed into shared memory by
 // eight warps before, 592 splits added up by one thread per weight).
@@ -533,13 +546,14 @@ __global__ void __launch_bounds__(kWgThreads) k_conv3_wgrad(const __grid_constan
 
   const int mtile = blockIdx.y % p.mtiles, cb = (int)(blockIdx.y / p.mtiles) * p.nb;
   const int nblk = min(p.nb, p.kc - cb);
+  const bool bias = p.bias && blockIdx.y == 0;
   const int s0 = (int)((long long)blockIdx.x * p.steps / gridDim.x);
   const int s1 = (int)((long long)(blockIdx.x + 1) * p.steps / gridDim.x);
 
   if (warp == 0) {
     if (lane < kWgStages) {
       mbar_init(full + lane, 1);
-      mbar_init(empty + lane, 1);
+      mbar_init(empty + lane, bias ? 5 : 1);
     } else if (lane == 31) {
       mbar_init(fin, 1);
       mbar_init(moved, 128);
@@ -656,16 +670,57 @@ __global__ void __launch_bounds__(kWgThreads) k_conv3_wgrad(const __grid_constan
     bool ok = true;
     if (moves)
       for (int c0 = 0; c0 < 3 * p.N; c0 += 16) tmem_zero16(lanes + sums + (uint32_t)c0);
-    for (int f = 0; f < moves && ok; ++f) {
+    int f = 0;
+    auto move = [&]() {
       ok = mbar_wait(fin, (unsigned)f & 1u, p.err, 13);
       ok = __all_sync(0xffffffffu, ok);
-      if (!ok) break;
+      if (!ok) return;
       tmem_st_wait();
       tc_fence_after();
       for (int c0 = 0; c0 < 3 * p.N; c0 += 16) tmem_add16(lanes + (uint32_t)c0, lanes + sums + (uint32_t)c0);
       tmem_st_wait();
       tc_fence_before();
       mbar_arrive(moved);
+      ++f;
+    };
+    if (bias) {
+      // thread t takes every 128th 16-byte row (8 channels of a voxel) of a stage's 16 inner rows of dY, always
+      // of channel block (t / 8) % dc (dc divides 16)
+      const int t = (int)threadIdx.x - 64, group = p.P * p.dc * 8, n = 16 * group;
+      float acc[8] = {0, 0, 0, 0, 0, 0, 0, 0};
+      int s = 0, run = 0;
+      unsigned phase = 0;
+      for (int i = 0; i < s1 - s0 && ok; ++i) {
+        ok = __all_sync(0xffffffffu, mbar_wait(full + s, phase, p.err, 15));
+        if (!ok) break;
+        for (int g = 0; g < p.G; ++g) {
+          const uint4* rows = (const uint4*)(smem + (size_t)s * p.stage_bytes + (size_t)g * p.dy_pitch) + group;
+          for (int e = t; e < n; e += 128) {
+            float v[8];
+            unpack8(rows[e], v);
+#pragma unroll
+            for (int q = 0; q < 8; ++q) acc[q] += v[q];
+          }
+        }
+        __syncwarp();
+        if (lane == 0) mbar_arrive(empty + s);
+        if (p.flush && ++run == p.flush && i + 1 < s1 - s0) {
+          run = 0;
+          move();
+        }
+        if (++s == p.nstage) {
+          s = 0;
+          phase ^= 1u;
+        }
+      }
+#pragma unroll
+      for (int q = 0; q < 8; ++q)
+        for (int o = 1; o < 8; o *= 2) acc[q] += __shfl_xor_sync(0xffffffffu, acc[q], o);
+      if ((lane & 7) == 0)
+#pragma unroll
+        for (int q = 0; q < 8; ++q) p.bias[((size_t)blockIdx.x * 16 + (t >> 3)) * 8 + q] = acc[q];
+    } else {
+      while (f < moves && ok) move();
     }
     ok = ok && mbar_wait(fin, (unsigned)moves & 1u, p.err, 13);
     if (__all_sync(0xffffffffu, ok)) {
@@ -698,8 +753,23 @@ __global__ void __launch_bounds__(kWgThreads) k_conv3_wgrad(const __grid_constan
 constexpr int kWrWarps = 8;
 
 __global__ void __launch_bounds__(32 * kWrWarps) k_wgrad_reduce(const ConvWgradParams p, int splits, int gy, int cout,
-                                                                float* __restrict__ dw) {
+                                                                float* __restrict__ dw, float* __restrict__ db) {
   __shared__ float sh[kWrWarps][8][8];
+  if (blockIdx.z == 9) {  // the bias gradient: a warp per channel
+    const int c = (blockIdx.x + gridDim.x * blockIdx.y) * (blockDim.x >> 5) + (threadIdx.x >> 5), l = threadIdx.x & 31;
+    if (c >= cout) return;
+    CompSum v;
+    const int per = 16 / p.dc;  // groups of a split that hold the channel
+    for (int k = l; k < splits * per; k += 32)
+      v.add(p.bias[((size_t)(k / per) * 16 + (c >> 3) + (k % per) * p.dc) * 8 + (c & 7)]);
+    for (int o = 16; o > 0; o >>= 1) {
+      const float hi = __shfl_xor_sync(0xffffffffu, v.s, o), lo = __shfl_xor_sync(0xffffffffu, v.c, o);
+      v.add(hi);
+      v.c += lo;
+    }
+    if (l == 0) db[c] = v.s + v.c;
+    return;
+  }
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, warps = blockDim.x >> 5;
   const int cdy = p.dc * 8, i = blockIdx.x * 32 + (lane & 7) * 4;
   const bool in = i < 3 * cdy;
@@ -779,16 +849,6 @@ __global__ void k_pack_scalar(const float* __restrict__ f, size_t V, const float
   uint4 a = make_uint4(*(uint32_t*)&h0, 0, 0, 0), z = make_uint4(0, 0, 0, 0);
   ((uint4*)x)[v] = a;
   ((uint4*)x)[V + v] = z;
-}
-
-__device__ __forceinline__ void unpack8(uint4 u, float (&f)[8]) {
-  const __nv_bfloat162* h = reinterpret_cast<const __nv_bfloat162*>(&u);
-#pragma unroll
-  for (int q = 0; q < 4; ++q) {
-    float2 t = __bfloat1622float2(h[q]);
-    f[2 * q] = t.x;
-    f[2 * q + 1] = t.y;
-  }
 }
 
 __device__ __forceinline__ uint4 pack8(const float (&f)[8]) {
@@ -1270,11 +1330,11 @@ extern "C" int pfm_nn_wgrad_workspace(const pfm_conv3_wgrad_args* a, size_t* byt
   WgradPlan w;
   *bytes = 0;  // of a shape that pfm_nn_conv3_wgrad refuses
   if (grid_ok(a->d0, a->d1, a->d2) && wgrad_shape_ok(a) && wgrad_plan(a, &w))
-    *bytes = (size_t)w.gx * w.gy * 3 * w.p.N * w.p.rows * sizeof(float);
+    *bytes = ((size_t)w.gx * w.gy * 3 * w.p.N * w.p.rows + (size_t)w.gx * 128) * sizeof(float);
   return PFM_OK;
 }
 
-extern "C" int pfm_nn_conv3_wgrad(const pfm_conv3_wgrad_args* a, void* stream) {
+static int conv3_wgrad(const pfm_conv3_wgrad_args* a, float* db, cudaStream_t st) {
   if (!a || !a->x1 || !a->dy || !a->dw || !a->partial || !a->err) return PFM_ERR_NULL;
   if (!grid_ok(a->d0, a->d1, a->d2)) return PFM_ERR_SHAPE;
   if (!wgrad_shape_ok(a) || (a->c2 > 0 && !a->x2)) return PFM_ERR_SHAPE;
@@ -1295,16 +1355,27 @@ extern "C" int pfm_nn_conv3_wgrad(const pfm_conv3_wgrad_args* a, void* stream) {
   }
   if (!make_wgrad_map(&tmdy, a->dy, a->cdy, a->d0, a->d1, a->d2, w.p.P)) return PFM_ERR_CUDA;
   w.p.partial = a->partial;
+  w.p.bias = db ? a->partial + (size_t)w.gx * w.gy * 3 * w.p.N * w.p.rows : nullptr;
   w.p.err = a->err;
   static std::atomic<unsigned long long> attr{0};  // above the default 48 KB: opt in per device
   if (pfm::opt_in_smem(k_conv3_wgrad, kMaxDynSmem, attr) != cudaSuccess) return PFM_ERR_CUDA;
-  cudaStream_t st = (cudaStream_t)stream;
   k_conv3_wgrad<<<dim3((unsigned)w.gx, (unsigned)w.gy), kWgThreads, w.smem, st>>>(tm1, tm2, tmdy, w.p);
   int warps = 1;  // some eight loads per thread
   while (warps < kWrWarps && warps * 32 < w.gx * w.p.P) warps *= 2;
-  const dim3 rgrid((unsigned)(3 * a->cdy + 31) / 32, (unsigned)(a->c1 + a->c2), 9);
-  k_wgrad_reduce<<<rgrid, 32 * warps, 0, st>>>(w.p, w.gx, w.gy, a->cout, a->dw);
+  const dim3 rgrid((unsigned)(3 * a->cdy + 31) / 32, (unsigned)(a->c1 + a->c2), db ? 10 : 9);
+  k_wgrad_reduce<<<rgrid, 32 * warps, 0, st>>>(w.p, w.gx, w.gy, a->cout, a->dw, db);
   return cudaGetLastError() == cudaSuccess ? PFM_OK : PFM_ERR_CUDA;
+}
+
+extern "C" int pfm_nn_conv3_wgrad(const pfm_conv3_wgrad_args* a, void* stream) {
+  return conv3_wgrad(a, nullptr, (cudaStream_t)stream);
+}
+
+extern "C" int pfm_nn_conv3_wgrad_bias(const pfm_conv3_wgrad_args* a, float* db, float* scratch, void* stream) {
+  if (!a || !db || !scratch) return PFM_ERR_NULL;
+  if (a->cdy > 0 && 128 % a->cdy == 0) return conv3_wgrad(a, db, (cudaStream_t)stream);
+  const int rc = conv3_wgrad(a, nullptr, (cudaStream_t)stream);  // the epilogue's threads would mix channel blocks
+  return rc ? rc : pfm_nn_bias_grad(a->dy, a->cdy, a->d0, a->d1, a->d2, a->cout, db, scratch, stream);
 }
 
 extern "C" int pfm_nn_pack_weights(const float* W, int cout, int cin, int flip, int kin, int npad, void* wp,

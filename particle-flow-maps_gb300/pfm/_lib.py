@@ -167,6 +167,7 @@ SIGNATURES = {
     "pfm3_add_buoyancy_impulse": [_P, _P, _P, _P, _P, _P, _F, _I, _P],
     "pfm_nn_conv3": [ctypes.POINTER(Conv3Args), _P],
     "pfm_nn_conv3_wgrad": [ctypes.POINTER(Conv3WgradArgs), _P],
+    "pfm_nn_conv3_wgrad_bias": [ctypes.POINTER(Conv3WgradArgs), _P, _P, _P],
     "pfm_nn_wgrad_workspace": [ctypes.POINTER(Conv3WgradArgs), ctypes.POINTER(ctypes.c_size_t)],
     "pfm_nn_pack_weights": [_P, _I, _I, _I, _I, _I, _P, _P],
     "pfm_nn_pack_scalar": [_P, _I, _I, _I, _P, _P, _P],

@@ -198,9 +198,7 @@ class UNet3D:
         a = _lib.Conv3WgradArgs(g[0], g[1], g[2], _p(x1), l.c1, _p(x2), l.c2, _p(dy), l.kin_t, l.cout, _p(l.gw),
                                 _p(B["partial"]), B["partial"].numel() * 4, _p(self.err))
         st = self._stream() if st is None else st
-        self._check(self.lib.pfm_nn_conv3_wgrad(ctypes.byref(a), st), "wgrad", l.name)
-        self._check(self.lib.pfm_nn_bias_grad(_p(dy), l.kin_t, g[0], g[1], g[2], l.cout, _p(l.gb), _p(self.scratch), st),
-                    "bias grad", l.name)
+        self._check(self.lib.pfm_nn_conv3_wgrad_bias(ctypes.byref(a), _p(l.gb), _p(self.scratch), st), "wgrad", l.name)
 
     def _resample(self, x, y, c, fine, mode, st=None):
         st = self._stream() if st is None else st

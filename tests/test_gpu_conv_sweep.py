@@ -94,6 +94,15 @@ def test_weight_gradient_groups(c1, c2, cout, cdy, dims):
     torch.cuda.synchronize()
     assert int(err.item()) == 0
     ref, bound = O.conv3_wgrad(x, dy[:cout]), O.conv3_wgrad(np.abs(x), np.abs(dy[:cout]))
+    db, scratch = torch.full((cout,), float("nan"), device="cuda"), torch.empty(296 * max(cdy, 2), device="cuda")
+    dw2 = torch.full_like(dw, float("nan"))
+    a.dw = ptr(dw2)
+    assert lib.pfm_nn_conv3_wgrad_bias(ctypes.byref(a), ptr(db), ptr(scratch), None) == 0
+    torch.cuda.synchronize()
+    assert int(err.item()) == 0 and torch.equal(dw, dw2)
+    flat = dy[:cout].reshape(cout, -1).astype(np.float64)
+    # partial sums of a few hundred f32 additions each, compensated from there
+    assert np.all(np.abs(db.cpu().numpy() - flat.sum(1)) <= 2e-5 * np.abs(flat).sum(1))
     # a sum of at most V / 16 / 45 + 48 truncated steps of 2^-23 each stays below 1e-4 of the absolute sum
     got = dw.cpu().numpy()
     assert np.all(np.abs(got - ref) <= 1e-4 * bound + 1e-6), np.nanmax(np.abs(got - ref) / (bound + 1e-6))
