@@ -564,6 +564,20 @@ using namespace pfm;
 
 extern "C" {
 
+// Launches the step graph, ordered against the other streams' calls that use the padded velocity copies
+// (not in a caller's capture, whose graph cannot wait for work outside it).
+static int launch_step_graph(pfm_handle* h, cudaStream_t s) {
+  bool ordered = h->pad_done != nullptr;
+  cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+  if (ordered && cudaStreamIsCapturing(s, &cap) != cudaSuccess) cudaGetLastError();
+  ordered = ordered && cap == cudaStreamCaptureStatusNone;
+  int rc = PFM_OK;
+  if (ordered) rc = check_cuda(h, cudaStreamWaitEvent(s, h->pad_done, 0), "step graph wait");
+  if (!rc) rc = check_cuda(h, cudaGraphLaunch(h->g_step, s), "step graph launch");
+  if (!rc && ordered) rc = check_cuda(h, cudaEventRecord(h->pad_done, s), "step graph event");
+  return rc;
+}
+
 int pfm3_step(pfm_handle* h, const pfm3_step_fields* f, const pfm_step_params* p, void* stream) {
   int rc = check_fields3(h, f, p);
   if (rc) return rc;
@@ -580,7 +594,7 @@ int pfm3_step(pfm_handle* h, const pfm3_step_fields* f, const pfm_step_params* p
     }
     h->rec_valid = 1;
   }
-  return check_cuda(h, cudaGraphLaunch(h->g_step, s), "step graph launch");
+  return launch_step_graph(h, s);
 }
 
 int pfm2_step(pfm_handle* h, const pfm2_step_fields* f, const pfm_step_params* p, void* stream) {
@@ -598,7 +612,7 @@ int pfm2_step(pfm_handle* h, const pfm2_step_fields* f, const pfm_step_params* p
       return rc;
     }
   }
-  return check_cuda(h, cudaGraphLaunch(h->g_step, s), "step graph launch");
+  return launch_step_graph(h, s);
 }
 
 int pfm_batch_create(pfm_batch** out) {

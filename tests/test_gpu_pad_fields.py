@@ -70,3 +70,40 @@ def test_padded_streams_and_capture():
     for a, b in zip(want + [want[1]], got + [cap]):
         for x, y in zip(a, b):
             assert torch.equal(x, y)
+
+
+def test_padded_beside_a_step_graph():
+    """Midpoint calls on another stream while step graphs of the same handle run: both as when run alone."""
+    res = (72, 64, 80)
+    dx = 1.0 / 64
+
+    def sim():
+        g = torch.Generator(device="cuda").manual_seed(7)
+        u = [torch.randn([n + (a == f) for a, n in enumerate(res)], device="cuda", generator=g) for f in range(3)]
+        for f in range(3):
+            u[f].select(f, 0).zero_()
+            u[f].select(f, res[f]).zero_()
+        return pfm.Sim3D(u, pfm.jittered(res, dx, 8, seed=2), res, dx, reinit_every=4,
+                         poisson_opts=dict(tol=1e-6, tol_mode=1, max_iters=60), graph=True)
+
+    alone = sim()
+    for _ in range(4):
+        alone.step()
+    other = _fields(alone.scene, 9)
+    want = alone.scene.alloc_faces()
+    alone.scene.midpoint(other, want, 0.003)
+    torch.cuda.synchronize()
+    both, side = sim(), torch.cuda.Stream()
+    got = [both.scene.alloc_faces() for _ in range(8)]
+    torch.cuda.synchronize()
+    for k in range(4):
+        both.step()
+        with torch.cuda.stream(side):
+            for mid in got[2 * k:2 * k + 2]:
+                both.scene.midpoint(other, mid, 0.003)
+    torch.cuda.synchronize()
+    for mid in got:
+        for x, y in zip(want, mid):
+            assert torch.equal(x, y)
+    for x, y in zip(alone.u + [alone.pos], both.u + [both.pos]):
+        assert torch.equal(x, y)
