@@ -16,13 +16,15 @@ def test_vector_passes_equal_worklist(opts):
     from pfm import _lib
 
     def make(res, graph):
+        levels = 2 if res[2] % 4 else 0  # every level halves exactly
         dx = 1.0 / res[1]
         g = torch.Generator(device="cuda").manual_seed(sum(res))
         u = [torch.randn([n + (a == f) for a, n in enumerate(res)], device="cuda", generator=g) for f in range(3)]
         for f in range(3):
             u[f].select(f, 0).zero_()
             u[f].select(f, res[f]).zero_()
-        sim = pfm.Sim3D(u, pfm.jittered(res, dx, 8, seed=2), res, dx, reinit_every=4, poisson_opts=opts, graph=graph)
+        sim = pfm.Sim3D(u, pfm.jittered(res, dx, 8, seed=2), res, dx, reinit_every=4, poisson_opts=opts, graph=graph,
+                        mg_levels=levels)
         sim.scene.set_tuning(_lib.TUNE_MG_CLUSTER, 0)
         return sim
 
