@@ -41,3 +41,25 @@ def test_vector_passes_equal_worklist(opts):
         assert torch.equal(a.p, b.p)
         for f in range(3):
             assert torch.equal(a.u[f], b.u[f])
+
+
+@pytest.mark.parametrize("res,precision,walls", [((141, 200, 184), "fp16", [[2, 2]] * 3),
+                                                 ((143, 250, 144), "bf16", [[1, 2], [2, 1], [2, 1]]),
+                                                 ((142, 196, 184), "fp16", [[2, 1], [1, 2], [1, 2]])])
+def test_plane_march_equals_tma_tiles(res, precision, walls):
+    """16-bit levels large enough for the half-sweep that goes up several planes, with 1 to 3 planes left at the
+    end: bitwise the tiled kernel, whose update is the per-cell one's."""
+    import pfm
+    from pfm import _lib
+
+    sc = pfm.Scene(3, res, 1.0 / res[1], 0, mg_levels=1, boundary=walls, bottom_smoothing=3)
+    g = torch.Generator(device="cuda").manual_seed(11)
+    u0 = [torch.randn(s, device="cuda", generator=g) for s in sc.face_shapes]
+    out = []
+    for tma in (0, 1):
+        sc.set_tuning(_lib.TUNE_SMOOTH_TMA, tma)
+        p = torch.zeros(sc.cell_shape, device="cuda")
+        sc.poisson([x.clone() for x in u0], p, precision=precision, tol=1e-6, tol_mode=1, max_iters=3)
+        out.append(p)
+    assert torch.isfinite(out[0]).all() and out[0].abs().max() > 0
+    assert torch.equal(out[0], out[1])
