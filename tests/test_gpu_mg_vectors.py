@@ -63,3 +63,28 @@ def test_plane_march_equals_tma_tiles(res, precision, walls):
         out.append(p)
     assert torch.isfinite(out[0]).all() and out[0].abs().max() > 0
     assert torch.equal(out[0], out[1])
+
+
+@pytest.mark.parametrize("nz", [31, 32, 63, 64, 127, 128, 160])
+@pytest.mark.parametrize("walls", [[2, 2], [1, 2], [2, 1]])
+def test_z_faces_lose_the_pressure_gradient(nz, walls):
+    """The last axis' faces after a projection: bitwise u - (p above - p below), zero on the walls."""
+    import pfm
+
+    res = (9, 7, nz)
+    sc = pfm.Scene(3, res, 1.0 / 8, 0, mg_levels=1, boundary=[[2, 2], [2, 2], walls])
+    g = torch.Generator(device="cuda").manual_seed(nz)
+    u = [torch.randn(s, device="cuda", generator=g) for s in sc.face_shapes]
+    if walls[0] == 2:
+        u[2][..., 0] = 0
+    if walls[1] == 2:
+        u[2][..., nz] = 0
+    before, p = u[2].clone(), torch.zeros(sc.cell_shape, device="cuda")
+    sc.poisson(u, p, tol=1e-6, tol_mode=1, max_iters=20)
+    pad = torch.zeros(res[0], res[1], 1, device="cuda")
+    want = before - (torch.cat([p, pad], 2) - torch.cat([pad, p], 2))
+    if walls[0] == 2:
+        want[..., 0] = 0
+    if walls[1] == 2:
+        want[..., nz] = 0
+    assert torch.equal(u[2], want)
