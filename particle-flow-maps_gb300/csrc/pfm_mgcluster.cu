@@ -4,15 +4,15 @@
 // A solve of a few hundred thousand cells is a serial chain: at 256 x 256 one PCG iteration is 27
 // kernels, 16 of them half-sweeps of 2-8 us of launch, drain and memory latency for well under 1 us
 // of work.  Here the multigrid vectors of every level live in the shared memory of one cluster of up to
-// 16 CTAs, a half-sweep ends with a cluster barrier instead of a launch, and the iteration's scalars
-// never leave the cluster.
+// 16 CTAs, a half-sweep ends with its edge rows' arrival in the neighbour's memory instead of a launch,
+// and the iteration's scalars never leave the cluster.
 //
 //  * Rows (the first axis) of the distributed levels l0 .. lg-1 are split into contiguous shares, one
 //    per CTA, nested so that a coarse row and its two fine rows have the same owner.  A share holds a
 //    ghost row on either side; the owner of a boundary row stores it into its neighbour's ghost row
 //    as well (distributed shared memory), so every stencil reads local memory.
-//  * The levels from lg on (at most tail_cells cells) are solo: the first CTA runs them alone, FP32,
-//    while the others wait at the next cluster barrier.
+//  * The levels from lg on (at most tail_cells cells) are solo: the first CTA runs them alone, FP32;
+//    the rows it restricts from and prolongs to travel by st.async, and the others wait for theirs.
 //  * A level's vectors are split by colour ([colour][row][middle][half of the last axis, rounded up to
 //    four]): a thread updates four consecutive cells of a colour with 16-byte (8-byte) accesses, free of
 //    bank conflicts.  The cells beyond the last axis stay zero.
@@ -811,18 +811,49 @@ struct ClusterRed {  // in shared memory
   uint64_t full[2];     // the ranks' totals of a buffer have arrived
 };
 
+// The sum of r, for its mean: r's own mean was subtracted before, so the terms cancel to some 1e-11 of their
+// magnitudes, and the 1e-15 that pairs lose would be 1e-4 of the mean.  A second compensation per thread and FP64
+// above it keep what the grid-wide solve's FP64 sums keep.  3D only (64^3: with pairs three steps ended on
+// other last bits than the grid-wide solve's in 5 of 6 fields, with this in 2; in 2D they agreed either way), for 12 us
+// per solve of a 64^3 step of 1200.
+struct WideSum {
+  float s = 0.f, c = 0.f, d = 0.f;
+  __device__ __forceinline__ void add(float x) {
+    const float t = s + x, e = (fabsf(s) >= fabsf(x)) ? ((s - t) + x) : ((x - t) + s);
+    s = t;
+    const float u = c + e;
+    d += (fabsf(c) >= fabsf(e)) ? ((c - u) + e) : ((e - u) + c);
+    c = u;
+  }
+  __device__ __forceinline__ double value() const { return (double)s + ((double)c + (double)d); }
+};
+__device__ __forceinline__ Pair bits_of(double x) {
+  return Pair{__int_as_float(__double2loint(x)), __int_as_float(__double2hiint(x))};
+}
+__device__ __forceinline__ double of_bits(Pair p) {
+  return __hiloint2double(__float_as_int(p.c), __float_as_int(p.s));
+}
+template <int WIDTH>
+__device__ __forceinline__ double wide_reduce(double v) {
+#pragma unroll
+  for (int o = WIDTH / 2; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+  return v;
+}
+
 // The cluster's total of N sums, in total[] of the calling CTA's first warp (the others' are
-// undefined).  A non-finite term gives a non-finite total.  Every CTA sends its total to every CTA with
+// undefined).  With WIDE the last of them is the sum of `wide`, as the bits of a double.  A non-finite term gives a non-finite total.  Every CTA sends its total to every CTA with
 // st.async; `uses` numbers the calls (two buffers alternate: a CTA is at most one call ahead).
-template <int N>
+template <int N, bool WIDE = false>
 __device__ __forceinline__ void cluster_sum(const CompSum (&v)[N], ClusterRed* red, Exchange* ex, int nc, int rank,
-                                            unsigned& uses, Pair (&total)[N]) {
+                                            unsigned& uses, Pair (&total)[N], double wide = 0.0) {
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, buf = (int)(uses & 1u);
   const unsigned parity = (uses >> 1) & 1u;
   ++uses;
 #pragma unroll
   for (int n = 0; n < N; ++n) {
-    const Pair w = pair_reduce<32>(Pair{v[n].s, v[n].c});
+    Pair w;
+    if (WIDE && n == N - 1) w = bits_of(wide_reduce<32>(wide));
+    else w = pair_reduce<32>(Pair{v[n].s, v[n].c});
     if (lane == 0) red->warp[n][wid] = w;
   }
   __syncthreads();
@@ -830,7 +861,9 @@ __device__ __forceinline__ void cluster_sum(const CompSum (&v)[N], ClusterRed* r
     if (lane == 0) mbar_expect_tx(&red->full[buf], (unsigned)(N * nc * sizeof(Pair)));
 #pragma unroll
     for (int n = 0; n < N; ++n) {
-      const Pair w = pair_reduce<kWarps>(red->warp[n][lane % kWarps]);
+      Pair w = red->warp[n][lane % kWarps];
+      if (WIDE && n == N - 1) w = bits_of(wide_reduce<kWarps>(of_bits(w)));
+      else w = pair_reduce<kWarps>(w);
       if (lane < nc)
         push_async<8>(remote_addr(su32(&red->slot[buf][n][rank]), lane), &w, remote_addr(su32(&red->full[buf]), lane));
     }
@@ -839,7 +872,8 @@ __device__ __forceinline__ void cluster_sum(const CompSum (&v)[N], ClusterRed* r
     for (int n = 0; n < N; ++n) {
       Pair w{0.f, 0.f};
       if ((lane & 15) < nc) w = red->slot[buf][n][lane & 15];
-      total[n] = pair_reduce<16>(w);
+      if (WIDE && n == N - 1) total[n] = bits_of(wide_reduce<16>(of_bits(w)));
+      else total[n] = pair_reduce<16>(w);
     }
   }
 }
@@ -938,7 +972,7 @@ __global__ void __launch_bounds__(kT, 1) k_cluster_solve(const __grid_constant__
     *reinterpret_cast<Vec<2, S>*>(rl + c * v.cr + e) = pack<2, S>(p);
     *reinterpret_cast<Vec<2, S>*>(rl + (1 - c) * v.cr + e) = pack<2, S>(q);
   };
-  auto add4 = [](CompSum& q, float4 x) {
+  auto add4 = [](auto& q, float4 x) {
     q.add(x.x);
     q.add(x.y);
     q.add(x.z);
@@ -970,10 +1004,12 @@ __global__ void __launch_bounds__(kT, 1) k_cluster_solve(const __grid_constant__
                        (float)cell_neighbours<D>(v, P.bc, rn, k + 3) * c.w - n[3]);
   };
   auto mean_of = [&](Pair t) {
+    if (D == 3) return (float)(of_bits(t) * ((double)A.inv_n_s + (double)A.inv_n_c));
     const float m = t.s * A.inv_n_s;
     return m + (fmaf(t.s, A.inv_n_s, -m) + fmaf(t.s, A.inv_n_c, t.c * A.inv_n_s));
   };
-  // 1 / RMS rounded to f32: a Newton step on the f32 reciprocal square root with the pair's remainder
+  constexpr bool WIDE = D == 3;
+  using MeanSum = std::conditional_t<WIDE, WideSum, CompSum>;
   auto scale_of = [&](Pair t) {
     const float m = t.s * A.inv_n_s, mc = fmaf(t.s, A.inv_n_s, -m) + fmaf(t.s, A.inv_n_c, t.c * A.inv_n_s);
     if (!(t.s > 0.f)) return 1.f;
@@ -999,7 +1035,7 @@ __global__ void __launch_bounds__(kT, 1) k_cluster_solve(const __grid_constant__
 
   // ---- setup: r0, recenter, b, the warm start's residual, r0.r0
   {
-    CompSum q;
+    MeanSum q;
     for_groups([&](int e, int g, int, int, int, int c) {
       const float4 b = ld4f(A.rhs + g);
       put4(rf, v.cr, e, c, b);
@@ -1008,7 +1044,7 @@ __global__ void __launch_bounds__(kT, 1) k_cluster_solve(const __grid_constant__
     });
     if (A.neu) {
       Pair t[1];
-      cluster_sum<1>({q}, &red, &ex, P.nc, rank, uses, t);
+      cluster_sum<1, WIDE>({CompSum{q.s, q.c}}, &red, &ex, P.nc, rank, uses, t, WIDE ? q.value() : 0.0);
       if (tid == 0) sc.mean = mean_of(t[0]);
     }
     __syncthreads();
@@ -1119,7 +1155,8 @@ __global__ void __launch_bounds__(kT, 1) k_cluster_solve(const __grid_constant__
     }
     {
       const float alpha = sc.alpha;
-      CompSum qr, qm;
+      CompSum qr;
+      MeanSum qm;
       for_groups([&](int e, int g, int, int, int, int c) {
         const float4 x = ld4f(A.x + g), p = ld4f(A.p + g), a = ld4f(A.Ap + g);
         float4 r = get4(rf, v.cr, e, c);
@@ -1131,7 +1168,7 @@ __global__ void __launch_bounds__(kT, 1) k_cluster_solve(const __grid_constant__
         add4(qm, r);
       });
       Pair t[2];
-      cluster_sum<2>({qr, qm}, &red, &ex, P.nc, rank, uses, t);
+      cluster_sum<2, WIDE>({qr, CompSum{qm.s, qm.c}}, &red, &ex, P.nc, rank, uses, t, WIDE ? qm.value() : 0.0);
       if (tid == 0) {
         sc.rTr = t[0];
         if (ex.lost) sc.done = 4;
