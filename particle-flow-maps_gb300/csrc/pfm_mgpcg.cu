@@ -722,9 +722,9 @@ __device__ __forceinline__ void smooth8_blk(S* __restrict__ z, const S* __restri
 // plane's neighbour, the next plane's centre and the one after's neighbour below, read and converted once, and
 // the rows' addresses are formed once.  Element for element smooth8_blk.
 // 16-bit levels only, and where the threads fill the resident blocks once (kMarchCells): 256^3 cells 19.2 -> 16.0 us,
-// 192^3 9.2 -> 8.4, 128^3 4.2 either way, below that too few loads are in flight (96^3 2.5 -> 3.6).  2 and 8 planes
-// took 18.2 and 17.0 us at 256^3; the next plane's loads issued before the current one's update, at 3 blocks
-// per SM for their registers, 17.5.  FP32 levels: 34.6 -> 38 us.
+// 192^3 9.2 -> 8.4, 128^3 4.2 either way, below that too few loads are in flight (96^3 2.5 -> 3.6).  2 planes took
+// 18.4 us at 256^3, 8 the same as 4 (and need twice the cells to fill the blocks); the next plane's loads issued before
+// the current one's update, at 3 blocks per SM for their registers, 17.6.  FP32 levels: 34.6 -> 38 us.
 constexpr int kMarch = 4;
 constexpr int64_t kMarchCells = (int64_t)152 * PFM_SMOOTH8_MINB16 * 256 * 8 * kMarch;
 

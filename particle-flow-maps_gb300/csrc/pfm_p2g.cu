@@ -239,11 +239,11 @@ __global__ void __launch_bounds__(kBinThreads) k_payload2(const int* __restrict_
 //
 // Tile of 4 x 4 x 16 cells (256 threads, 128 registers each): 16 along the last axis, the length
 // of the seeding order's cell groups (pfm_seed_jittered), so the records of a group's particles
-// are read by one tile in one launch (with 8-cell tiles a group's 128-particle runs are split
-// between tiles of different parity launches and every record line is fetched twice).  With a
+// are read by one tile (with 8-cell tiles a group's 128-particle runs are split between two tiles
+// and every record line is fetched twice).  With a
 // ring of 2 a block holds 90 KB of shared memory, so two blocks share an SM and one block's
-// barriers and window merge overlap the other's particle loop.  Measured at 256^3 (the P2G phase:
-// sort, 8 tile launches, normalisation): 4 x 8 x 16 cells with a ring of 5 (one 224 KB block per
+// barriers and window merge overlap the other's particle loop.  Measured at 256^3 (the P2G phase
+// when the tiles still ran in 8 launches by parity): 4 x 8 x 16 cells with a ring of 5 (one 224 KB block per
 // SM) 10.33 ms; 4 x 4 x 16 with rings of 4 / 3 / 2 / 1 (two blocks per SM) 9.65 / 9.37 / 9.25 /
 // 10.96 ms; 4 x 3 x 16 with rings of 5 / 4: 11.14 / 10.82 ms.
 #ifndef PFM_TILE_X
