@@ -458,13 +458,16 @@ inline void with_cube(const pfm_handle* h, Fn&& f) {
 }
 
 // The pitch of the padded copies of a grid's fields: the smallest of 128, 256 and 512 that holds its rows and
-// planes, where that is at most four times the fields; 0 (no copies) for cubes with an instance of their own and
-// for grids below 64^3 cells, where a copy takes as long as it saves (3 us of a midpoint's 77).
+// planes, where that is at most four times the fields and a copy has fewer than 2^31 elements (the kernels index
+// it with 32-bit integers, as the fields: 9000 x 256 x 256 cells at pitch 512 would be 2.4e9); 0 (no copies) for
+// cubes with an instance of their own and for grids below 64^3 cells, where a copy takes as long as it saves (3 us
+// of a midpoint's 77).
 inline int pad_pitch_of(const MacGeom& g) {
   if (g.dim != 3 || cube_extent(g) || (int64_t)g.N[0] * g.N[1] * g.N[2] < 262144) return 0;
   const int n = (g.N[1] > g.N[2] ? g.N[1] : g.N[2]) + 1;
   const int p = n <= 128 ? 128 : n <= 256 ? 256 : n <= 512 ? 512 : 0;
-  return p && (int64_t)p * p <= 4ll * (g.N[1] + 1) * (g.N[2] + 1) ? p : 0;
+  const int64_t plane = (int64_t)p * p;
+  return plane <= 4ll * (g.N[1] + 1) * (g.N[2] + 1) && (g.N[0] + 1) * plane < (int64_t(1) << 31) ? p : 0;
 }
 inline size_t pad_set_bytes(const MacGeom& g, int pitch) {
   return 3 * (size_t)(g.N[0] + 1) * pitch * pitch * sizeof(float);
