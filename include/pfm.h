@@ -154,6 +154,9 @@ int pfm_measure_fp32_peak(float* sink, int blocks_per_sm, int iters, int reps, i
                                      one's V-cycle; 0: grid-wide kernels (1).  The other MGPCG keys act
                                      on what runs grid-wide; sums are grouped differently, so the two
                                      settings agree to rounding. */
+#define PFM_TUNE_MG_CLUSTER_WAIT 7 /* not a launch shape: the limit in microseconds, 0..4000000 (2000000), of a wait
+                                     between the blocks of that cluster.  A solve in which one runs out ends with
+                                     PFM_ERR_CUDA and the handle stays usable; 0 lets every wait run out. */
 int pfm_set_tuning(pfm_handle* h, int key, int value);
 int pfm_get_tuning(const pfm_handle* h, int key, int* value);
 

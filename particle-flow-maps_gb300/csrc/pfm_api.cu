@@ -236,6 +236,7 @@ int pfm_create(const pfm_config* cfg, pfm_handle** out) {
   h->cube_kernels = 1;
   h->mid_centre = 1;
   h->mg_cluster = 1;
+  h->cluster_wait_us = 2000000;
   if (cudaHostAlloc((void**)&h->h_state, sizeof(SolveState), cudaHostAllocDefault) != cudaSuccess) {
     cudaGetLastError();
     if (h->pad_done) cudaEventDestroy(h->pad_done);
@@ -315,6 +316,9 @@ int pfm_set_tuning(pfm_handle* h, int key, int value) {
   } else if (key == PFM_TUNE_MG_CLUSTER) {
     if (value != 0 && value != 1) return set_error(h, PFM_ERR_ARG, "MGPCG cluster form must be 0 or 1");
     h->mg_cluster = value;
+  } else if (key == PFM_TUNE_MG_CLUSTER_WAIT) {
+    if (value < 0 || value > 4000000) return set_error(h, PFM_ERR_ARG, "MGPCG cluster wait must be 0 to 4000000 us");
+    h->cluster_wait_us = value;
   } else {
     return set_error(h, PFM_ERR_ARG, "unknown tuning key");
   }
@@ -337,6 +341,7 @@ int pfm_get_tuning(const pfm_handle* h, int key, int* value) {
   else if (key == PFM_TUNE_CUBE_KERNELS) *value = h->cube_kernels;
   else if (key == PFM_TUNE_MIDPOINT_CENTRE) *value = h->mid_centre;
   else if (key == PFM_TUNE_MG_CLUSTER) *value = h->mg_cluster;
+  else if (key == PFM_TUNE_MG_CLUSTER_WAIT) *value = h->cluster_wait_us;
   else return PFM_ERR_ARG;
   return PFM_OK;
 }

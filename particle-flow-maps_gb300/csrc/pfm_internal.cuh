@@ -38,7 +38,7 @@ struct SolveState {
   float mean;      // recenter mean
   float hscale;    // 16-bit level storage holds r * hscale (unit RMS), z is read back / hscale
   int it;          // completed iterations
-  int done;        // 1 converged, 2 iteration limit, 3 non-finite, 4 a tile copy did not arrive
+  int done;        // 1 converged, 2 iteration limit, 3 non-finite, 4 a bounded wait of a kernel gave up
   int conv_it;     // iteration index at convergence
   unsigned ticket; // last-block counter of the reductions
   int it_stop;     // the device loop pauses when `it` reaches this count
@@ -152,6 +152,7 @@ struct pfm_handle {
   int smooth_tma;  // 3D 16-bit MGPCG levels smoothed from TMA-staged tiles (same results)
   int cube_kernels;  // 3D interpolating kernels instantiated for the grid's cube extent (same results)
   int mg_cluster;    // small MGPCG solves and coarse V-cycle levels on one thread-block cluster
+  int cluster_wait_us;  // limit of a wait between that cluster's CTAs
   int mid_centre;    // 3D midpoint's first stage at the face centre in constant-weight form (same results)
   // whole-step graph (pfm3_step / pfm2_step), rebuilt when its fields or parameters change
   cudaGraphExec_t g_step;

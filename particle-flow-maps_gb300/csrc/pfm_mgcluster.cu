@@ -24,8 +24,12 @@
 //    every cell update is bitwise the grid-wide kernels'.
 //
 // The waits for other CTAs' rows and totals are mbarrier waits bounded in time; the others are hardware
-// cluster or block barriers that all threads reach the same number of times: the branches around them
-// depend only on values every CTA computes alike.
+// cluster or block barriers that all threads reach the same number of times.  A wait that gives up says so in
+// every CTA's shared memory (Exchange::lost).  From then on totals, and what is decided on them, may differ
+// between CTAs, so a CTA acts on a decision to end only behind one more cluster barrier: whatever each of them
+// decided, they meet at that barrier, and behind it all see that a wait gave up before it and end together
+// (pass_barrier).  A thread that has seen it neither pushes nor expects rows any more, and no CTA returns its
+// shared memory before the rows in flight have landed (leave).
 //
 // Measured (one PCG iteration, FP32, GB300): 128^2 103 -> 23 us, 256^2 125 -> 31 us, 512^2 165 -> 54 us,
 // 32^3 107 -> 28 us, 64^3 155 -> 60 us; the coarse levels of 128^3 and 1024^2 as one launch: 210 -> 185 and
@@ -73,11 +77,14 @@ __device__ __forceinline__ T* remote(T* p, int rank) {
 // level restricts and prolongs within a share) is [b0, b1), the share above begins at up0.
 struct Me {
   int rank, up0, b0, b1;
+  unsigned limit;  // of a wait, in ns; 0: every wait gives up at once
+  int passed;   // cluster barriers so far
+  bool gone;    // this thread has seen that a wait gave up: it pushes and expects nothing any more
 };
 
 __device__ __forceinline__ Me who_am_i(const CPlan& P) {
   const int rank = (int)cg::this_cluster().block_rank();
-  return Me{rank, (rank - 1) * P.nbase / P.nc, rank * P.nbase / P.nc, (rank + 1) * P.nbase / P.nc};
+  return Me{rank, (rank - 1) * P.nbase / P.nc, rank * P.nbase / P.nc, (rank + 1) * P.nbase / P.nc, P.wait_ns, 0, false};
 }
 
 struct Share {  // this CTA's rows of a level
@@ -268,7 +275,7 @@ __device__ __forceinline__ void update_spot(const F* __restrict__ zo, const F* _
 struct Exchange {
   uint64_t full[2];  // in shared memory, one arrival (the expected bytes) per half-sweep
   uint64_t up, down;  // per V-cycle: the solo level's r is complete (rank 0); its z rows are here (the others)
-  int lost;          // a row did not arrive in time: later waits return at once
+  int lost;          // 0, or once a wait gave up 1 + the cluster barriers passed by then: later waits return at once
 };
 
 __device__ __forceinline__ uint32_t remote_addr(uint32_t local, int rank) {
@@ -295,19 +302,40 @@ __device__ __forceinline__ void push_async(uint32_t dst, const void* src, uint32
                  : "memory");
 }
 
-// Waits for the phase of `bar` with the given parity; gives up after kWaitNs and says so in every CTA's
-// `lost`, which ends their waits and the solve.
-__device__ __forceinline__ void wait_rows(Exchange* x, uint64_t* bar, unsigned parity) {
-  if (mbar_try_wait_cluster(bar, parity)) return;
+// Waits for the phase of `bar` with the given parity; false (and me.gone) once a wait has given up.  This one does
+// after me.limit and says so in every CTA's `lost`, which ends their waits and the solve.
+__device__ __forceinline__ bool wait_rows(Exchange* x, uint64_t* bar, unsigned parity, Me& me) {
+  if (me.gone) return false;
+  if (me.limit && mbar_try_wait_cluster(bar, parity)) return true;
   const unsigned long long t0 = now_ns();
-  while (!mbar_try_wait_cluster(bar, parity)) {
-    if (*(volatile int*)&x->lost) return;
-    if (now_ns() - t0 > kWaitNs) {
+  while (!(me.limit && mbar_try_wait_cluster(bar, parity))) {
+    me.gone = *(volatile int*)&x->lost != 0;
+    if (!me.gone && (!me.limit || now_ns() - t0 > me.limit)) {
       const int n = (int)cg::this_cluster().num_blocks();
-      for (int c = 0; c < n; ++c) *(volatile int*)remote(&x->lost, c) = 1;
-      return;
+      for (int c = 0; c < n; ++c) *(volatile int*)remote(&x->lost, c) = me.passed + 1;
+      me.gone = true;
     }
+    if (me.gone) return false;
   }
+  return true;
+}
+
+// A cluster barrier; true if a wait gave up before it -- the same answer in every thread of the cluster: what was
+// written before the barrier is seen by all, and a wait that gives up behind it writes a larger number.
+__device__ __forceinline__ bool pass_barrier(const Exchange* x, Me& me) {
+  cluster_barrier();
+  ++me.passed;
+  const int lost = *(const volatile int*)&x->lost;
+  return lost != 0 && lost <= me.passed;
+}
+
+// The end of a cluster in which a wait gave up, behind the barrier that said so: nobody pushes any more, and rows
+// in flight land (in well under a microsecond) before any CTA gives its shared memory back.
+__device__ __forceinline__ void leave() {
+  const unsigned long long t0 = now_ns();
+  while (now_ns() - t0 < 1000000) {
+  }
+  cluster_barrier();
 }
 
 // `half_sweeps` half-sweeps of a distributed level, colours `first`, 1 - first, ..; `fresh`: z starts at
@@ -315,14 +343,15 @@ __device__ __forceinline__ void wait_rows(Exchange* x, uint64_t* bar, unsigned p
 // four vectors keeps their places in registers (64^3 on 16 CTAs has four).
 template <int D, typename S>
 __device__ __forceinline__ void sweeps_dist(const CPlan& P, const CLev& v, unsigned char* sm, const float2* inv,
-                                            Exchange* ex, const Me& me, int half_sweeps, int first, bool fresh,
+                                            Exchange* ex, Me& me, int half_sweeps, int first, bool fresh,
                                             unsigned& count) {
   using VS = Vec<4, S>;
   const int lo = me.b0 << v.shift, rows = (me.b1 - me.b0) << v.shift;
   const int plane = v.plane, T = rows * plane / 4;
   S* z = reinterpret_cast<S*>(sm + v.z) + plane;  // this share's row 0 of colour 0
   const S* r = reinterpret_cast<const S*>(sm + v.r);
-  const bool up = me.rank > 0, down = me.rank + 1 < P.nc;
+  if (*(volatile int*)&ex->lost) me.gone = true;
+  bool up = me.rank > 0 && !me.gone, down = me.rank + 1 < P.nc && !me.gone;
   // element e of this share in the neighbours' ghost rows, of colour 0: its first row above, its last below
   const uint32_t zs = su32(z - plane);
   const uint32_t up_z =
@@ -330,7 +359,7 @@ __device__ __forceinline__ void sweeps_dist(const CPlan& P, const CLev& v, unsig
   const uint32_t dn_z = down ? remote_addr(zs, me.rank + 1) - (uint32_t)((rows - 1) * plane * (int)sizeof(S)) : 0u;
   const uint32_t bs = su32(&ex->full[0]);
   const uint32_t up_b = up ? remote_addr(bs, me.rank - 1) : 0u, dn_b = down ? remote_addr(bs, me.rank + 1) : 0u;
-  const unsigned expect = (unsigned)((up + down) * plane * (int)sizeof(S));
+  unsigned expect = (unsigned)((up + down) * plane * (int)sizeof(S));
   const bool one = T <= kT, four = T <= 4 * kT;
   Spot mine{};
   Place at[4] = {};
@@ -369,7 +398,10 @@ __device__ __forceinline__ void sweeps_dist(const CPlan& P, const CLev& v, unsig
       for (int t = threadIdx.x; t < T; t += kT) update(unpack<D>(v, P.bc, inv, make_place<D>(v, P.bc, lo, t)));
     }
     __syncthreads();
-    if (expect) wait_rows(ex, &ex->full[which], (count >> 1) & 1u);
+    if (expect && !wait_rows(ex, &ex->full[which], (count >> 1) & 1u, me)) {
+      up = down = false;
+      expect = 0;
+    }
     ++count;
   }
 }
@@ -656,7 +688,7 @@ __device__ __forceinline__ void push_solo(const CPlan& P, const CLev& v, const C
 // the first half-sweep up before anything reads it), so that no barrier parts the prolongation from that push.
 template <int D, typename S>
 __device__ __forceinline__ void cluster_vcycle(const CPlan& P, unsigned char* sm, const float2* inv, Exchange* ex,
-                                               const Me& me, unsigned& count, unsigned& cycles) {
+                                               Me& me, unsigned& count, unsigned& cycles) {
   const int bottom = P.L - 1, n = (P.lg < P.L ? P.lg : bottom) - P.l0;  // distributed levels that restrict
   const unsigned parity = cycles++ & 1u;
   // down: t = 0 .. n-1; the solo levels or the distributed bottom: t = n; up: t = n+1 .. 2n
@@ -665,10 +697,10 @@ __device__ __forceinline__ void cluster_vcycle(const CPlan& P, unsigned char* sm
     if (t == n && P.lg < P.L) {
       if (me.rank == 0) {
         const CLev v = P.lv[P.lg - 1], c = P.lv[P.lg];
-        if (threadIdx.x == 0) mbar_expect_tx(&ex->up, (unsigned)(c.n0 * c.n1 * (v.hs >> 2) * 16));
-        wait_rows(ex, &ex->up, parity);
+        if (threadIdx.x == 0 && !me.gone) mbar_expect_tx(&ex->up, (unsigned)(c.n0 * c.n1 * (v.hs >> 2) * 16));
+        wait_rows(ex, &ex->up, parity, me);
         solo_vcycle<D>(P, sm, inv);
-        push_solo(P, v, c, sm, ex);
+        if (!me.gone) push_solo(P, v, c, sm, ex);
       }
       continue;
     }
@@ -684,8 +716,9 @@ __device__ __forceinline__ void cluster_vcycle(const CPlan& P, unsigned char* sm
                                  s.lo >> 1);
       } else {
         if (me.rank > 0) {
-          if (threadIdx.x == 0) mbar_expect_tx(&ex->down, (unsigned)(rows_under(v, s.lo, s.rows).rows * c.plane * 8));
-          wait_rows(ex, &ex->down, parity);
+          if (threadIdx.x == 0 && !me.gone)
+            mbar_expect_tx(&ex->down, (unsigned)(rows_under(v, s.lo, s.rows).rows * c.plane * 8));
+          wait_rows(ex, &ex->down, parity, me);
         }
         prolong_rows<D, S, S, float>(v, c, z, s.lo, i0, i1, s.lo, s.lo + s.rows,
                                      reinterpret_cast<const float*>(sm + c.z) + c.plane, 0);
@@ -703,8 +736,9 @@ __device__ __forceinline__ void cluster_vcycle(const CPlan& P, unsigned char* sm
         __syncthreads();
       } else {
         float* rc = reinterpret_cast<float*>(sm + c.r);
-        restrict_rows<D, S, S, float>(v, c, P.bc, z, r, s.lo, rc, 0, s.lo >> 1, s.rows >> 1, remote_addr(su32(rc), 0),
-                                   remote_addr(su32(&ex->up), 0));
+        // (a thread that pushes no more writes its own CTA's rows instead, which nothing reads)
+        restrict_rows<D, S, S, float>(v, c, P.bc, z, r, s.lo, rc, 0, s.lo >> 1, s.rows >> 1,
+                                   me.gone ? 0 : remote_addr(su32(rc), 0), remote_addr(su32(&ex->up), 0));
       }
     }
   }
@@ -761,7 +795,7 @@ __global__ void __launch_bounds__(kT, 1) k_cluster_tail(S* __restrict__ zg, cons
   __shared__ float2 inv[8];
   __shared__ Exchange ex;
   if (st && st->done) return;  // the same for the whole cluster
-  const Me me = who_am_i(P);
+  Me me = who_am_i(P);
   unsigned count = 0, cycles = 0;
   init_exchange(&ex);
   fill_inverses(inv);
@@ -786,7 +820,7 @@ __global__ void __launch_bounds__(kT, 1) k_cluster_tail(S* __restrict__ zg, cons
     r[c * v.cr + e] = rg[g];
     if (both) r[(1 - c) * v.cr + e] = rg[g + 1];
   }
-  cluster_barrier();  // every CTA of the cluster runs before the first remote store
+  pass_barrier(&ex, me);  // every CTA of the cluster runs before the first remote store
   cluster_vcycle<D, S>(P, sm, inv, &ex, me, count, cycles);
   const S* z = reinterpret_cast<const S*>(sm + v.z) + v.plane;
   for (int t = threadIdx.x; t < T; t += kT) {
@@ -796,8 +830,10 @@ __global__ void __launch_bounds__(kT, 1) k_cluster_tail(S* __restrict__ zg, cons
     zg[g] = z[c * v.cz + e];
     if (both) zg[g + 1] = z[(1 - c) * v.cz + e];
   }
-  if (ex.lost && threadIdx.x == 0 && st) atomicCAS(&st->done, 0, 4);
-  cluster_barrier();  // no CTA leaves while another may still read its shared memory
+  if (pass_barrier(&ex, me)) {  // no CTA leaves while another may still write its shared memory
+    if (threadIdx.x == 0 && st) atomicCAS(&st->done, 0, 4);
+    leave();
+  }
 }
 
 // ---------------------------------------------------------------------------------------------
@@ -844,7 +880,7 @@ __device__ __forceinline__ double wide_reduce(double v) {
 // undefined).  With WIDE the last of them is the sum of `wide`, as the bits of a double.  A non-finite term gives a non-finite total.  Every CTA sends its total to every CTA with
 // st.async; `uses` numbers the calls (two buffers alternate: a CTA is at most one call ahead).
 template <int N, bool WIDE = false>
-__device__ __forceinline__ void cluster_sum(const CompSum (&v)[N], ClusterRed* red, Exchange* ex, int nc, int rank,
+__device__ __forceinline__ void cluster_sum(const CompSum (&v)[N], ClusterRed* red, Exchange* ex, int nc, Me& me,
                                             unsigned& uses, Pair (&total)[N], double wide = 0.0) {
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, buf = (int)(uses & 1u);
   const unsigned parity = (uses >> 1) & 1u;
@@ -858,16 +894,16 @@ __device__ __forceinline__ void cluster_sum(const CompSum (&v)[N], ClusterRed* r
   }
   __syncthreads();
   if (wid == 0) {
-    if (lane == 0) mbar_expect_tx(&red->full[buf], (unsigned)(N * nc * sizeof(Pair)));
+    if (lane == 0 && !me.gone) mbar_expect_tx(&red->full[buf], (unsigned)(N * nc * sizeof(Pair)));
 #pragma unroll
     for (int n = 0; n < N; ++n) {
       Pair w = red->warp[n][lane % kWarps];
       if (WIDE && n == N - 1) w = bits_of(wide_reduce<kWarps>(of_bits(w)));
       else w = pair_reduce<kWarps>(w);
-      if (lane < nc)
-        push_async<8>(remote_addr(su32(&red->slot[buf][n][rank]), lane), &w, remote_addr(su32(&red->full[buf]), lane));
+      if (lane < nc && !me.gone)
+        push_async<8>(remote_addr(su32(&red->slot[buf][n][me.rank]), lane), &w, remote_addr(su32(&red->full[buf]), lane));
     }
-    wait_rows(ex, &red->full[buf], parity);
+    wait_rows(ex, &red->full[buf], parity, me);
 #pragma unroll
     for (int n = 0; n < N; ++n) {
       Pair w{0.f, 0.f};
@@ -910,8 +946,8 @@ __global__ void __launch_bounds__(kT, 1) k_cluster_solve(const __grid_constant__
   __shared__ Scalars sc;
   __shared__ Exchange ex;
   constexpr bool MIXED = sizeof(S) == 2;
-  const Me me = who_am_i(P);
-  const int rank = me.rank, tid = threadIdx.x;
+  Me me = who_am_i(P);
+  const int tid = threadIdx.x;
   unsigned count = 0, cycles = 0;
   init_exchange(&ex);
   fill_inverses(inv);
@@ -923,7 +959,7 @@ __global__ void __launch_bounds__(kT, 1) k_cluster_solve(const __grid_constant__
     const Pair none{0.f, 0.f};
     sc = Scalars{0.f, 0.f, 0.f, 1.f, 0, 0, 0, none, none, none, none, none, none, Pair{A.tol_s, A.tol_c}};
   }
-  cluster_barrier();  // every CTA of the cluster runs before the first remote store
+  pass_barrier(&ex, me);  // every CTA of the cluster runs before the first remote store
   const CLev v = P.lv[0];
   const Share s = share_of(v, me);
   const int T = s.rows * v.n1 * (v.half / 2);  // groups of four cells (2h .. 2h + 3) of this CTA
@@ -1019,9 +1055,9 @@ __global__ void __launch_bounds__(kT, 1) k_cluster_solve(const __grid_constant__
     const float e = fmaf(-my, y, 1.f) - myc * y;             // 1 - m y y
     return fmaf(0.5f * y, e, y);
   };
-  // |b - A x|^2 of the current x into thread 0's rTr_true
+  // |b - A x|^2 of the current x into thread 0's rTr_true; true if a wait gave up before
   auto true_residual = [&]() {
-    cluster_barrier();  // x of the neighbouring rows
+    if (pass_barrier(&ex, me)) return true;  // x of the neighbouring rows
     CompSum q;
     for_groups([&](int, int g, int i, int j, int h, int) {
       const float4 b = ld4f(A.b + g), a = apply_A(A.x, g, i, j, h, ld4f(A.x + g));
@@ -1029,8 +1065,9 @@ __global__ void __launch_bounds__(kT, 1) k_cluster_solve(const __grid_constant__
       add4(q, make_float4(d.x * d.x, d.y * d.y, d.z * d.z, d.w * d.w));
     });
     Pair t[1];
-    cluster_sum<1>({q}, &red, &ex, P.nc, rank, uses, t);
+    cluster_sum<1>({q}, &red, &ex, P.nc, me, uses, t);
     if (tid == 0) sc.rTr_true = t[0];
+    return false;
   };
 
   // ---- setup: r0, recenter, b, the warm start's residual, r0.r0
@@ -1044,7 +1081,7 @@ __global__ void __launch_bounds__(kT, 1) k_cluster_solve(const __grid_constant__
     });
     if (A.neu) {
       Pair t[1];
-      cluster_sum<1, WIDE>({CompSum{q.s, q.c}}, &red, &ex, P.nc, rank, uses, t, WIDE ? q.value() : 0.0);
+      cluster_sum<1, WIDE>({CompSum{q.s, q.c}}, &red, &ex, P.nc, me, uses, t, WIDE ? q.value() : 0.0);
       if (tid == 0) sc.mean = mean_of(t[0]);
     }
     __syncthreads();
@@ -1065,7 +1102,7 @@ __global__ void __launch_bounds__(kT, 1) k_cluster_solve(const __grid_constant__
       add4(qr, make_float4(r.x * r.x, r.y * r.y, r.z * r.z, r.w * r.w));
     });
     Pair t[2];
-    cluster_sum<2>({qr, qb}, &red, &ex, P.nc, rank, uses, t);
+    cluster_sum<2>({qr, qb}, &red, &ex, P.nc, me, uses, t);
     if (tid == 0) {
       sc.rTr = sc.rTr0 = t[0];
       sc.bTb = A.keep_b ? t[1] : Pair{0.f, 0.f};
@@ -1086,7 +1123,7 @@ __global__ void __launch_bounds__(kT, 1) k_cluster_solve(const __grid_constant__
     }
   }
 
-  bool first = true;
+  bool first = true, lost = false;
 #pragma unroll 1
   while (true) {
     // ---- V-cycle, z.r, beta, p
@@ -1098,7 +1135,7 @@ __global__ void __launch_bounds__(kT, 1) k_cluster_solve(const __grid_constant__
         add4(q, make_float4(z.x * r.x, z.y * r.y, z.z * r.z, z.w * r.w));
       });
       Pair t[1];
-      cluster_sum<1>({q}, &red, &ex, P.nc, rank, uses, t);
+      cluster_sum<1>({q}, &red, &ex, P.nc, me, uses, t);
       if (tid == 0) {
         // a 16-bit level vector answers the scaled residual
         Pair zTr = t[0];
@@ -1120,7 +1157,6 @@ __global__ void __launch_bounds__(kT, 1) k_cluster_solve(const __grid_constant__
           }
         }
         sc.zTr_old = zTr;
-        if (ex.lost) sc.done = 4;
       }
       __syncthreads();
     }
@@ -1135,8 +1171,9 @@ __global__ void __launch_bounds__(kT, 1) k_cluster_solve(const __grid_constant__
         *reinterpret_cast<float4*>(A.p + g) = z;
       });
       first = false;
-      cluster_barrier();  // p of the neighbouring rows
+      lost = pass_barrier(&ex, me);  // p of the neighbouring rows
     }
+    if (lost) break;
     // ---- A p, alpha, x and r, r.r, the stop test
     {
       CompSum q;
@@ -1146,7 +1183,7 @@ __global__ void __launch_bounds__(kT, 1) k_cluster_solve(const __grid_constant__
         add4(q, make_float4(p.x * a.x, p.y * a.y, p.z * a.z, p.w * a.w));
       });
       Pair t[1];
-      cluster_sum<1>({q}, &red, &ex, P.nc, rank, uses, t);
+      cluster_sum<1>({q}, &red, &ex, P.nc, me, uses, t);
       if (tid == 0) {
         sc.pAp = t[0];
         sc.alpha = quotient(sc.zTr_old, t[0], Pair{A.eps_s, A.eps_c});
@@ -1168,10 +1205,9 @@ __global__ void __launch_bounds__(kT, 1) k_cluster_solve(const __grid_constant__
         add4(qm, r);
       });
       Pair t[2];
-      cluster_sum<2, WIDE>({qr, CompSum{qm.s, qm.c}}, &red, &ex, P.nc, rank, uses, t, WIDE ? qm.value() : 0.0);
+      cluster_sum<2, WIDE>({qr, CompSum{qm.s, qm.c}}, &red, &ex, P.nc, me, uses, t, WIDE ? qm.value() : 0.0);
       if (tid == 0) {
         sc.rTr = t[0];
-        if (ex.lost) sc.done = 4;
         if (A.neu) sc.mean = mean_of(t[1]);
         if (MIXED && t[0].s > 0.f) sc.hscale = scale_of(t[0]);
         if (!isfinite(t[0].s + t[0].c)) {
@@ -1184,8 +1220,8 @@ __global__ void __launch_bounds__(kT, 1) k_cluster_solve(const __grid_constant__
       }
       __syncthreads();
     }
-    if (A.true_every > 0 && !sc.done && (sc.it + 1) % A.true_every == 0) true_residual();
-    if (sc.done) break;
+    if (A.true_every > 0 && !sc.done && (sc.it + 1) % A.true_every == 0) lost = true_residual();
+    if (lost || sc.done) break;
     // ---- recenter, the level-storage copy
     if (A.neu || MIXED) {
       const float mean = sc.mean, hs = sc.hscale;
@@ -1200,8 +1236,10 @@ __global__ void __launch_bounds__(kT, 1) k_cluster_solve(const __grid_constant__
       __syncthreads();
     }
   }
-  if (A.true_every > 0) true_residual();
-  if (rank == 0 && tid == 0) {
+  // behind this barrier the end is agreed; then no CTA leaves while another may still write its shared memory
+  if (!lost) lost = pass_barrier(&ex, me);
+  if (!lost && A.true_every > 0) lost = true_residual() || pass_barrier(&ex, me);
+  if (me.rank == 0 && tid == 0) {
     SolveState* st = A.st;
     st->zTr_old = pair_value(sc.zTr_old);
     st->pAp = pair_value(sc.pAp);
@@ -1215,12 +1253,12 @@ __global__ void __launch_bounds__(kT, 1) k_cluster_solve(const __grid_constant__
     st->mean = sc.mean;
     st->hscale = sc.hscale;
     st->it = sc.it;
-    st->done = ex.lost ? 4 : sc.done;
+    st->done = lost ? 4 : sc.done;
     st->conv_it = sc.conv_it;
     st->ticket = 0u;
     st->it_stop = sc.it;
   }
-  cluster_barrier();  // no CTA leaves while another may still read its shared memory
+  if (lost) leave();
 }
 
 // ---------------------------------------------------------------------------------------------
@@ -1357,6 +1395,7 @@ bool make_plan(const pfm_handle* h, int l0, int esz, bool whole, int max_nc, CPl
   P.bc = bc_of(h);
   P.pre_post = h->cfg.pre_post_smoothing;
   P.bottom = h->cfg.bottom_smoothing;
+  P.wait_ns = (unsigned)h->cluster_wait_us * 1000u;
   if (whole) {
     if ((D == 3 ? h->lv[0].n[2] : h->lv[0].n[1]) % 4 != 0) return false;  // 16-byte groups of cells
     P.lg = std::max(l0 + 1, first_below(kSoloCells));

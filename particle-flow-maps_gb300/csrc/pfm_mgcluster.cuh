@@ -26,6 +26,7 @@ struct CPlan {
   int nc, L, l0, lg;  // CTAs; levels l0 .. lg-1 distributed, lg .. L-1 solo
   int ld, nbase;      // the level whose rows define the shares (the first solo level, else the last), its rows
   int pre_post, bottom;
+  unsigned wait_ns;   // limit of a wait for other CTAs
   BC bc;
   CLev lv[kMaxLevels];
 };

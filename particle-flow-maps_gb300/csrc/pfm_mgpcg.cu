@@ -2440,7 +2440,7 @@ static int solve_result(pfm_handle* h, const SolveState& hs, bool true_res, pfm_
     stats->rTr_true = true_res ? hs.rTr_true : -1.0;
   }
   if (hs.done == 3) return set_error(h, PFM_ERR_NONFINITE, "MGPCG: non-finite residual");
-  if (hs.done == 4) return set_error(h, PFM_ERR_CUDA, "MGPCG: a smoother's tile copy did not arrive");
+  if (hs.done == 4) return set_error(h, PFM_ERR_CUDA, "MGPCG: a kernel's bounded wait gave up");
   if (hs.done != 1) return set_error(h, PFM_ERR_NOT_CONVERGED, "MGPCG: iteration limit reached");
   return PFM_OK;
 }

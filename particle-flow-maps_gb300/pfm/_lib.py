@@ -185,6 +185,7 @@ TUNE_SMOOTH_TMA = 3
 TUNE_CUBE_KERNELS = 4
 TUNE_MIDPOINT_CENTRE = 5
 TUNE_MG_CLUSTER = 6
+TUNE_MG_CLUSTER_WAIT = 7
 # scratch limits of pfm_sort_particles_noalloc (include/pfm.h)
 NOALLOC_MAX_PARTICLES = 1 << 21
 NOALLOC_MAX_CELLS = 1 << 18
