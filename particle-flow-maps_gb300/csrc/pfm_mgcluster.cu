@@ -843,15 +843,14 @@ constexpr int kWarps = kT / 32;
 
 struct ClusterRed {  // in shared memory
   Pair warp[2][kWarps];
+  double part[kWarps * 8];
   Pair slot[2][2][16];  // [buffer][sum][rank]
   uint64_t full[2];     // the ranks' totals of a buffer have arrived
 };
 
 // The sum of r, for its mean: r's own mean was subtracted before, so the terms cancel to some 1e-11 of their
 // magnitudes, and the 1e-15 that pairs lose would be 1e-4 of the mean.  A second compensation per thread and FP64
-// above it keep what the grid-wide solve's FP64 sums keep.  3D only (64^3: with pairs three steps ended on
-// other last bits than the grid-wide solve's in 5 of 6 fields, with this in 2; in 2D they agreed either way), for 12 us
-// per solve of a 64^3 step of 1200.
+// above it keep what the grid-wide solve's FP64 sums keep.
 struct WideSum {
   float s = 0.f, c = 0.f, d = 0.f;
   __device__ __forceinline__ void add(float x) {
@@ -863,53 +862,66 @@ struct WideSum {
   }
   __device__ __forceinline__ double value() const { return (double)s + ((double)c + (double)d); }
 };
+
 __device__ __forceinline__ Pair bits_of(double x) {
   return Pair{__int_as_float(__double2loint(x)), __int_as_float(__double2hiint(x))};
 }
 __device__ __forceinline__ double of_bits(Pair p) {
   return __hiloint2double(__float_as_int(p.c), __float_as_int(p.s));
 }
-template <int WIDTH>
-__device__ __forceinline__ double wide_reduce(double v) {
-#pragma unroll
-  for (int o = WIDTH / 2; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-  return v;
-}
 
-// The cluster's total of N sums, in total[] of the calling CTA's first warp (the others' are
-// undefined).  With WIDE the last of them is the sum of `wide`, as the bits of a double.  A non-finite term gives a non-finite total.  Every CTA sends its total to every CTA with
-// st.async; `uses` numbers the calls (two buffers alternate: a CTA is at most one call ahead).
-template <int N, bool WIDE = false>
+// The cluster's totals of the threads' sums: total[] of those in v by trees of f32 pairs, and *mean of the wide one if
+// there is one, in the calling CTA's first warp (the others' are undefined; the threads from `busy` on
+// hold zero).  A non-finite term gives a non-finite total.  Every CTA sends its totals to every CTA with st.async;
+// `uses` numbers the calls (two buffers alternate: a CTA is at most one call ahead).  The wide sum's tree stops at
+// eight partial sums per warp, which the second warp adds up: an FP64 addition takes 16 cycles of the SM per warp.
+template <int N>
 __device__ __forceinline__ void cluster_sum(const CompSum (&v)[N], ClusterRed* red, Exchange* ex, int nc, Me& me,
-                                            unsigned& uses, Pair (&total)[N], double wide = 0.0) {
+                                            unsigned& uses, Pair (&total)[N], int busy = 0, const WideSum* wide = nullptr,
+                                            double* mean = nullptr) {
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, buf = (int)(uses & 1u);
   const unsigned parity = (uses >> 1) & 1u;
   ++uses;
+  auto push = [&](int n, Pair w) {
+    if (lane < nc && !me.gone)
+      push_async<8>(remote_addr(su32(&red->slot[buf][n][me.rank]), lane), &w, remote_addr(su32(&red->full[buf]), lane));
+  };
 #pragma unroll
   for (int n = 0; n < N; ++n) {
-    Pair w;
-    if (WIDE && n == N - 1) w = bits_of(wide_reduce<32>(wide));
-    else w = pair_reduce<32>(Pair{v[n].s, v[n].c});
+    const Pair w = pair_reduce<32>(Pair{v[n].s, v[n].c});
     if (lane == 0) red->warp[n][wid] = w;
   }
-  __syncthreads();
-  if (wid == 0) {
-    if (lane == 0 && !me.gone) mbar_expect_tx(&red->full[buf], (unsigned)(N * nc * sizeof(Pair)));
-#pragma unroll
-    for (int n = 0; n < N; ++n) {
-      Pair w = red->warp[n][lane % kWarps];
-      if (WIDE && n == N - 1) w = bits_of(wide_reduce<kWarps>(of_bits(w)));
-      else w = pair_reduce<kWarps>(w);
-      if (lane < nc && !me.gone)
-        push_async<8>(remote_addr(su32(&red->slot[buf][n][me.rank]), lane), &w, remote_addr(su32(&red->full[buf]), lane));
+  if (wide) {
+    double w = 0.0;
+    if (wid * 32 < busy) {
+      w = wide->value();
+      w += __shfl_xor_sync(0xffffffffu, w, 16);
+      w += __shfl_xor_sync(0xffffffffu, w, 8);
     }
+    if (lane < 8) red->part[wid * 8 + lane] = w;
+  }
+  __syncthreads();
+  if (wide && wid == 1) {
+    static_assert(kWarps == 16, "four partial sums per lane");
+    const double* q = red->part + lane;
+    double w = (q[0] + q[32]) + (q[64] + q[96]);
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) w += __shfl_xor_sync(0xffffffffu, w, o);
+    push(N, bits_of(w));
+  }
+  if (wid == 0) {
+    if (lane == 0 && !me.gone) mbar_expect_tx(&red->full[buf], (unsigned)((N + (wide ? 1 : 0)) * nc * sizeof(Pair)));
+#pragma unroll
+    for (int n = 0; n < N; ++n) push(n, pair_reduce<kWarps>(red->warp[n][lane % kWarps]));
     wait_rows(ex, &red->full[buf], parity, me);
 #pragma unroll
-    for (int n = 0; n < N; ++n) {
-      Pair w{0.f, 0.f};
-      if ((lane & 15) < nc) w = red->slot[buf][n][lane & 15];
-      if (WIDE && n == N - 1) total[n] = bits_of(wide_reduce<16>(of_bits(w)));
-      else total[n] = pair_reduce<16>(w);
+    for (int n = 0; n < N; ++n)
+      total[n] = pair_reduce<16>((lane & 15) < nc ? red->slot[buf][n][lane & 15] : Pair{0.f, 0.f});
+    if (wide) {
+      double w = (lane & 15) < nc ? of_bits(red->slot[buf][N][lane & 15]) : 0.0;
+#pragma unroll
+      for (int o = 8; o > 0; o >>= 1) w += __shfl_xor_sync(0xffffffffu, w, o);
+      *mean = w;
     }
   }
 }
@@ -1039,13 +1051,6 @@ __global__ void __launch_bounds__(kT, 1) k_cluster_solve(const __grid_constant__
     return make_float4((float)cell_neighbours<D>(v, P.bc, rn, k) * c.x - n[0], m * c.y - n[1], m * c.z - n[2],
                        (float)cell_neighbours<D>(v, P.bc, rn, k + 3) * c.w - n[3]);
   };
-  auto mean_of = [&](Pair t) {
-    if (D == 3) return (float)(of_bits(t) * ((double)A.inv_n_s + (double)A.inv_n_c));
-    const float m = t.s * A.inv_n_s;
-    return m + (fmaf(t.s, A.inv_n_s, -m) + fmaf(t.s, A.inv_n_c, t.c * A.inv_n_s));
-  };
-  constexpr bool WIDE = D == 3;
-  using MeanSum = std::conditional_t<WIDE, WideSum, CompSum>;
   auto scale_of = [&](Pair t) {
     const float m = t.s * A.inv_n_s, mc = fmaf(t.s, A.inv_n_s, -m) + fmaf(t.s, A.inv_n_c, t.c * A.inv_n_s);
     if (!(t.s > 0.f)) return 1.f;
@@ -1072,7 +1077,7 @@ __global__ void __launch_bounds__(kT, 1) k_cluster_solve(const __grid_constant__
 
   // ---- setup: r0, recenter, b, the warm start's residual, r0.r0
   {
-    MeanSum q;
+    WideSum q;
     for_groups([&](int e, int g, int, int, int, int c) {
       const float4 b = ld4f(A.rhs + g);
       put4(rf, v.cr, e, c, b);
@@ -1081,8 +1086,9 @@ __global__ void __launch_bounds__(kT, 1) k_cluster_solve(const __grid_constant__
     });
     if (A.neu) {
       Pair t[1];
-      cluster_sum<1, WIDE>({CompSum{q.s, q.c}}, &red, &ex, P.nc, me, uses, t, WIDE ? q.value() : 0.0);
-      if (tid == 0) sc.mean = mean_of(t[0]);
+      double sum;
+      cluster_sum<1>({CompSum{}}, &red, &ex, P.nc, me, uses, t, T, &q, &sum);
+      if (tid == 0) sc.mean = (float)(sum * A.inv_n);
     }
     __syncthreads();
     const float mean = sc.mean;
@@ -1193,7 +1199,7 @@ __global__ void __launch_bounds__(kT, 1) k_cluster_solve(const __grid_constant__
     {
       const float alpha = sc.alpha;
       CompSum qr;
-      MeanSum qm;
+      WideSum qm;
       for_groups([&](int e, int g, int, int, int, int c) {
         const float4 x = ld4f(A.x + g), p = ld4f(A.p + g), a = ld4f(A.Ap + g);
         float4 r = get4(rf, v.cr, e, c);
@@ -1204,11 +1210,12 @@ __global__ void __launch_bounds__(kT, 1) k_cluster_solve(const __grid_constant__
         add4(qr, make_float4(r.x * r.x, r.y * r.y, r.z * r.z, r.w * r.w));
         add4(qm, r);
       });
-      Pair t[2];
-      cluster_sum<2, WIDE>({qr, CompSum{qm.s, qm.c}}, &red, &ex, P.nc, me, uses, t, WIDE ? qm.value() : 0.0);
+      Pair t[1];
+      double sum;
+      cluster_sum<1>({qr}, &red, &ex, P.nc, me, uses, t, T, &qm, &sum);
       if (tid == 0) {
         sc.rTr = t[0];
-        if (A.neu) sc.mean = mean_of(t[1]);
+        if (A.neu) sc.mean = (float)(sum * A.inv_n);
         if (MIXED && t[0].s > 0.f) sc.hscale = scale_of(t[0]);
         if (!isfinite(t[0].s + t[0].c)) {
           sc.done = 3;
@@ -1474,7 +1481,8 @@ int cluster_solve_launch(pfm_handle* h, const pfm_solve_opts& o, cudaStream_t s)
     };
     split(o.eps, A.eps_s, A.eps_c);
     split(o.tol, A.tol_s, A.tol_c);
-    split(1.0 / (double)h->cells, A.inv_n_s, A.inv_n_c);
+    A.inv_n = 1.0 / (double)h->cells;
+    split(A.inv_n, A.inv_n_s, A.inv_n_c);
     A.tol = o.tol;
     A.tol_mode = o.tol_mode;
     A.max_iters = o.max_iters;

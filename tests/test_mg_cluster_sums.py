@@ -1,0 +1,44 @@
+"""The sums of a solve on a thread-block cluster (csrc/pfm_mgcluster.cu) against the grid-wide kernels' FP64 sums."""
+import pytest
+
+torch = pytest.importorskip("torch")
+pytestmark = pytest.mark.gpu
+
+import pfm  # noqa: E402
+from pfm import _lib  # noqa: E402
+
+
+def _smooth_divergence(res, seed):
+    """The divergence of the f32 gradient of a few Gaussian blobs: its sum is the rounding of its terms."""
+    g = torch.Generator(device="cuda").manual_seed(seed)
+    phi = torch.zeros(res, device="cuda", dtype=torch.float64)
+    for _ in range(6):
+        e = torch.ones([1] * len(res), device="cuda", dtype=torch.float64) * float(torch.randn(1, generator=g, device="cuda"))
+        for a, n in enumerate(res):
+            shape = [1] * len(res)
+            shape[a] = n
+            at = torch.arange(n, device="cuda", dtype=torch.float64) / n
+            e = e * torch.exp(-((at - float(torch.rand(1, generator=g, device="cuda")) * 0.6 - 0.2) / 0.06) ** 2).view(shape)
+        phi += e
+    d = torch.zeros_like(phi)
+    for a, n in enumerate(res):
+        q = (phi.narrow(a, 1, n - 1) - phi.narrow(a, 0, n - 1)).float().double()
+        d.narrow(a, 0, n - 1).add_(q)
+        d.narrow(a, 1, n - 1).sub_(q)
+    return d.float()
+
+
+@pytest.mark.parametrize("res,seed", [((448, 512), 67), ((448, 512), 12), ((512, 512), 48), ((64, 64, 64), 45)])
+def test_mean_of_the_residual(res, seed):
+    """All walls Neumann: the residual's mean is what its own rounding leaves, and an error in it moves the pressure's
+    constant through the singular coarsest level.  After eight iterations the pressure is the grid-wide solve's
+    to the rounding of its FP32 storage, 2^-24 of its norm."""
+    r = _smooth_divergence(res, seed)
+    sc = pfm.Scene(len(res), res, 1.0 / res[1], 0)
+    x = []
+    for cluster in (1, 0):
+        sc.set_tuning(_lib.TUNE_MG_CLUSTER, cluster)
+        x.append(torch.zeros_like(r))
+        sc.mgpcg_solve(r, x[-1], tol=0.0, max_iters=8)
+    a, b = (t.double() for t in x)
+    assert (a - b).norm() <= 2.0 ** -24 * b.norm()
