@@ -120,10 +120,13 @@ __device__ __forceinline__ Pair pair_reduce(Pair v) {
 
 // the stopping rule of k_update_xr / k_true_residual; the relative rules accept an exactly zero
 // residual, so a zero right-hand side (a fluid at rest) ends at the first check
-__device__ __forceinline__ bool converged(double rTr, const SolveState* st, double tol, int tol_mode) {
+// (ref: the r.r or b.b that tol_mode 1 or 2 compares with)
+__device__ __forceinline__ bool converged(double rTr, double ref, double tol, int tol_mode) {
   if (tol_mode == 0) return rTr < tol;
-  const double ref = (tol_mode == 1) ? st->rTr0 : st->bTb;
   return rTr == 0.0 || sqrt(rTr) < tol * sqrt(ref);
+}
+__device__ __forceinline__ bool converged(double rTr, const SolveState* st, double tol, int tol_mode) {
+  return converged(rTr, tol_mode == 1 ? st->rTr0 : st->bTb, tol, tol_mode);
 }
 
 static inline BC bc_of(const pfm_handle* h) {

@@ -941,7 +941,7 @@ struct Scalars {  // in shared memory: broadcast from thread 0 to its CTA, and t
   float alpha, beta, mean, hscale;
   int done, it, conv_it;
   Pair zTr_old, pAp, rTr, rTr0, bTb, rTr_true;
-  Pair stop;  // the sum of squares below which the solve has converged
+  float stop;  // a residual above this cannot meet the rule: `converged` is asked below it
 };
 
 // ---------------------------------------------------------------------------------------------
@@ -969,7 +969,7 @@ __global__ void __launch_bounds__(kT, 1) k_cluster_solve(const __grid_constant__
     mbar_init(&red.full[1], 1);
     fence_mbar_init();
     const Pair none{0.f, 0.f};
-    sc = Scalars{0.f, 0.f, 0.f, 1.f, 0, 0, 0, none, none, none, none, none, none, Pair{A.tol_s, A.tol_c}};
+    sc = Scalars{0.f, 0.f, 0.f, 1.f, 0, 0, 0, none, none, none, none, none, none, (float)(1.0001 * A.tol)};
   }
   pass_barrier(&ex, me);  // every CTA of the cluster runs before the first remote store
   const CLev v = P.lv[0];
@@ -1113,10 +1113,7 @@ __global__ void __launch_bounds__(kT, 1) k_cluster_solve(const __grid_constant__
       sc.rTr = sc.rTr0 = t[0];
       sc.bTb = A.keep_b ? t[1] : Pair{0.f, 0.f};
       sc.hscale = scale_of(t[0]);
-      if (A.tol_mode != 0) {
-        const double s_ = A.tol * sqrt(pair_value(A.tol_mode == 1 ? sc.rTr0 : sc.bTb));
-        sc.stop = to_pair(s_ * s_);
-      }
+      if (A.tol_mode != 0) sc.stop = (float)(1.0001 * A.tol * A.tol * pair_value(A.tol_mode == 1 ? sc.rTr0 : sc.bTb));
     }
     __syncthreads();
     if (MIXED) {
@@ -1220,7 +1217,8 @@ __global__ void __launch_bounds__(kT, 1) k_cluster_solve(const __grid_constant__
         if (!isfinite(t[0].s + t[0].c)) {
           sc.done = 3;
           sc.conv_it = sc.it;
-        } else if ((t[0].s - sc.stop.s) + (t[0].c - sc.stop.c) < 0.f || (A.tol_mode != 0 && t[0].s == 0.f)) {
+        } else if (!(t[0].s > sc.stop) &&
+                   converged(pair_value(t[0]), pair_value(A.tol_mode == 1 ? sc.rTr0 : sc.bTb), A.tol, A.tol_mode)) {
           sc.done = 1;
           sc.conv_it = sc.it;
         }
@@ -1480,7 +1478,6 @@ int cluster_solve_launch(pfm_handle* h, const pfm_solve_opts& o, cudaStream_t s)
       c = (float)(x - (double)s);
     };
     split(o.eps, A.eps_s, A.eps_c);
-    split(o.tol, A.tol_s, A.tol_c);
     A.inv_n = 1.0 / (double)h->cells;
     split(A.inv_n, A.inv_n_s, A.inv_n_c);
     A.tol = o.tol;

@@ -36,7 +36,7 @@ struct CSolve {
   float *x, *p, *Ap, *b;
   SolveState* st;
   double tol, inv_n;
-  float eps_s, eps_c, tol_s, tol_c, inv_n_s, inv_n_c;  // eps, tol and 1 / cells as sums of two floats
+  float eps_s, eps_c, inv_n_s, inv_n_c;  // eps and 1 / cells as sums of two floats
   int tol_mode, max_iters, warm, true_every, keep_b, neu;
   unsigned rf;  // byte offset of the FP32 residual
 };

@@ -42,3 +42,21 @@ def test_mean_of_the_residual(res, seed):
         sc.mgpcg_solve(r, x[-1], tol=0.0, max_iters=8)
     a, b = (t.double() for t in x)
     assert (a - b).norm() <= 2.0 ** -24 * b.norm()
+
+
+# tolerances an f32 cannot hold, beside ordinary ones
+@pytest.mark.parametrize("mode,tol", [(0, 1e-60), (0, 0.0), (0, -1.0), (0, 1e-6), (0, 1e300), (0, float("inf")),
+                                      (0, float("nan")), (1, 1e-60), (1, 0.0), (1, 1e-6), (1, 1e200), (1, float("inf")),
+                                      (2, 1e-5), (2, 1e-40), (2, float("inf"))])
+def test_stopping_rule(mode, tol):
+    """Every tolerance ends a solve where it ends the grid-wide one, for a right-hand side and for a fluid at rest."""
+    res = (64, 48)
+    sc = pfm.Scene(2, res, 1 / 48, 0)
+    g = torch.Generator(device="cuda").manual_seed(3)
+    for r in (torch.randn(res, device="cuda", generator=g), torch.zeros(res, device="cuda")):
+        got = []
+        for cluster in (1, 0):
+            sc.set_tuning(_lib.TUNE_MG_CLUSTER, cluster)
+            info = sc.mgpcg_solve(r, torch.zeros_like(r), tol=tol, tol_mode=mode, max_iters=12)
+            got.append((info.iterations, info.converged, info.status))
+        assert got[0] == got[1]
