@@ -870,14 +870,14 @@ __device__ __forceinline__ double of_bits(Pair p) {
   return __hiloint2double(__float_as_int(p.c), __float_as_int(p.s));
 }
 
-// The cluster's totals of the threads' sums: total[] of those in v by trees of f32 pairs, and *mean of the wide one if
+// The cluster's totals of the threads' sums: total[] of those in v times `unit` by trees of f32 pairs, and *mean of the wide one if
 // there is one, in the calling CTA's first warp (the others' are undefined; the threads from `busy` on
 // hold zero).  A non-finite term gives a non-finite total.  Every CTA sends its totals to every CTA with st.async;
 // `uses` numbers the calls (two buffers alternate: a CTA is at most one call ahead).  The wide sum's tree stops at
 // eight partial sums per warp, which the second warp adds up: an FP64 addition takes 16 cycles of the SM per warp.
 template <int N>
 __device__ __forceinline__ void cluster_sum(const CompSum (&v)[N], ClusterRed* red, Exchange* ex, int nc, Me& me,
-                                            unsigned& uses, Pair (&total)[N], int busy = 0, const WideSum* wide = nullptr,
+                                            unsigned& uses, float unit, Pair (&total)[N], int busy = 0, const WideSum* wide = nullptr,
                                             double* mean = nullptr) {
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, buf = (int)(uses & 1u);
   const unsigned parity = (uses >> 1) & 1u;
@@ -888,7 +888,7 @@ __device__ __forceinline__ void cluster_sum(const CompSum (&v)[N], ClusterRed* r
   };
 #pragma unroll
   for (int n = 0; n < N; ++n) {
-    const Pair w = pair_reduce<32>(Pair{v[n].s, v[n].c});
+    const Pair w = pair_reduce<32>(Pair{v[n].s * unit, v[n].c * unit});
     if (lane == 0) red->warp[n][wid] = w;
   }
   if (wide) {
@@ -938,7 +938,7 @@ __device__ __forceinline__ float quotient(Pair a, Pair b, Pair eps) {
 }
 
 struct Scalars {  // in shared memory: broadcast from thread 0 to its CTA, and thread 0's own
-  float alpha, beta, mean, hscale;
+  float alpha, beta, mean, hscale, unit;
   int done, it, conv_it;
   Pair zTr_old, pAp, rTr, rTr0, bTb, rTr_true;
   float stop;  // a residual above this cannot meet the rule: `converged` is asked below it
@@ -969,7 +969,7 @@ __global__ void __launch_bounds__(kT, 1) k_cluster_solve(const __grid_constant__
     mbar_init(&red.full[1], 1);
     fence_mbar_init();
     const Pair none{0.f, 0.f};
-    sc = Scalars{0.f, 0.f, 0.f, 1.f, 0, 0, 0, none, none, none, none, none, none, (float)(1.0001 * A.tol)};
+    sc = Scalars{0.f, 0.f, 0.f, 1.f, 1.f, 0, 0, 0, none, none, none, none, none, none, 0.f};
   }
   pass_barrier(&ex, me);  // every CTA of the cluster runs before the first remote store
   const CLev v = P.lv[0];
@@ -980,6 +980,10 @@ __global__ void __launch_bounds__(kT, 1) k_cluster_solve(const __grid_constant__
   const S* zl = reinterpret_cast<const S*>(sm + v.z) + v.plane;
   const int sx = v.n1 * v.nk, sy = v.nk;
   unsigned uses = 0;
+  // The sums of products are held in units of 1 / unit: 1, or 2^60 where they could leave f32's range before
+  // the f32 products do (all of them are compared with each other only, and with the tolerance and eps)
+  float unit = 1.f;
+  double back = 1.0;
 
   // f(element of the first pair, global index of the first cell, i, j, h, colour of the even cells)
   auto for_groups = [&](auto&& f) {
@@ -1052,6 +1056,7 @@ __global__ void __launch_bounds__(kT, 1) k_cluster_solve(const __grid_constant__
                        (float)cell_neighbours<D>(v, P.bc, rn, k + 3) * c.w - n[3]);
   };
   auto scale_of = [&](Pair t) {
+    if (unit != 1.f && t.s > 0.f) return (float)(1.0 / sqrt(pair_value(t) * back * A.inv_n));
     const float m = t.s * A.inv_n_s, mc = fmaf(t.s, A.inv_n_s, -m) + fmaf(t.s, A.inv_n_c, t.c * A.inv_n_s);
     if (!(t.s > 0.f)) return 1.f;
     if (!(m > 1e-30f && m < 1e30f)) return (float)(1.0 / sqrt(pair_value(t) * ((double)A.inv_n_s + (double)A.inv_n_c)));
@@ -1070,7 +1075,7 @@ __global__ void __launch_bounds__(kT, 1) k_cluster_solve(const __grid_constant__
       add4(q, make_float4(d.x * d.x, d.y * d.y, d.z * d.z, d.w * d.w));
     });
     Pair t[1];
-    cluster_sum<1>({q}, &red, &ex, P.nc, me, uses, t);
+    cluster_sum<1>({q}, &red, &ex, P.nc, me, uses, unit, t);
     if (tid == 0) sc.rTr_true = t[0];
     return false;
   };
@@ -1087,7 +1092,7 @@ __global__ void __launch_bounds__(kT, 1) k_cluster_solve(const __grid_constant__
     if (A.neu) {
       Pair t[1];
       double sum;
-      cluster_sum<1>({CompSum{}}, &red, &ex, P.nc, me, uses, t, T, &q, &sum);
+      cluster_sum<1>({CompSum{}}, &red, &ex, P.nc, me, uses, unit, t, T, &q, &sum);
       if (tid == 0) sc.mean = (float)(sum * A.inv_n);
     }
     __syncthreads();
@@ -1108,12 +1113,21 @@ __global__ void __launch_bounds__(kT, 1) k_cluster_solve(const __grid_constant__
       add4(qr, make_float4(r.x * r.x, r.y * r.y, r.z * r.z, r.w * r.w));
     });
     Pair t[2];
-    cluster_sum<2>({qr, qb}, &red, &ex, P.nc, me, uses, t);
+#pragma unroll 1
+    for (bool again = true; again;) {
+      cluster_sum<2>({qr, qb}, &red, &ex, P.nc, me, uses, unit, t);
+      if (tid == 0) sc.unit = unit == 1.f && !(t[0].s < 1e25f && t[1].s < 1e25f) ? 0x1p-60f : unit;
+      __syncthreads();
+      again = sc.unit != unit;
+      unit = sc.unit;
+    }
+    back = unit == 1.f ? 1.0 : 0x1p60;
     if (tid == 0) {
       sc.rTr = sc.rTr0 = t[0];
       sc.bTb = A.keep_b ? t[1] : Pair{0.f, 0.f};
       sc.hscale = scale_of(t[0]);
-      if (A.tol_mode != 0) sc.stop = (float)(1.0001 * A.tol * A.tol * pair_value(A.tol_mode == 1 ? sc.rTr0 : sc.bTb));
+      sc.stop = (float)(1.0001 * (A.tol_mode == 0 ? A.tol * unit
+                                                  : A.tol * A.tol * pair_value(A.tol_mode == 1 ? sc.rTr0 : sc.bTb)));
     }
     __syncthreads();
     if (MIXED) {
@@ -1138,7 +1152,7 @@ __global__ void __launch_bounds__(kT, 1) k_cluster_solve(const __grid_constant__
         add4(q, make_float4(z.x * r.x, z.y * r.y, z.z * r.z, z.w * r.w));
       });
       Pair t[1];
-      cluster_sum<1>({q}, &red, &ex, P.nc, me, uses, t);
+      cluster_sum<1>({q}, &red, &ex, P.nc, me, uses, unit, t);
       if (tid == 0) {
         // a 16-bit level vector answers the scaled residual
         Pair zTr = t[0];
@@ -1152,7 +1166,7 @@ __global__ void __launch_bounds__(kT, 1) k_cluster_solve(const __grid_constant__
             sc.conv_it = 0;
           }
         } else {
-          sc.beta = quotient(zTr, sc.zTr_old, Pair{A.eps_s, A.eps_c});
+          sc.beta = quotient(zTr, sc.zTr_old, Pair{A.eps_s * unit, A.eps_c * unit});
           sc.it += 1;
           if (sc.it >= A.max_iters) {
             sc.done = 2;
@@ -1186,10 +1200,10 @@ __global__ void __launch_bounds__(kT, 1) k_cluster_solve(const __grid_constant__
         add4(q, make_float4(p.x * a.x, p.y * a.y, p.z * a.z, p.w * a.w));
       });
       Pair t[1];
-      cluster_sum<1>({q}, &red, &ex, P.nc, me, uses, t);
+      cluster_sum<1>({q}, &red, &ex, P.nc, me, uses, unit, t);
       if (tid == 0) {
         sc.pAp = t[0];
-        sc.alpha = quotient(sc.zTr_old, t[0], Pair{A.eps_s, A.eps_c});
+        sc.alpha = quotient(sc.zTr_old, t[0], Pair{A.eps_s * unit, A.eps_c * unit});
       }
       __syncthreads();
     }
@@ -1209,7 +1223,7 @@ __global__ void __launch_bounds__(kT, 1) k_cluster_solve(const __grid_constant__
       });
       Pair t[1];
       double sum;
-      cluster_sum<1>({qr}, &red, &ex, P.nc, me, uses, t, T, &qm, &sum);
+      cluster_sum<1>({qr}, &red, &ex, P.nc, me, uses, unit, t, T, &qm, &sum);
       if (tid == 0) {
         sc.rTr = t[0];
         if (A.neu) sc.mean = (float)(sum * A.inv_n);
@@ -1218,7 +1232,7 @@ __global__ void __launch_bounds__(kT, 1) k_cluster_solve(const __grid_constant__
           sc.done = 3;
           sc.conv_it = sc.it;
         } else if (!(t[0].s > sc.stop) &&
-                   converged(pair_value(t[0]), pair_value(A.tol_mode == 1 ? sc.rTr0 : sc.bTb), A.tol, A.tol_mode)) {
+                   converged(pair_value(t[0]) * back, pair_value(A.tol_mode == 1 ? sc.rTr0 : sc.bTb) * back, A.tol, A.tol_mode)) {
           sc.done = 1;
           sc.conv_it = sc.it;
         }
@@ -1246,12 +1260,12 @@ __global__ void __launch_bounds__(kT, 1) k_cluster_solve(const __grid_constant__
   if (!lost && A.true_every > 0) lost = true_residual() || pass_barrier(&ex, me);
   if (me.rank == 0 && tid == 0) {
     SolveState* st = A.st;
-    st->zTr_old = pair_value(sc.zTr_old);
-    st->pAp = pair_value(sc.pAp);
-    st->rTr = pair_value(sc.rTr);
-    st->rTr0 = pair_value(sc.rTr0);
-    st->bTb = pair_value(sc.bTb);
-    st->rTr_true = pair_value(sc.rTr_true);
+    st->zTr_old = pair_value(sc.zTr_old) * back;
+    st->pAp = pair_value(sc.pAp) * back;
+    st->rTr = pair_value(sc.rTr) * back;
+    st->rTr0 = pair_value(sc.rTr0) * back;
+    st->bTb = pair_value(sc.bTb) * back;
+    st->rTr_true = pair_value(sc.rTr_true) * back;
     st->sum = 0.0;
     st->alpha = sc.alpha;
     st->beta = sc.beta;

@@ -60,3 +60,24 @@ def test_stopping_rule(mode, tol):
             info = sc.mgpcg_solve(r, torch.zeros_like(r), tol=tol, tol_mode=mode, max_iters=12)
             got.append((info.iterations, info.converged, info.status))
         assert got[0] == got[1]
+
+
+@pytest.mark.parametrize("precision", ["fp32", "fp16"])
+@pytest.mark.parametrize("res", [(512, 512), (64, 64, 64)])
+def test_large_residuals(res, precision):
+    """A right-hand side whose products are f32 numbers and whose sum of squares is not: the solve is that of the
+    same numbers a power of two smaller.  Beside eps = 1e-12 and the FP16 scale (one rounding), every operation
+    scales exactly; each of the few iterations may round alpha and beta otherwise, 2^-24 of the pressure each."""
+    g = torch.Generator(device="cuda").manual_seed(7)
+    r = torch.randn(res, device="cuda", generator=g)
+    sc = pfm.Scene(len(res), res, 1.0 / res[1], 0)
+    kw = dict(tol=1e-5, tol_mode=2, max_iters=40, precision=precision, true_residual_every=3)
+    a, b = torch.zeros_like(r), torch.zeros_like(r)
+    small = sc.mgpcg_solve(r, a, **kw)
+    f = 2.0 ** 56
+    assert float((r.double() * f).square().sum()) > 3.5e38 > float((r * f).square().max())
+    large = sc.mgpcg_solve(r * f, b, **kw)
+    assert small.converged and (small.iterations, small.converged) == (large.iterations, large.converged)
+    assert (a.double() - b.double() / f).norm() <= 2.0 ** -20 * a.double().norm()
+    for x, y in ((small.rTr0, large.rTr0), (small.bTb, large.bTb)):
+        assert abs(x - y / f / f) <= 1e-12 * x
