@@ -125,38 +125,42 @@ __device__ bool grid_sum2(double v0, double v1, double* partials, unsigned* tick
   return true;
 }
 
-// The same for compensated f32 sums, by trees of f32 pairs (48 bits): in FP64, at one warp instruction per 16 cycles and SM, the two trees of
-// 64 resident warps took some 6000 cycles per sum.
-__device__ __forceinline__ bool grid_sum(const CompSum& v, double* partials, unsigned* ticket, double* total,
-                                         unsigned bid, unsigned nb) {
-  __shared__ Pair ws[32];
-  __shared__ bool last;
-  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = blockDim.x >> 5;
-  const Pair w = pair_reduce<32>(Pair{v.s, v.c});
-  if (lane == 0) ws[wid] = w;
+// The same with fewer FP64 instructions, each of which takes 16 cycles of the SM per warp: one warp adds up the
+// block's values, eight per lane, and reduces those (12 warp additions where the warps' trees take 44).
+__device__ __forceinline__ double block_sum64(double v) {
+  __shared__ double ws[kReduceThreads];
+  const int lane = threadIdx.x & 31;
+  static_assert(kReduceThreads == 256, "eight values per lane");
+  ws[threadIdx.x] = v;
   __syncthreads();
-  if (wid == 0) {
-    const Pair b = pair_reduce<32>(lane < nw ? ws[lane] : Pair{0.f, 0.f});
-    if (lane == 0) {
-      partials[bid] = pair_value(b);
-      __threadfence();
-      last = atomicAdd(ticket, 1u) == nb - 1;
-    }
+  if (threadIdx.x < 32) {
+    v = ((ws[lane] + ws[lane + 32]) + (ws[lane + 64] + ws[lane + 96])) +
+        ((ws[lane + 128] + ws[lane + 160]) + (ws[lane + 192] + ws[lane + 224]));
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+  }
+  __syncthreads();
+  return v;  // in the first warp
+}
+
+__device__ __forceinline__ bool grid_sum64(double v, double* partials, unsigned* ticket, double* total, unsigned bid,
+                                           unsigned nb) {
+  __shared__ bool last;
+  v = block_sum64(v);
+  if (threadIdx.x == 0) {
+    partials[bid] = v;
+    __threadfence();
+    last = atomicAdd(ticket, 1u) == nb - 1;
   }
   __syncthreads();
   if (!last) return false;
   __threadfence();
-  Pair s{0.f, 0.f};
-  for (int b = threadIdx.x; b < (int)nb; b += blockDim.x) s = pair_add(s, to_pair(((volatile double*)partials)[b]));
-  s = pair_reduce<32>(s);
-  if (lane == 0) ws[wid] = s;
-  __syncthreads();
-  if (wid == 0) {
-    s = pair_reduce<32>(lane < nw ? ws[lane] : Pair{0.f, 0.f});
-    if (lane == 0) {
-      *total = pair_value(s);
-      *ticket = 0u;
-    }
+  double s = 0.0;
+  for (int b = threadIdx.x; b < (int)nb; b += blockDim.x) s += ((volatile double*)partials)[b];
+  s = block_sum64(s);
+  if (threadIdx.x == 0) {
+    *total = s;
+    *ticket = 0u;
   }
   __syncthreads();
   return true;
@@ -1269,7 +1273,7 @@ __device__ __forceinline__ void dot_blk(const SA* __restrict__ a, const float* _
   const double us = (f64 && sizeof(SA) == 2) ? 1.0 / (double)st->hscale : 1.0;
   double total;
   if (RUNS) {
-    if (!grid_sum(acc, rb.partials, &st->ticket, &total, bid, nb)) return;
+    if (!grid_sum64(acc.value(), rb.partials, &st->ticket, &total, bid, nb)) return;
     total *= us;
   } else if (!grid_sum(acc.value() * us, rb.partials, &st->ticket, &total, bid, nb)) {
     return;
@@ -1442,7 +1446,7 @@ __device__ __forceinline__ void Ap_dot_blk(const float* __restrict__ p, float* _
     }
   }
   double total;
-  if (RUNS ? !grid_sum(acc, rb.partials, &st->ticket, &total, bid, nb)
+  if (RUNS ? !grid_sum64(acc.value(), rb.partials, &st->ticket, &total, bid, nb)
            : !grid_sum(f64 ? acc.value() : (double)acc.s, rb.partials, &st->ticket, &total, bid, nb))
     return;
   if (threadIdx.x == 0) {
@@ -1737,7 +1741,7 @@ __device__ __forceinline__ void true_residual_blk(const float* __restrict__ b, c
     }
   }
   double total;
-  if (RUNS ? !grid_sum(acc, rb.partials, &st->ticket, &total, bid, nb)
+  if (RUNS ? !grid_sum64(acc.value(), rb.partials, &st->ticket, &total, bid, nb)
            : !grid_sum(acc.value(), rb.partials, &st->ticket, &total, bid, nb))
     return;
   if (threadIdx.x == 0) st->rTr_true = total;

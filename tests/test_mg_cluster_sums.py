@@ -1,4 +1,4 @@
-"""The sums of a solve on a thread-block cluster (csrc/pfm_mgcluster.cu) against the grid-wide kernels' FP64 sums."""
+"""The sums of a pressure solve, on a thread-block cluster (csrc/pfm_mgcluster.cu) and grid-wide (csrc/pfm_mgpcg.cu)."""
 import pytest
 
 torch = pytest.importorskip("torch")
@@ -63,14 +63,15 @@ def test_stopping_rule(mode, tol):
 
 
 @pytest.mark.parametrize("precision", ["fp32", "fp16"])
-@pytest.mark.parametrize("res", [(512, 512), (64, 64, 64)])
-def test_large_residuals(res, precision):
+@pytest.mark.parametrize("res,cluster", [((512, 512), 1), ((64, 64, 64), 1), ((64, 64, 64), 0), ((512, 512), 0)])
+def test_large_residuals(res, cluster, precision):
     """A right-hand side whose products are f32 numbers and whose sum of squares is not: the solve is that of the
     same numbers a power of two smaller.  Beside eps = 1e-12 and the FP16 scale (one rounding), every operation
     scales exactly; each of the few iterations may round alpha and beta otherwise, 2^-24 of the pressure each."""
     g = torch.Generator(device="cuda").manual_seed(7)
     r = torch.randn(res, device="cuda", generator=g)
     sc = pfm.Scene(len(res), res, 1.0 / res[1], 0)
+    sc.set_tuning(_lib.TUNE_MG_CLUSTER, cluster)
     kw = dict(tol=1e-5, tol_mode=2, max_iters=40, precision=precision, true_residual_every=3)
     a, b = torch.zeros_like(r), torch.zeros_like(r)
     small = sc.mgpcg_solve(r, a, **kw)
