@@ -677,6 +677,8 @@ struct CompSum {
     s = t;
   }
   __device__ __forceinline__ double value() const { return (double)s + (double)c; }
+  // in f32; infinite where the plain sum is (the compensation of an infinite sum is NaN)
+  __device__ __forceinline__ float value32() const { return isfinite(s) ? s + c : s; }
 };
 
 }  // namespace pfm

@@ -726,7 +726,7 @@ __global__ void __launch_bounds__(kWgThreads) k_conv3_wgrad(const __grid_constan
         }
       if ((lane & 7) == 0)
 #pragma unroll
-        for (int q = 0; q < 8; ++q) p.bias[((size_t)blockIdx.x * 16 + (t >> 3)) * 8 + q] = acc[q].s + acc[q].c;
+        for (int q = 0; q < 8; ++q) p.bias[((size_t)blockIdx.x * 16 + (t >> 3)) * 8 + q] = acc[q].value32();
     } else {
       while (f < moves && ok) move();
     }
@@ -775,7 +775,7 @@ __global__ void __launch_bounds__(32 * kWrWarps) k_wgrad_reduce(const ConvWgradP
       v.add(hi);
       v.c += lo;
     }
-    if (l == 0) db[c] = v.s + v.c;
+    if (l == 0) db[c] = v.value32();
     return;
   }
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, warps = blockDim.x >> 5;
@@ -822,7 +822,7 @@ __global__ void __launch_bounds__(32 * kWrWarps) k_wgrad_reduce(const ConvWgradP
       v.add(sh[k][lane >> 2][2 * (lane & 3)]);
       v.c += sh[k][lane >> 2][2 * (lane & 3) + 1];
     }
-    if (r < 3 * cdy && cr < cout) dw[((size_t)cr * cin + ci) * 27 + a * 9 + (2 - sr) * 3 + c] = v.s + v.c;
+    if (r < 3 * cdy && cr < cout) dw[((size_t)cr * cin + ci) * 27 + a * 9 + (2 - sr) * 3 + c] = v.value32();
   }
 }
 
@@ -992,7 +992,7 @@ __global__ void __launch_bounds__(32) k_sum_parts(const float* __restrict__ part
     s.add(hi);
     s.c += lo;
   }
-  if (threadIdx.x == 0) out[blockIdx.x] = s.s + s.c;
+  if (threadIdx.x == 0) out[blockIdx.x] = s.value32();
 }
 
 // Reads of kLossAhead elements per thread are in flight (one at a time: 45 us for 7.1M elements, 14 now; 8.0 and 4.1 for

@@ -40,3 +40,33 @@ def test_small_terms_beside_large_ones(cdy, dims):
     want = dy.double().sum((1, 2, 3)).reshape(-1)
     _, db = _gradients(dims, 16, cdy, dy)
     assert ((db.double() - want).abs() <= 40 * 2.0 ** -24 * want).all(), ((db.double() - want) / want).abs().max()
+
+
+@pytest.mark.parametrize("cdy", [16, 24])
+def test_infinite_sums(cdy):
+    """Gradients that overflow come out as the infinities of a plain f32 sum, in db (both of its paths) and in dW: an
+    infinite term in channel 0, a sum beyond f32 in channel 1; the other channels keep their sums."""
+    dims = (12, 40, 24)
+    V = dims[0] * dims[1] * dims[2]
+    dy = torch.zeros((cdy // 8, *dims, 8), dtype=torch.bfloat16, device="cuda")
+    dy[0, 5, 7, 9, 0] = float("-inf")
+    dy[0, ..., 1] = 3e38
+    dy[0, ..., 2] = 0.5
+    dw, db = _gradients(dims, 16, cdy, dy)
+    assert db[0] == float("-inf") and db[1] == float("inf") and db[2] == 0.5 * V
+    assert (dw[1:] == 0).all()
+    # dW: the sum of 2 x 3e38 over the grid's inner voxels
+    lib = _lib.load()
+    p = lambda t: ctypes.c_void_p(t.data_ptr())  # noqa: E731
+    x = torch.full((2, *dims, 8), 2.0, dtype=torch.bfloat16, device="cuda")
+    dy[0, 5, 7, 9, 0] = 0
+    err = torch.zeros(1, dtype=torch.int32, device="cuda")
+    a = _lib.Conv3WgradArgs(*dims, p(x), 16, None, 0, p(dy), cdy, cdy, p(dw), None, 0, p(err))
+    nb = ctypes.c_size_t()
+    assert lib.pfm_nn_wgrad_workspace(ctypes.byref(a), ctypes.byref(nb)) == 0
+    part = torch.empty(nb.value // 4, device="cuda")
+    a.partial, a.partial_bytes = p(part), nb.value
+    assert lib.pfm_nn_conv3_wgrad(ctypes.byref(a), None) == 0
+    torch.cuda.synchronize()
+    assert int(err.item()) == 0
+    assert (dw[1] == float("inf")).all() and (dw[0] == 0).all() and torch.isfinite(dw[2]).all()
