@@ -44,11 +44,11 @@ struct CSolve {
 // Whether a solve of this handle and these options runs as one cluster launch, and that launch: from
 // the right-hand side in r_0 (and x, warm-started) of the workspace to x and the solve state.
 bool cluster_solve_fits(const pfm_handle* h, const pfm_solve_opts& o);
-int cluster_solve_launch(pfm_handle* h, const pfm_solve_opts& o, cudaStream_t s);
+[[nodiscard]] int cluster_solve_launch(pfm_handle* h, const pfm_solve_opts& o, cudaStream_t s);
 
 // The first level (at least 1) from which a V-cycle runs as one cluster launch, or h->L; the launch.
 int cluster_tail_level(const pfm_handle* h, int precision);
-int cluster_tail_launch(pfm_handle* h, int precision, int l0, void* z, const void* r, const SolveState* st,
-                        cudaStream_t s);
+[[nodiscard]] int cluster_tail_launch(pfm_handle* h, int precision, int l0, void* z, const void* r,
+                                      const SolveState* st, cudaStream_t s);
 
 }  // namespace pfm

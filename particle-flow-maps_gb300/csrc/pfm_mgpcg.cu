@@ -2170,14 +2170,16 @@ int set_tail_cells(pfm_handle* h, int cells) {
 // apply_preconditioner (3D/mgpcg.py:182-200) with level storage S
 // The levels' z start at zero: each level's zeroing is folded into its first half-sweep (which
 // then reads no neighbours), or launched on its own where the level's first use is not a sweep
-// (no pre-smoothing); the updates are the same, two to four launches fewer per V-cycle.
+// (no pre-smoothing); the updates are the same, two to four launches fewer per V-cycle.  The status is that of
+// the cluster launch, which can fail where ordinary launches do not.
 template <int D, typename S>
-static void vcycle(pfm_handle* h, const SolveState* st, cudaStream_t s) {
+[[nodiscard]] static int vcycle(pfm_handle* h, const SolveState* st, cudaStream_t s) {
   const int L = h->L;
   const BC bc = bc_of(h);
   const int precision = sizeof(S) == 4 ? 0 : (std::is_same<S, __half>::value ? 1 : 2);
   const int lc = cluster_tail_level(h, precision);  // from here on one cluster launch, where the level fits
   const int l0 = std::min(lc, tail_level(h));
+  int rc = PFM_OK;
   bool zero_first[kMaxLevels] = {};
   auto flush = [&](int l) {  // a use of z_l other than a half-sweep: zero it now if still due
     if (zero_first[l]) {
@@ -2204,7 +2206,7 @@ static void vcycle(pfm_handle* h, const SolveState* st, cudaStream_t s) {
   }
   if (lc < L) {
     zero_first[lc] = false;  // the cluster writes all of z_lc
-    cluster_tail_launch(h, precision, lc, level_z<S>(h, lc), level_r<S>(h, lc), st, s);
+    rc = cluster_tail_launch(h, precision, lc, level_z<S>(h, lc), level_r<S>(h, lc), st, s);
   } else if (l0 < L) {
     TailPlan T{};
     T.l0 = l0;
@@ -2242,6 +2244,7 @@ static void vcycle(pfm_handle* h, const SolveState* st, cudaStream_t s) {
       smooth_launch<D, S>(h, l, 0, st, s);
     }
   }
+  return rc;
 }
 
 static bool all_neumann(const pfm_handle* h) {
@@ -2290,6 +2293,7 @@ static int append_solve_loop(GraphCursor& gc, K& k) {
   const uint64_t b0 = h->launches;
   gc.capture_body(body, [&](cudaStream_t q) { k.body(q, cond); });
   const int nodes = (int)(h->launches - b0);
+  if (!gc.rc) gc.rc = k.rc;
   if (!gc.rc) k.finish(gc.seg());
   return nodes;
 }
@@ -2321,6 +2325,7 @@ struct SolveKernels {
   S *z0, *rh;
   Lvl L0;
   BC bc;
+  int rc = PFM_OK;  // of the launches of setup and body
 
   SolveKernels(pfm_handle* hh, const pfm_solve_opts& oo) : h(hh), o(oo) {
     mixed = sizeof(S) == 2;
@@ -2412,14 +2417,14 @@ struct SolveKernels {
     launch_dot<float>(h, q, r0, r0, n, rb, (int)RED_RTR0, o.eps, inv_n, mi, f64);
     // the scaled level-storage copy of r0, once r0.r0 (and so the scale) is known
     if (mixed) launch(h, k_to_storage<S>, stream_blocks(n), 256, 0, q, rh, (const float*)r0, n, (const SolveState*)st);
-    vcycle<D, S>(h, st, q);
+    rc = vcycle<D, S>(h, st, q);
     update_p(q);
     launch_dot<S>(h, q, z0, r0, n, rb, (int)RED_ZTR_INIT, o.eps, inv_n, mi, f64);
     first_half(q);
   }
   void body(cudaStream_t q, cudaGraphConditionalHandle cond) {
     recenter(q, true, fuse_mean);
-    vcycle<D, S>(h, st, q);
+    if (const int e = vcycle<D, S>(h, st, q)) rc = e;
     launch_dot<S>(h, q, z0, r0, n, rb, (int)RED_ZTR, o.eps, inv_n, mi, f64);
     update_p(q);
     first_half(q);
@@ -2476,6 +2481,7 @@ static int solve_impl(pfm_handle* h, const pfm_solve_opts& o, pfm_solve_stats* s
     h->g_setup = h->g_loop = nullptr;
     h->g_valid = 0;
     int rc = capture(h, [&](cudaStream_t q) { K.setup(q); }, &h->g_setup, &h->g_setup_nodes);
+    if (!rc) rc = K.rc;
     if (rc) return rc;
     cudaGraph_t top = nullptr;
     rc = check_cuda(h, cudaGraphCreate(&top, 0), "graph create");
@@ -2694,6 +2700,7 @@ int append_poisson_pre(GraphCursor& gc, float* const* u, float* p_io, const pfm_
   dispatch_solve(D, o.precision, [&](auto dd, auto ss) {
     SolveKernels<decltype(dd)::value, decltype(ss)> K(h, o);
     K.setup(gc.seg());
+    if (!gc.rc) gc.rc = K.rc;
   });
   return gc.rc;
 }
