@@ -124,6 +124,9 @@ const char* pfm_last_error(const pfm_handle* h);
 const char* pfm_status_string(int status);
 /* Number of MGPCG levels the handle uses. */
 int pfm_mg_levels(const pfm_handle* h, int* levels);
+/* Whether a solve with these options (NULL: the defaults) runs as one thread-block cluster launch, on which the
+ * tunables of the grid-wide kernels do not act. */
+int pfm_mg_on_cluster(const pfm_handle* h, const pfm_solve_opts* opts, int* on_cluster);
 /* Number of kernels launched through this handle since pfm_create (bookkeeping for benchmarks). */
 int pfm_launch_count(const pfm_handle* h, uint64_t* launches);
 /* FP32 roofline denominator: times `reps` launches of an FMA-throughput kernel (8 independent

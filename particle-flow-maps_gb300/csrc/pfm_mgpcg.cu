@@ -2522,9 +2522,11 @@ static int solve_impl(pfm_handle* h, const pfm_solve_opts& o, pfm_solve_stats* s
   return solve_result(h, *hs, K.true_res, stats);
 }
 
+constexpr pfm_solve_opts kDefaultOpts{400, 1e-12, 1e-12, 0, 4, 0, 0, 0, 0};
+
 template <int D>
 static int solve_dispatch(pfm_handle* h, const pfm_solve_opts* opts, pfm_solve_stats* stats, cudaStream_t s) {
-  pfm_solve_opts o{400, 1e-12, 1e-12, 0, 4, 0, 0, 0, 0};
+  pfm_solve_opts o = kDefaultOpts;
   if (opts) o = *opts;
   if (o.check_every < 1) o.check_every = 1;
   if (o.tol_mode < 0 || o.tol_mode > 2) return set_error(h, PFM_ERR_ARG, "MGPCG: tol_mode must be 0, 1 or 2");
@@ -3092,6 +3094,14 @@ int pfm2_poisson(pfm_handle* h, float* u_x, float* u_y, float* p_out, const pfm_
   if (!u_x || !u_y) return set_error(h, PFM_ERR_NULL, "pfm2_poisson: null velocity");
   float* u[2] = {u_x, u_y};
   return poisson_impl<2>(h, u, p_out, opts, stats, (cudaStream_t)stream);
+}
+
+int pfm_mg_on_cluster(const pfm_handle* h, const pfm_solve_opts* opts, int* on_cluster) {
+  if (!h || !on_cluster) return PFM_ERR_NULL;
+  const pfm_solve_opts& o = opts ? *opts : kDefaultOpts;
+  if (o.precision < 0 || o.precision > 2) return PFM_ERR_ARG;
+  *on_cluster = cluster_solve_fits(h, o) ? 1 : 0;
+  return PFM_OK;
 }
 
 int pfm_mgpcg_solve(pfm_handle* h, const float* r, float k, float* x_out, const pfm_solve_opts* opts,

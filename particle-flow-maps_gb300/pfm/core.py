@@ -420,6 +420,15 @@ class Scene:
                          allow=(_lib.PFM_ERR_NOT_CONVERGED,))
         return SolveInfo(s, st)
 
+    def solve_on_cluster(self, max_iters=400, tol=1e-12, tol_mode=0, check_every=4, precision=0, warm_start=False,
+                         true_residual_every=0, true_residual_replace=False):
+        """Whether a solve with these options runs as one thread-block cluster launch."""
+        o = self._opts(max_iters, tol, tol_mode, check_every, precision=precision, warm_start=warm_start,
+                       true_residual_every=true_residual_every, true_residual_replace=true_residual_replace)
+        v = ctypes.c_int()
+        self._check(self.lib.pfm_mg_on_cluster(self.h, ctypes.byref(o), ctypes.byref(v)))
+        return bool(v.value)
+
     def _cells(self, t, name):
         self._dev(t, name)
         if tuple(t.shape) != self.cell_shape:

@@ -6,9 +6,12 @@ simulation; it is done once per scene size, before the step or batch graphs are 
   * ``mg_tail_cells``: the MGPCG levels with at most this many cells run the rest of the V-cycle
     in one thread block (fewer launches, one SM) instead of grid-wide kernels; timed on a solve of
     the scene's current divergence (into a scratch pressure);
-  * ``p2g2_column`` (2D): kept for callers; the P2G picks its faces per thread by size;
   * ``smooth_tma`` (3D, 16-bit MGPCG levels): smoothing from tiles the TMA stages in shared memory
-    (1) or from global memory (0); timed on the same solve.
+    (1) or from global memory (0); timed on the same solve;
+  * ``p2g2_column`` (2D): kept for callers; the P2G picks its faces per thread by size.
+
+A knob that acts on nothing in the scene keeps its value and is not timed: the column, and the solver's where
+the whole solve is one thread-block cluster launch.
 """
 import statistics
 
@@ -19,7 +22,6 @@ from . import _lib
 __all__ = ["autotune", "apply"]
 
 TAILS = (0, 256, 1024, 4096, 16384)
-COLUMNS = (2, 4, 8, 16, 32)
 
 
 def _time(fn, reps):
@@ -35,41 +37,36 @@ def _time(fn, reps):
     return statistics.median(times)
 
 
-def autotune(sim, reps=3, tails=TAILS, columns=COLUMNS):
-    """Tunes ``sim.scene`` (a Sim2D / Sim3D) in place; returns {key: (chosen value, {value: ms})}."""
+def autotune(sim, reps=3, tails=TAILS, columns=()):
+    """Tunes ``sim.scene`` (a Sim2D / Sim3D) in place; returns {key: (chosen value, {value: ms})}, without times for a
+    knob that acts on nothing.  ``columns`` is accepted for callers that pass it."""
     sc = sim.scene
     out = {}
     r = torch.empty(sc.cell_shape, device=sc.device)
     sc.divergence(sim.u, r)
     x = torch.zeros_like(r)
     opts = {k: v for k, v in sim.poisson_opts.items() if k not in ("warm_start", "raise_on_limit")}
+    grid_wide = not sc.solve_on_cluster(**opts)
     times = {}
-    for t in tails:
+    for t in tails if grid_wide else ():
         try:
             sc.set_tuning(_lib.TUNE_MG_TAIL_CELLS, t)
         except _lib.PfmError:  # the tail levels would not fit in shared memory
             continue
         times[t] = _time(lambda: sc.mgpcg_solve(r, x, **opts), reps)
-    best = min(times, key=times.get)
+    best = min(times, key=times.get) if times else sc.get_tuning(_lib.TUNE_MG_TAIL_CELLS)
     sc.set_tuning(_lib.TUNE_MG_TAIL_CELLS, best)
     out["mg_tail_cells"] = (best, times)
     if sc.dim == 3 and opts.get("precision", 0) in (1, 2):
         times = {}
-        for v in (0, 1):
+        for v in (0, 1) if grid_wide else ():
             sc.set_tuning(_lib.TUNE_SMOOTH_TMA, v)
             times[v] = _time(lambda: sc.mgpcg_solve(r, x, **opts), reps)
-        best = min(times, key=times.get)
+        best = min(times, key=times.get) if times else sc.get_tuning(_lib.TUNE_SMOOTH_TMA)
         sc.set_tuning(_lib.TUNE_SMOOTH_TMA, best)
         out["smooth_tma"] = (best, times)
     if sc.dim == 2:
-        times = {}
-        for k in columns:
-            sc.set_tuning(_lib.TUNE_P2G2_COLUMN, k)
-            times[k] = _time(lambda: sc.p2g2(sim.imp, sim.pos, sim.C, sim.psi, sim.u_mid, sim.w,
-                                              psi_out=sim.psi_grid), reps)
-        best = min(times, key=times.get)
-        sc.set_tuning(_lib.TUNE_P2G2_COLUMN, best)
-        out["p2g2_column"] = (best, times)
+        out["p2g2_column"] = (sc.get_tuning(_lib.TUNE_P2G2_COLUMN), {})
     return out
 
 
