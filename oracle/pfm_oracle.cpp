@@ -367,11 +367,12 @@ struct MG {
         }
   }
 
-  void prolongate(int l) {  // mgpcg.py:160-163
+  void prolongate(int l) {  // mgpcg.py:160-163; nothing is added from behind the coarse level's end
     R* zl = z[l].data();
     const R* zc = z[l + 1].data();
     for_cells(l, [&](int i, int j, int k) {
-      zl[idx(l, i, j, k)] += zc[idx(l + 1, i / 2, j / 2, dim == 3 ? k / 2 : 0)];
+      const size_t c = (size_t)idx(l + 1, i / 2, j / 2, dim == 3 ? k / 2 : 0);
+      if (c < z[l + 1].size()) zl[idx(l, i, j, k)] += zc[c];
     }, true);
   }
 

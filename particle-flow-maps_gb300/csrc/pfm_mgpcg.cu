@@ -1053,7 +1053,8 @@ __global__ void __launch_bounds__(256) k_restrict(const S* __restrict__ zf, cons
   restrict_blk<D, S>(zf, rf, Lf, rc, Lc, bc, st, blockIdx.x);
 }
 
-// prolongate(l): z_l[I] += z_{l+1}[I//2]
+// prolongate(l): z_l[I] += z_{l+1}[I//2].  Over a first axis of odd length the last plane lies over no coarse one:
+// what would be read behind the level's end is zero (it held whatever the workspace held, NaN at worst).
 template <int D, typename S>
 __device__ __forceinline__ void prolong_blk(S* __restrict__ zf, const Lvl& Lf, const S* __restrict__ zc,
                                             const Lvl& Lc, const SolveState* st, unsigned bid) {
@@ -1064,7 +1065,7 @@ __device__ __forceinline__ void prolong_blk(S* __restrict__ zf, const Lvl& Lf, c
   decode(Lf, e, i, j, k);
   int64_t ce = (D == 3) ? ((int64_t)(i >> 1) * Lc.n1 + (j >> 1)) * Lc.n2 + (k >> 1)
                         : (int64_t)(i >> 1) * Lc.n1 + (j >> 1);
-  stv(zf + e, ldv(zf + e) + ldv(zc + ce));
+  if (ce < Lc.count) stv(zf + e, ldv(zf + e) + ldv(zc + ce));
 }
 
 template <int D, typename S>
@@ -1099,6 +1100,7 @@ __device__ __forceinline__ void prolong8_blk(S* __restrict__ zf, const Lvl& Lf, 
   const int i = (int)i_, j = (int)(row - i_ * (unsigned)Lf.n1);
   const int64_t c0 = ((int64_t)i * Lf.n1 + j) * Lf.n2 + k0;
   const int64_t cc = ((int64_t)(i >> 1) * Lc.n1 + (j >> 1)) * Lc.n2 + (k0 >> 1);
+  if (cc >= Lc.count) return;
   float a[8], out[8], b[4];
   ld8(zf + c0, a);
   ld4(zc + cc, b);
@@ -1989,7 +1991,7 @@ __device__ __forceinline__ void tail_blk(S* __restrict__ zg, const S* __restrict
       decode(Lf, e, i, j, k);
       int64_t ce = (D == 3) ? ((int64_t)(i >> 1) * Lc.n1 + (j >> 1)) * Lc.n2 + (k >> 1)
                             : (int64_t)(i >> 1) * Lc.n1 + (j >> 1);
-      z[e] += zc[ce];
+      if (ce < Lc.count) z[e] += zc[ce];
     }
     __syncthreads();
     tail_sweeps<D>(z, r, Lf, bc, pre_post, 1);
