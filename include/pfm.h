@@ -67,7 +67,9 @@ typedef struct pfm_handle pfm_handle;
  * precision 0 is the reference's FP32 solve.  precision 1 / 2 is the mixed form: the multigrid
  * levels (the V-cycle's z and r on every level) are stored in FP16 / BF16 and smoothed,
  * restricted and prolonged with FP32 arithmetic; the PCG vectors x, r, p, Ap stay FP32; inner
- * products and norms are compensated FP32 sums per thread combined in FP64.
+ * products and norms are compensated FP32 sums per thread combined in FP64.  In a solve on one
+ * thread-block cluster (PFM_TUNE_MG_CLUSTER), of any precision, they are compensated per thread and
+ * combined in pairs of FP32 (48 bits), but for the residual's mean, which is combined in FP64.
  * warm_start 1 starts from the caller's current pressure (p_out of pfm3/pfm2_poisson, x_out of
  * pfm_mgpcg_solve) instead of zero; warm_start 2 starts from the linear extrapolation
  * 2 p - p_before of that pressure and what the same buffer held at the start of its previous solve
@@ -116,7 +118,9 @@ typedef struct pfm_solve_stats {
  * index with 32-bit integers. */
 int pfm_create(const pfm_config* cfg, pfm_handle** out);
 int pfm_destroy(pfm_handle* h);
-/* Bytes of device scratch the handle needs (sort buffers, P2G payload, MGPCG hierarchy). */
+/* Bytes of device scratch the handle needs: sort buffers, P2G payload and (3D) tile sums of 71 bytes
+ * per cell, MGPCG hierarchy, and on 3D grids from 64^3 cells up that are no cube of 64, 128, 256 or 512 at
+ * most one padded copy of a velocity field, two with particles, of 12 to 48 bytes per cell each. */
 int pfm_workspace_size(const pfm_handle* h, size_t* bytes);
 /* Binds caller-allocated device scratch (>= pfm_workspace_size bytes, 256-byte aligned). */
 int pfm_set_workspace(pfm_handle* h, void* dptr, size_t bytes);
@@ -191,7 +195,10 @@ int pfm3_rk4_T_forward(pfm_handle* h, float* pos, float* T, const float* u_x, co
 /* Midpoint velocity (3D/run_3D.py:779-788 before the projection): reset_to_identity_grid,
  * RK4_grid over -dt_half for every face family, then advect_u: u1 = T . u0(psi).
  * u0 and u1 must not alias.  psi_out/T_out ([F][3] per family, AoS like the reference grids)
- * may be NULL; when given they receive psi_{x,y,z}_grid / T_{x,y,z}_grid. */
+ * may be NULL; when given they receive psi_{x,y,z}_grid / T_{x,y,z}_grid.
+ * Where the workspace holds padded copies of velocity fields (pfm_workspace_size), midpoint, RK4 and
+ * step-graph calls of one handle on different streams wait for each other's use of them, and a call
+ * that a caller captures does without them; the results are the same bit for bit. */
 int pfm3_midpoint(pfm_handle* h, const float* u0_x, const float* u0_y, const float* u0_z,
                   float* u1_x, float* u1_y, float* u1_z, float dt_half, float* psi_out[3],
                   float* T_out[3], void* stream);

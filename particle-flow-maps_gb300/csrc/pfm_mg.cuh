@@ -89,8 +89,10 @@ __device__ __forceinline__ void decode(const Lvl& L, int64_t e, int& i, int& j, 
 }
 
 // GB300 issues one FP64 warp instruction per 16 cycles and SM, with 63 cycles of latency for an addition
-// and 670 for a division, so the sums of compensated f32 terms are trees of f32 pairs (Knuth's TwoSum,
-// about 48 bits: far below the rounding of the f32 terms themselves).
+// and 670 for a division, so the sums of f32 products in a cluster solve, a serial chain, are trees of f32 pairs
+// (Knuth's TwoSum, about 48 bits; in FP64 an iteration took 26.3 us instead of 23.2 at 128 x 128, 35.5 instead of
+// 31.0 at 256 x 256).  A sum of 1,024 to 262,144 squares differs from the FP64 sum by at most 5e-15 of itself; its
+// error against 64 bits is the rounding of the f32 terms, 5e-10 to 8e-9, the same to three digits either way.
 struct Pair {
   float s, c;
 };

@@ -21,7 +21,7 @@
 //    floating-point division when the divisor is known in advance", IEEE Trans. Computers 53(8),
 //    2004): q = fma(x, zh, x zl) with zh = RN(1/m), zl = RN(1/m - zh).  For m = 1..6 it equals the
 //    IEEE quotient for every significand (tests/test_mg_cluster.py checks all 2^23 on the CPU), so
-//    every cell update is bitwise the grid-wide kernels'.
+//    every cell update is bitwise the grid-wide kernels' (below some 1e-30 the last bit may differ).
 //
 // The waits for other CTAs' rows and totals are mbarrier waits bounded in time; the others are hardware
 // cluster or block barriers that all threads reach the same number of times.  A wait that gives up says so in
@@ -31,9 +31,9 @@
 // (pass_barrier).  A thread that has seen it neither pushes nor expects rows any more, and no CTA returns its
 // shared memory before the rows in flight have landed (leave).
 //
-// Measured (one PCG iteration, FP32, GB300): 128^2 103 -> 23 us, 256^2 125 -> 31 us, 512^2 165 -> 54 us,
-// 32^3 107 -> 28 us, 64^3 155 -> 60 us; the coarse levels of 128^3 and 1024^2 as one launch: 210 -> 185 and
-// 180 -> 141 us per iteration.  What bounds it: the chain of half-sweeps -- about 850 cycles each on the
+// Measured (one PCG iteration, FP32, GB300; against the grid-wide kernels of now): 128^2 89 -> 24 us, 256^2
+// 111 -> 33 us, 512^2 141 -> 56 us, 32^3 91 -> 31 us, 64^3 125 -> 62 us; the coarse levels of 128^3 and 1024^2 as one
+// launch: 190 -> 157 and 182 -> 132 us per iteration.  What bounds it: the chain of half-sweeps -- about 850 cycles each on the
 // distributed levels (a row's flight through the cluster is some 400 of them), 60 to 200 on the solo ones.
 #include <cooperative_groups.h>
 

@@ -647,7 +647,9 @@ struct Colour8<float> {
 };
 
 // x / m for m = 1 .. 6 fluid neighbours in two operations, correctly rounded (as the cluster's smoother:
-// Brisebarre, Muller and Raina, 2004): inv = (RN(1/m), RN(1/m - RN(1/m))).
+// Brisebarre, Muller and Raina, 2004): inv = (RN(1/m), RN(1/m - RN(1/m))).  For |x| below some 1e-30 the low part is
+// subnormal and the last bit may differ; an infinite x, which an IEEE quotient keeps, gives NaN (a solve that meets
+// either ends as non-finite).
 constexpr float inv_hi(int m) { return (float)(1.0 / m); }
 constexpr float inv_lo(int m) { return (float)((1.0 - (double)inv_hi(m) * m) / m); }
 // The pairs travel with a kernel's parameters: in __constant__ memory they made every launch of this file's kernels
@@ -1165,8 +1167,8 @@ __global__ void __launch_bounds__(256) k_zero(S* __restrict__ a, int64_t n, cons
 // ---------------------------------------------------------------------------------------------
 // The passes over whole vectors of the finest level (dots, x and r updates, A p, true residual) read 16-byte
 // vectors where the grid allows: one 4-byte load per thread and array left too few bytes in flight.  The mixed
-// solve's dots, A p and true residual take runs of eight elements per thread and f32 pair trees (four blocks of
-// 64 registers a thread per SM instead of eight of 32); the sums that its 16-bit rounding or the plain FP32
+// solve's dots, A p and true residual take runs of eight elements per thread and one FP64 tree per block (four blocks
+// of 64 registers a thread per SM instead of eight of 32); the sums that its 16-bit rounding or the plain FP32
 // solve depend on keep the order of one element per thread, bit for bit (lanes_sum).  256^3, FP16 levels: x/r
 // update 104 -> 69 us, A p 69 -> 44, r . z 31 -> 23, true residual 23 -> 12, recentring 34 -> 23, p update
 // 34 -> 20; 160 x 96 x 72, FP32: x/r update 22 -> 13 us, A p 13 -> 9.6, dots 10 -> 8.4.  Small grids, where

@@ -227,8 +227,8 @@ __global__ void __launch_bounds__(kBinThreads) k_payload2(const int* __restrict_
 // (Adding into the face grids from 8 launches by tile parity gives the same sums, but each launch ends
 // in a wave that fills part of the SMs -- 128 of 304 resident blocks at 64^3 -- and reads the faces back.
 // With its zeroing and normalisation passes it took 505 us at 96^3, 8 particles per cell, this 350; 7.11
-// and 6.35 ms at 256^3.)  k_tile3 is bound by latency and by the longest cell of a warp (two blocks of 128
-// registers a thread per SM), k_tile_faces3 by memory.
+// and 6.35 ms at 256^3.)  k_tile3 is bound by issue and by the longest cell of a warp (two blocks of 128
+// registers a thread per SM: 61% of the issue slots, DRAM 20%), k_tile_faces3 by issue (77%, DRAM 29%).
 //
 // Record staging: a cell's particles are gathered through the sorted order, so each one costs a
 // memory round trip.  Every thread keeps a ring of kRing particle slots in shared memory (pos4 and
